@@ -212,23 +212,6 @@ __global__ void k_divergence(Geo G, int nx, int ny, int nz, double a, const doub
   }
 }
 
-// Correctly rounded IEEE double operations on the host and the device, for
-// constants that the host forms once per launch (the host's double
-// arithmetic is IEEE binary64 with round to nearest, as __ddiv_rn is).
-__host__ __device__ __forceinline__ double div_rn(double a, double b) {
-#ifdef __CUDA_ARCH__
-  return __ddiv_rn(a, b);
-#else
-  return a / b;
-#endif
-}
-__host__ __device__ __forceinline__ double mul_rn(double a, double b) {
-#ifdef __CUDA_ARCH__
-  return __dmul_rn(a, b);
-#else
-  return a * b;
-#endif
-}
 __host__ __device__ __forceinline__ double quiet_nan() {
 #ifdef __CUDA_ARCH__
   return __longlong_as_double(0x7ff8000000000000LL);
@@ -249,45 +232,6 @@ __host__ __device__ __forceinline__ double quiet_nan() {
 // west, south and bottom faces of its cell; the faces on the domain
 // boundary are not touched (they hold the walls' values, which
 // bnd_update_nooutlet restores in the reference), nor is w in 2-D.
-// Division by a divisor b known in advance (the spacing h, the density of a
-// pure phase), rounded to nearest like a / b itself: with y = RN(1/b) formed
-// once, q0 = RN(a y) lies within one ulp of a/b, the remainder r = a - b q0
-// is exact in one FMA, and RN(q0 + r y) = RN(a/b) (Markstein's theorem:
-// P. Markstein, IBM J. Res. Develop. 34(1), 1990; its use for a divisor
-// known in advance: N. Brisebarre, J.-M. Muller and S. K. Raina, IEEE Trans.
-// Comput. 53(8), 2004). The theorem needs every intermediate normal, so b
-// is restricted to [2^-60, 2^60] and |a| to (2^-900, 2^900); zero, infinite
-// and NaN dividends, and everything outside those ranges, take the division
-// itself.
-struct KnownDiv {
-  double b, y;
-  bool ok;
-  KnownDiv() = default;
-  __host__ __device__ __forceinline__ explicit KnownDiv(double b_) : b(b_) {
-    y = div_rn(1.0, b_);
-    const double m = fabs(b_);
-    ok = m >= 0x1p-60 && m <= 0x1p60;
-  }
-  // a / b (a zero dividend: a b, the signed zero a / b is)
-  __device__ __forceinline__ double operator()(double a) const {
-    const double m = fabs(a);
-    if (ok && m > 0x1p-900 && m < 0x1p900) {
-      const double q0 = __dmul_rn(a, y);
-      return __fma_rn(__fma_rn(-q0, b, a), y, q0);
-    }
-    if (ok && m == 0.0) return __dmul_rn(a, b);
-    return __ddiv_rn(a, b);
-  }
-  // a / d for any d: the corrected product when d is b (b nonzero, so d == b
-  // means the same bits), else the division (a zero dividend over a finite
-  // nonzero d: a d, the same signed zero)
-  __device__ __forceinline__ double by(double a, double d) const {
-    if (d == b && ok) return (*this)(a);
-    if (a == 0.0 && d != 0.0 && isfinite(d)) return __dmul_rn(a, d);
-    return __ddiv_rn(a, d);
-  }
-};
-
 // Face densities of the two pure phases (colour 1 and 0) and the spacing:
 // the divisors the projection meets on every face away from an interface.
 struct PhaseDiv {

@@ -6,6 +6,7 @@
 #include <cstring>
 
 #include "pbg_ref_kernels.cuh"
+#include "pbg_sweep_kernels.cuh"
 
 namespace pbg {
 
@@ -381,110 +382,93 @@ __global__ void __launch_bounds__(kThreads, 4) k_cg_q(MatView<double> A, Geo G, 
 }
 
 // ---------------------------------------------------------------------------
-// Incomplete Cholesky preconditioners (Prec::ic0/ic2/ic3):
-// IncompleteCholesky0/2/3::form (preconditioner_form.cpp:16-144) and ::solve
-// (preconditioner_solve.cpp:14-110). The reference runs factor and sweeps in
-// lexicographic i, j, k order. Every value a cell reads was written by a cell
-// with a smaller index h = a i + b j + k (a = b = 2 for IC0/IC2; a = 5, b = 2
-// for IC3, whose Mnw term reaches (i-1, j+2, k)), so one launch per
-// hyperplane h processes independent cells, each with the reference's
-// arithmetic in the reference's order (__dmul_rn/__dsub_rn/__ddiv_rn/
-// __dsqrt_rn, no contraction): the results are the reference's bit for bit.
-// The arrays are compact and start at zero; the factor's writes outside the
-// domain (the reference's halo, which no interior cell reads) are skipped,
-// and so are the sweeps' terms with a neighbour outside (the reference
-// multiplies them by its zero halo).
+// IC3 (Prec::ic3): IncompleteCholesky3::form (preconditioner_form.cpp:99-144)
+// and ::solve (preconditioner_solve.cpp:14-110). The reference runs factor
+// and sweeps in lexicographic i, j, k order. Every value a cell reads was
+// written by a cell with a smaller index h = 5 i + 2 j + k (its Mnw term
+// reaches (i-1, j+2, k)), so one launch per plane h processes independent
+// cells, each with the reference's arithmetic in the reference's order: the
+// results are the reference's bit for bit. The arrays are compact and start
+// at zero; the factor's writes outside the domain (the reference's halo,
+// which no interior cell reads) are skipped, and so are the sweeps' terms
+// with a neighbour outside (the reference multiplies them by its zero halo).
+// IC0 and IC2 run as one launch a sweep (pbg_sweeps.cuh).
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ double msub(double s, double a, double b) { return __dsub_rn(s, __dmul_rn(a, b)); }
-
-// cell (i, j, k) of hyperplane h for thread index t over the (i, j) plane
-__device__ __forceinline__ bool ic_cell(const MatView<double> &A, int h, int wa, int wb, long long t, int &i,
-                                        int &j, int &k) {
+// cell (i, j, k) of plane h for thread index t over the (i, j) plane
+__device__ __forceinline__ bool ic3_cell(const MatView<double> &A, int h, long long t, int &i, int &j, int &k) {
   i = (int)(t / A.ny);
   j = (int)(t - (long long)i * A.ny);
-  k = h - wa * i - wb * j;
+  k = h - 5 * i - 2 * j;
   return k >= 0 && k < A.nz;
 }
 
-__global__ void k_ic_form(MatView<double> A, IcFactor M, int h) {
+__global__ void k_ic3_form(MatView<double> A, Ic3Factor M, int h) {
   const long long SI = (long long)A.ny * A.nz, SJ = A.nz;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < (long long)A.nx * A.ny;
        t += (long long)gridDim.x * blockDim.x) {
     int i, j, k;
-    if (!ic_cell(A, h, M.wa, M.wb, t, i, j, k)) continue;
+    if (!ic3_cell(A, h, t, i, j, k)) continue;
     const long long p = ((long long)i * A.ny + j) * A.nz + k;
     const bool xp = i + 1 < A.nx, yp = j + 1 < A.ny, zp = k + 1 < A.nz, zm = k > 0, ym = j > 0;
     double sum = A.c[p];
     sum = msub(sum, M.w[p], M.w[p]);
-    if (M.kind >= 2) sum = msub(sum, M.tw[p], M.tw[p]);
-    if (M.kind == 3) sum = msub(sum, M.nw[p], M.nw[p]);
+    sum = msub(sum, M.tw[p], M.tw[p]);
+    sum = msub(sum, M.nw[p], M.nw[p]);
     sum = msub(sum, M.s[p], M.s[p]);
-    if (M.kind >= 2) sum = msub(sum, M.ts[p], M.ts[p]);
+    sum = msub(sum, M.ts[p], M.ts[p]);
     sum = msub(sum, M.b[p], M.b[p]);
     sum = __dsqrt_rn(sum);
     M.c[p] = sum;
-    if (M.kind == 1) {
-      if (xp) M.w[p + SI] = __ddiv_rn(-A.w[p + SI], sum);
-      if (yp) M.s[p + SJ] = __ddiv_rn(-A.s[p + SJ], sum);
-      if (zp) M.b[p + 1] = __ddiv_rn(-A.b[p + 1], sum);
-      continue;
-    }
     if (xp) M.w[p + SI] = __ddiv_rn(-A.w[p + SI], sum);
     if (xp && zm) M.tw[p + SI - 1] = __ddiv_rn(__dmul_rn(-M.w[p + SI - 1], M.b[p]), sum);
-    if (M.kind == 3 && xp && ym)
+    if (xp && ym)
       M.nw[p + SI - SJ] = __ddiv_rn(__dsub_rn(__dmul_rn(-M.w[p + SI - SJ], M.s[p]),
                                               __dmul_rn(M.tw[p + SI - SJ], M.ts[p])), sum);
-    if (yp) {
-      if (M.kind == 2) M.s[p + SJ] = __ddiv_rn(-A.s[p + SJ], sum);
-      else M.s[p + SJ] = __ddiv_rn(msub(msub(-A.s[p + SJ], M.w[p + SJ], M.nw[p]), M.nw[p + SJ], M.s[p]), sum);
-    }
-    if (yp && zm) {
-      if (M.kind == 2) M.ts[p + SJ - 1] = __ddiv_rn(__dmul_rn(-M.s[p + SJ - 1], M.b[p]), sum);
-      else
-        M.ts[p + SJ - 1] = __ddiv_rn(__dsub_rn(__dmul_rn(-M.s[p + SJ - 1], M.b[p]),
-                                               __dmul_rn(M.tw[p + SJ - 1], M.nw[p])), sum);
-    }
+    if (yp) M.s[p + SJ] = __ddiv_rn(msub(msub(-A.s[p + SJ], M.w[p + SJ], M.nw[p]), M.nw[p + SJ], M.s[p]), sum);
+    if (yp && zm)
+      M.ts[p + SJ - 1] = __ddiv_rn(__dsub_rn(__dmul_rn(-M.s[p + SJ - 1], M.b[p]),
+                                             __dmul_rn(M.tw[p + SJ - 1], M.nw[p])), sum);
     if (zp) M.b[p + 1] = __ddiv_rn(msub(msub(-A.b[p + 1], M.w[p + 1], M.tw[p]), M.s[p + 1], M.ts[p]), sum);
   }
 }
 
-// forward sweep on hyperplane h: z = (r - lower terms) / Mc
-__global__ void k_ic_fwd(MatView<double> A, IcFactor M, int h, const double *__restrict__ r, double *z,
-                         const KrylovState *st) {
+// forward sweep on plane h: z = (r - lower terms) / Mc
+__global__ void k_ic3_fwd(MatView<double> A, Ic3Factor M, int h, const double *__restrict__ r, double *z,
+                          const KrylovState *st) {
   if (st->done) return;
   const long long SI = (long long)A.ny * A.nz, SJ = A.nz;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < (long long)A.nx * A.ny;
        t += (long long)gridDim.x * blockDim.x) {
     int i, j, k;
-    if (!ic_cell(A, h, M.wa, M.wb, t, i, j, k)) continue;
+    if (!ic3_cell(A, h, t, i, j, k)) continue;
     const long long p = ((long long)i * A.ny + j) * A.nz + k;
     double sum = r[p];
     if (i > 0) sum = msub(sum, M.w[p], z[p - SI]);
-    if (M.kind >= 2 && i > 0 && k + 1 < A.nz) sum = msub(sum, M.tw[p], z[p - SI + 1]);
-    if (M.kind == 3 && i > 0 && j + 1 < A.ny) sum = msub(sum, M.nw[p], z[p - SI + SJ]);
+    if (i > 0 && k + 1 < A.nz) sum = msub(sum, M.tw[p], z[p - SI + 1]);
+    if (i > 0 && j + 1 < A.ny) sum = msub(sum, M.nw[p], z[p - SI + SJ]);
     if (j > 0) sum = msub(sum, M.s[p], z[p - SJ]);
-    if (M.kind >= 2 && j > 0 && k + 1 < A.nz) sum = msub(sum, M.ts[p], z[p - SJ + 1]);
+    if (j > 0 && k + 1 < A.nz) sum = msub(sum, M.ts[p], z[p - SJ + 1]);
     if (k > 0) sum = msub(sum, M.b[p], z[p - 1]);
     z[p] = __ddiv_rn(sum, M.c[p]);
   }
 }
 
-// backward sweep on hyperplane h: z = (z - upper terms) / Mc
-__global__ void k_ic_bwd(MatView<double> A, IcFactor M, int h, double *z, const KrylovState *st) {
+// backward sweep on plane h: z = (z - upper terms) / Mc
+__global__ void k_ic3_bwd(MatView<double> A, Ic3Factor M, int h, double *z, const KrylovState *st) {
   if (st->done) return;
   const long long SI = (long long)A.ny * A.nz, SJ = A.nz;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < (long long)A.nx * A.ny;
        t += (long long)gridDim.x * blockDim.x) {
     int i, j, k;
-    if (!ic_cell(A, h, M.wa, M.wb, t, i, j, k)) continue;
+    if (!ic3_cell(A, h, t, i, j, k)) continue;
     const long long p = ((long long)i * A.ny + j) * A.nz + k;
     const bool xp = i + 1 < A.nx, yp = j + 1 < A.ny, zp = k + 1 < A.nz, zm = k > 0, ym = j > 0;
     double sum = z[p];
     if (xp) sum = msub(sum, M.w[p + SI], z[p + SI]);
-    if (M.kind >= 2 && xp && zm) sum = msub(sum, M.tw[p + SI - 1], z[p + SI - 1]);
-    if (M.kind == 3 && xp && ym) sum = msub(sum, M.nw[p + SI - SJ], z[p + SI - SJ]);
+    if (xp && zm) sum = msub(sum, M.tw[p + SI - 1], z[p + SI - 1]);
+    if (xp && ym) sum = msub(sum, M.nw[p + SI - SJ], z[p + SI - SJ]);
     if (yp) sum = msub(sum, M.s[p + SJ], z[p + SJ]);
-    if (M.kind >= 2 && yp && zm) sum = msub(sum, M.ts[p + SJ - 1], z[p + SJ - 1]);
+    if (yp && zm) sum = msub(sum, M.ts[p + SJ - 1], z[p + SJ - 1]);
     if (zp) sum = msub(sum, M.b[p + 1], z[p + 1]);
     z[p] = __ddiv_rn(sum, M.c[p]);
   }
@@ -1005,9 +989,10 @@ __global__ void k_ac_resnorm(MatView<double> A, const double *__restrict__ phi,
 // Gauss-Seidel's sweep runs i, then j, then k (for_vijk) and reads the new
 // values of the cells before the current one and the old values of the
 // cells after it. Every neighbour of (i, j, k) lies on the hyperplane
-// i + j + k - 1 (those before it) or i + j + k + 1 (those after it), so one
-// launch per hyperplane h = i + j + k, in increasing h, computes every cell
-// from exactly the values the sequential sweep uses.
+// i + j + k - 1 (those before it) or i + j + k + 1 (those after it), so a
+// schedule that keeps the planes' order computes every cell from exactly the
+// values the sequential sweep uses: k_gs_sweep (pbg_sweeps.cuh), or on
+// periodic matrices one launch of k_gs_plane per plane.
 // ---------------------------------------------------------------------------
 // all entries unreal (gaussseidel.cpp:28-33; CG also seeds the last with res0)
 __device__ void stale_fill_dev(KrylovState *st) {
@@ -1067,7 +1052,7 @@ __global__ void k_jacobi_x(long long N, const double *__restrict__ c, const doub
     x[p] = __dmul_rn(ci[p], __dadd_rn(r[p], __dmul_rn(c[p], x[p])));
 }
 
-// the cells of hyperplane h: x = ci (b + w xw + e xe + s xs + n xn + b xb
+// periodic matrices: the cells of hyperplane h: x = ci (b + w xw + e xe + s xs + n xn + b xb
 // + t xt), summed left to right (gaussseidel.cpp:50-60). One thread per
 // (i, j) column; k = h - i - j. Across a periodic face the reference reads
 // its halo, filled by the exchange before the sweep: xold, a copy of x
@@ -1171,25 +1156,70 @@ void RefKrylovWork::ensure(size_t n, int solver) {
   if (solver == 2) fit(u);
 }
 
-IcFactor RefKrylovWork::ic(int kind, size_t n) {
-  auto fit = [n](DBuf<double> &b) { if (b.n < n) b.alloc(n); };
-  fit(z); fit(mc); fit(mw); fit(ms); fit(mb);
-  if (kind >= 2) { fit(mtw); fit(mts); }
-  if (kind == 3) fit(mnw);
-  IcFactor M;
-  M.c = mc.p; M.w = mw.p; M.s = ms.p; M.b = mb.p;
-  M.tw = kind >= 2 ? mtw.p : nullptr;
-  M.ts = kind >= 2 ? mts.p : nullptr;
-  M.nw = kind == 3 ? mnw.p : nullptr;
-  M.kind = kind;
-  M.wa = kind == 3 ? 5 : 2;
-  M.wb = 2;
-  return M;
+Ic3Factor RefKrylovWork::ic3(size_t n) {
+  DBuf<double> *arr[8] = {&z, &mc, &mw, &ms, &mb, &mtw, &mts, &mnw};
+  for (DBuf<double> *a : arr)
+    if (a->n < n) a->alloc(n);
+  return {mc.p, mw.p, ms.p, mb.p, mtw.p, mts.p, mnw.p};
 }
 
-// hyperplanes of the IC schedule (h = wa i + wb j + k over the grid)
-static int ic_planes(const MatView<double> &A, const IcFactor &M) {
-  return M.wa * (A.nx - 1) + M.wb * (A.ny - 1) + (A.nz - 1) + 1;
+IcFactor RefKrylovWork::ic(int kind, const SweepGeo &g) {
+  const size_t n = g.size();
+  auto fit = [](DBuf<double> &b, size_t m) { if (b.n < m) b.alloc(m); };
+  fit(z, (size_t)g.nx * g.ny * g.nz);
+  for (DBuf<double> *a : {&zm, &mc, &my, &mw, &ms, &mb}) fit(*a, n);
+  if (kind == 2) { fit(mtw, n); fit(mts, n); }
+  return {mc.p, my.p, mw.p, ms.p, mb.p, mtw.p, mts.p};
+}
+
+GsOps RefKrylovWork::gs(const SweepGeo &g) {
+  for (DBuf<double> &b : go)
+    if (b.n < g.size()) b.alloc(g.size());
+  return {go[0].p, go[1].p, go[2].p, go[3].p, go[4].p, go[5].p, go[6].p, go[7].p, go[8].p};
+}
+
+// Exchange words and tickets; new memory is zeroed, which no epoch equals.
+void RefKrylovWork::sweep_alloc(size_t n, cudaStream_t s) {
+  if (words.n < n) {
+    words.alloc(n);
+    PBG_CUDA(cudaMemsetAsync(words.p, 0, words.bytes(), s));
+  }
+  if (!ticket.n) {
+    ticket.alloc(4);
+    PBG_CUDA(cudaMemsetAsync(ticket.p, 0, ticket.bytes(), s));
+  }
+  if (!hstuck) {
+    PBG_CUDA(cudaMallocHost((void **)&hstuck, sizeof(int)));
+    *hstuck = 0;
+  }
+}
+
+void RefKrylovWork::sweep_check_enqueue(cudaStream_t s) {
+  if (ticket.n) PBG_CUDA(cudaMemcpyAsync(hstuck, ticket.p + 2, sizeof(int), cudaMemcpyDeviceToHost, s));
+}
+
+void RefKrylovWork::sweep_check() {
+  if (!ticket.n || !*hstuck) return;
+  *hstuck = 0;
+  ticket.release();  // start over with cleared flags
+  throw CudaError("a sweep's wait for a neighbouring tile ran out");
+}
+
+RefKrylovWork::~RefKrylovWork() {
+  if (hstuck) cudaFreeHost(hstuck);
+}
+
+// planes of the IC3 schedule over the grid
+static int ic3_planes(const MatView<double> &A) { return 5 * (A.nx - 1) + 2 * (A.ny - 1) + A.nz; }
+
+// the factor of kind (1 IC0, 2 IC2) on every solve, as the reference forms it
+static void ic_form(const MatView<double> &A, int kind, RefKrylovWork &w, cudaStream_t s) {
+  const SweepGeo g = SweepGeo::make(A.nx, A.ny, A.nz, sweep_a(kind));
+  const IcFactor M = w.ic(kind, g);
+  w.sweep_alloc(g.words() * (kind == 2 ? 2 : 1), s);
+  if (kind == 2) k_ic_factor<2><<<g.tiles(), kSweepCols, 0, s>>>(g, A, M, w.sweep());
+  else k_ic_factor<1><<<g.tiles(), kSweepCols, 0, s>>>(g, A, M, w.sweep());
+  note_launch();
 }
 
 void enqueue_ref_setup(const MatView<double> &A, double *x, const double *b, const KrylovParams &pr,
@@ -1206,6 +1236,11 @@ void enqueue_ref_setup(const MatView<double> &A, double *x, const double *b, con
       k_recip<<<grid_for(N), kThreads, 0, s>>>(N, A.c, w.mcd.p); note_launch();
       w.ci = w.mcd.p;
     }
+    if (solver == 4 && !A.per) {  // the sweeps' operands in march order
+      const SweepGeo sg = SweepGeo::make(A.nx, A.ny, A.nz, sweep_a(1));
+      w.sweep_alloc(sg.words(), s);
+      k_gs_pack<<<grid_for((long long)sg.size()), kThreads, 0, s>>>(sg, A, w.ci, b, x, w.gs(sg)); note_launch();
+    }
     k_it_init<<<g, kThreads, 0, s>>>(A, x, b, w.r.p, st, red.slot_part(0), red.slot_count(0),
                                      solver == 4 ? 1 : 0); note_launch();
     PBG_CUDA(cudaGetLastError());
@@ -1216,13 +1251,14 @@ void enqueue_ref_setup(const MatView<double> &A, double *x, const double *b, con
     PBG_CUDA(cudaMemsetAsync(w.v.p, 0, sizeof(double) * N, s));
     PBG_CUDA(cudaMemsetAsync(w.q.p, 0, sizeof(double) * N, s));
   }
-  if (pr.prec > 0) {  // IncompleteCholesky*::form on every solve (precform)
-    const IcFactor M = w.ic(pr.prec, (size_t)N);
-    DBuf<double> *arr[8] = {&w.z, &w.mc, &w.mw, &w.ms, &w.mb, &w.mtw, &w.mts, &w.mnw};
-    for (DBuf<double> *a : arr)
-      if (a->p) PBG_CUDA(cudaMemsetAsync(a->p, 0, sizeof(double) * N, s));
-    const int H = ic_planes(A, M), gp = grid_for((long long)A.nx * A.ny);
-    for (int h = 0; h < H; ++h) { k_ic_form<<<gp, kThreads, 0, s>>>(A, M, h); note_launch(); }
+  if (pr.prec == 3) {  // IncompleteCholesky*::form on every solve (precform)
+    const Ic3Factor M = w.ic3((size_t)N);
+    for (double *a : {w.z.p, M.c, M.w, M.s, M.b, M.tw, M.ts, M.nw})
+      PBG_CUDA(cudaMemsetAsync(a, 0, sizeof(double) * N, s));
+    const int H = ic3_planes(A), gp = grid_for((long long)A.nx * A.ny);
+    for (int h = 0; h < H; ++h) { k_ic3_form<<<gp, kThreads, 0, s>>>(A, M, h); note_launch(); }
+  } else if (pr.prec > 0) {
+    ic_form(A, pr.prec, w, s);
   }
   k_recip<<<grid_for(N), kThreads, 0, s>>>(N, A.c, w.mcd.p); note_launch();
   if (solver == 0)
@@ -1233,12 +1269,27 @@ void enqueue_ref_setup(const MatView<double> &A, double *x, const double *b, con
   PBG_CUDA(cudaGetLastError());
 }
 
-// z = M^-1 r with the IC factor: forward then backward hyperplane sweeps
-static void ic_apply(const MatView<double> &A, const IcFactor &M, const double *r, double *z,
+// z = M^-1 r with the IC factor: forward, then backward sweep
+static void ic_apply(const MatView<double> &A, int prec, RefKrylovWork &w, const double *r, double *z,
                      const KrylovState *st, cudaStream_t s) {
-  const int H = ic_planes(A, M), gp = grid_for((long long)A.nx * A.ny);
-  for (int h = 0; h < H; ++h) { k_ic_fwd<<<gp, kThreads, 0, s>>>(A, M, h, r, z, st); note_launch(); }
-  for (int h = H - 1; h >= 0; --h) { k_ic_bwd<<<gp, kThreads, 0, s>>>(A, M, h, z, st); note_launch(); }
+  if (prec == 3) {
+    const Ic3Factor M = w.ic3((size_t)A.ncell());
+    const int H = ic3_planes(A), gp = grid_for((long long)A.nx * A.ny);
+    for (int h = 0; h < H; ++h) { k_ic3_fwd<<<gp, kThreads, 0, s>>>(A, M, h, r, z, st); note_launch(); }
+    for (int h = H - 1; h >= 0; --h) { k_ic3_bwd<<<gp, kThreads, 0, s>>>(A, M, h, z, st); note_launch(); }
+    return;
+  }
+  const SweepGeo g = SweepGeo::make(A.nx, A.ny, A.nz, sweep_a(prec));
+  const IcFactor M = w.ic(prec, g);
+  const int n = g.tiles();
+  if (prec == 2) {
+    k_ic_sweep<2, false><<<n, kSweepCols, 0, s>>>(g, M, r, w.zm.p, z, w.sweep(), st);
+    k_ic_sweep<2, true><<<n, kSweepCols, 0, s>>>(g, M, r, w.zm.p, z, w.sweep(), st);
+  } else {
+    k_ic_sweep<1, false><<<n, kSweepCols, 0, s>>>(g, M, r, w.zm.p, z, w.sweep(), st);
+    k_ic_sweep<1, true><<<n, kSweepCols, 0, s>>>(g, M, r, w.zm.p, z, w.sweep(), st);
+  }
+  note_launch(); note_launch();
 }
 
 void enqueue_ref_iters(const MatView<double> &A, double *x, int solver, int count,
@@ -1252,12 +1303,14 @@ void enqueue_ref_iters(const MatView<double> &A, double *x, int solver, int coun
   if (solver >= 3) {  // Jacobi, Gauss-Seidel
     const int gs = solver == 4 ? 1 : 0;
     const int H = A.nx + A.ny + A.nz - 2, gp = grid_for((long long)A.nx * A.ny);
+    const SweepGeo sg = SweepGeo::make(A.nx, A.ny, A.nz, sweep_a(1));
     for (int it = 0; it < count; ++it) {
-      if (gs) {
-        if (A.per) {  // the halo the exchange fills before each sweep
-          if (w.xold.n < (size_t)N) w.xold.alloc(N);
-          PBG_CUDA(cudaMemcpyAsync(w.xold.p, x, sizeof(double) * N, cudaMemcpyDeviceToDevice, s));
-        }
+      if (gs && !A.per) {
+        k_gs_sweep<<<sg.tiles(), kSweepCols, 0, s>>>(sg, w.gs(sg), x, w.sweep(), st); note_launch();
+      } else if (gs) {
+        // the halo the exchange fills before each sweep
+        if (w.xold.n < (size_t)N) w.xold.alloc(N);
+        PBG_CUDA(cudaMemcpyAsync(w.xold.p, x, sizeof(double) * N, cudaMemcpyDeviceToDevice, s));
         for (int h = 0; h < H; ++h) {
           k_gs_plane<<<gp, kThreads, 0, s>>>(A, w.ci, w.rhs, x, h, st, w.xold.p); note_launch();
         }
@@ -1269,12 +1322,10 @@ void enqueue_ref_iters(const MatView<double> &A, double *x, int solver, int coun
     PBG_CUDA(cudaGetLastError());
     return;
   }
-  IcFactor M{};
-  if (prec > 0) M = w.ic(prec, (size_t)N);
   for (int it = 0; it < count; ++it) {
     if (solver == 0 && prec > 0) {
       // z = M^-1 r (forward and backward sweeps), rho = r.z, then the CG step
-      ic_apply(A, M, w.r.p, w.z.p, st, s);
+      ic_apply(A, prec, w, w.r.p, w.z.p, st, s);
       k_cg_rho<<<g, kThreads, 0, s>>>(N, w.r.p, w.z.p, st, P0, C0); note_launch();
       k_cg_pq<<<g, kThreads, 0, s>>>(A, w.r.p, w.pA.p, w.pB.p, w.q.p, st, P0, C0, w.z.p, w.mcd.p); note_launch();
       k_cg_xr<true><<<g, kThreads, 0, s>>>(N, w.mcd.p, x, w.r.p, w.pA.p, w.pB.p, w.q.p, st, hist, P1, C1, 1); note_launch();
@@ -1289,19 +1340,19 @@ void enqueue_ref_iters(const MatView<double> &A, double *x, int solver, int coun
     } else if (solver == 1) {
       k_bi_rho<<<g, kThreads, 0, s>>>(N, w.rt.p, w.r.p, st, P0, C0); note_launch();
       k_bi_p<<<g, kThreads, 0, s>>>(N, w.mcd.p, w.r.p, w.pA.p, w.v.p, w.ph.p, st, diag); note_launch();
-      if (!diag) ic_apply(A, M, w.pA.p, w.ph.p, st, s);
+      if (!diag) ic_apply(A, prec, w, w.pA.p, w.ph.p, st, s);
       k_bi_spmv<<<g, kThreads, 0, s>>>(A, w.ph.p, w.v.p, w.rt.p, 0, st, P1, C1); note_launch();
       k_bi_s<<<g, kThreads, 0, s>>>(N, w.mcd.p, w.r.p, w.v.p, w.s.p, w.sh.p, st, P0, C0, diag); note_launch();
-      if (!diag) ic_apply(A, M, w.s.p, w.sh.p, st, s);
+      if (!diag) ic_apply(A, prec, w, w.s.p, w.sh.p, st, s);
       k_bi_spmv<<<g, kThreads, 0, s>>>(A, w.sh.p, w.t.p, w.s.p, 1, st, P1, C1); note_launch();
       k_bi_xr<<<g, kThreads, 0, s>>>(N, x, w.r.p, w.ph.p, w.sh.p, w.s.p, w.t.p, st, hist, P0, C0); note_launch();
     } else {
       k_cgs_rho<<<g, kThreads, 0, s>>>(N, w.rt.p, w.r.p, st, P0, C0); note_launch();
       k_cgs_up<<<g, kThreads, 0, s>>>(N, w.mcd.p, w.r.p, w.q.p, w.u.p, w.pA.p, w.ph.p, st, diag); note_launch();
-      if (!diag) ic_apply(A, M, w.pA.p, w.ph.p, st, s);
+      if (!diag) ic_apply(A, prec, w, w.pA.p, w.ph.p, st, s);
       k_bi_spmv<<<g, kThreads, 0, s>>>(A, w.ph.p, w.v.p, w.rt.p, 0, st, P1, C1); note_launch();
       k_cgs_qs<<<g, kThreads, 0, s>>>(N, w.mcd.p, w.u.p, w.v.p, w.q.p, w.s.p, w.sh.p, st, diag); note_launch();
-      if (!diag) ic_apply(A, M, w.s.p, w.sh.p, st, s);
+      if (!diag) ic_apply(A, prec, w, w.s.p, w.sh.p, st, s);
       k_cgs_xr<<<g, kThreads, 0, s>>>(A, x, w.r.p, w.sh.p, st, hist, P0, C0); note_launch();
     }
   }
@@ -1317,7 +1368,9 @@ RefKrylovResult ref_krylov_solve(const MatView<double> &A, double *x, const doub
   int enq = 0, chunk = 8;
   for (;;) {
     PBG_CUDA(cudaMemcpyAsync(hst, st, sizeof(KrylovState), cudaMemcpyDeviceToHost, s));
+    w.sweep_check_enqueue(s);
     PBG_CUDA(cudaStreamSynchronize(s));
+    w.sweep_check();
     if (hst->done || enq >= pr.maxit) break;
     int cnt = chunk;
     if (enq + cnt > pr.maxit) cnt = pr.maxit - enq;
@@ -1656,7 +1709,9 @@ RefACResult RefAC::cycle(double *x, const double *b, const RefACParams &pa, RefA
     }
   }
   PBG_CUDA(cudaMemcpyAsync(x, l0.phi.p, sizeof(double) * N0, cudaMemcpyDeviceToDevice, s));
+  cx.w->sweep_check_enqueue(s);
   PBG_CUDA(cudaStreamSynchronize(s));
+  cx.w->sweep_check();
   out.nhist = nh;
   out.visits = (int)flex_calls_;
   return out;

@@ -6,14 +6,14 @@
 
 #include "pbg_common.cuh"
 #include "pbg_session.h"
+#include "pbg_sweeps.cuh"
 
 namespace pbg {
 
-// Incomplete Cholesky factor (compact arrays; kind 1 = IC0, 2 = IC2, 3 =
-// IC3) and the hyperplane weights h = wa i + wb j + k of its schedule.
-struct IcFactor {
+// IC3 factor (compact arrays), run one launch per plane h = 5 i + 2 j + k.
+// The other sweeps (IC0, IC2, Gauss-Seidel) are in pbg_sweeps.cuh.
+struct Ic3Factor {
   double *c, *w, *s, *b, *tw, *ts, *nw;
-  int kind, wa, wb;
 };
 
 struct KrylovParams {
@@ -32,8 +32,24 @@ struct RefKrylovWork {
   DBuf<double> xold;                              // Gauss-Seidel: x before the sweep (periodic)
   const double *rhs = nullptr, *ci = nullptr;     // Jacobi / Gauss-Seidel operands of a solve
   DBuf<double> z, mc, mw, ms, mb, mtw, mts, mnw;  // IC preconditioner
+  DBuf<double> my, zm;                            // IC0/IC2: 1 / mc and z in march order
+  DBuf<double> go[9];                             // Gauss-Seidel operands in march order
+  DBuf<SweepWord> words;                          // sweeps: exchange between tiles
+  DBuf<unsigned> ticket;                          // sweeps: tickets [0..1], the stuck flag [2]
+  unsigned long long epoch = 0;                   // sweeps: the last launch's epoch
+  int *hstuck = nullptr;                          // pinned copy of the stuck flag
+  ~RefKrylovWork();
   void ensure(size_t n, int solver);
-  IcFactor ic(int kind, size_t n);
+  Ic3Factor ic3(size_t n);
+  IcFactor ic(int kind, const SweepGeo &g);
+  GsOps gs(const SweepGeo &g);
+  void sweep_alloc(size_t words_needed, cudaStream_t s);
+  SweepSync sweep() {
+    return {words.p, ticket.p, reinterpret_cast<int *>(ticket.p + 2), ++epoch};
+  }
+  // enqueue the copy of the stuck flag / after a synchronisation, throw if it is set
+  void sweep_check_enqueue(cudaStream_t s);
+  void sweep_check();
 };
 
 struct RefKrylovResult {

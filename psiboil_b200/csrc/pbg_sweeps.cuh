@@ -1,0 +1,98 @@
+// Lexicographic sweeps as one launch: the incomplete Cholesky factor and its
+// triangular solves (Prec::ic0 and ic2) and the Gauss-Seidel sweep of the
+// reference-parity solvers. (IC3 also reads the column (i-1, j+1), which
+// would make neighbouring tiles wait for each other both ways; it keeps one
+// launch per plane, k_ic3_* in pbg_ref_kernels.cu.)
+//
+// The reference runs them cell after cell in i, j, k order. A cell needs the
+// results of a few cells before it, all of which lie on an earlier plane
+// h = a (i + j) + k (a = 1 or 2), so any schedule that keeps the planes'
+// order gives each cell exactly the values of the sequential sweep, and the
+// arithmetic per cell is the reference's, in its order (no contraction).
+//
+// One block of 64 threads owns the 8 x 8 columns of a tile of the (i, j)
+// plane and marches along k: at step t thread (li, lj) is at
+// k = t - a (li + lj), so the values it needs from the columns beside it
+// were formed in the step before and come from shared memory. Values crossing a tile's edge go through global memory as 16-byte
+// (value, epoch) words written and read whole: a word is valid when it
+// carries the sweep's epoch, so no fence and no reset is needed, and a
+// reader that finds an old word polls it (bounded). Blocks take their tiles
+// by ticket in an order in which every tile's predecessors come first, so a
+// block only ever waits for blocks that are already running.
+//
+// What bounds it: the chain of a (nx + ny - 2) + nz dependent steps
+// (shared-memory read, four to six dependent FP64 operations, a division)
+// plus about a microsecond for each tile edge on the way. One launch per
+// plane, the form before this, paid a launch for every step. All operands
+// that the sweeps own are stored in march order (SweepGeo::off), so that a
+// step's 64 loads are two contiguous rows, and are loaded kSweepAhead steps
+// early into registers.
+#pragma once
+
+#include "pbg_common.cuh"
+#include "pbg_session.h"
+
+namespace pbg {
+
+constexpr int kSweepTile = 8;                            // columns of a tile per direction
+constexpr int kSweepCols = kSweepTile * kSweepTile;      // threads of a block
+constexpr int kSweepAhead = 6;                           // steps an operand is loaded early
+constexpr int kSweepPoll = 1 << 22;                      // polls of one word before giving up
+// rows from which the march-order storage is skewed: below it the skew's
+// empty rows would outweigh the cells (2-D grids have one row)
+constexpr int kSweepSkewMin = 32;
+
+// weight a = b of the schedule: IC0 (kind 1) and Gauss-Seidel read the
+// columns beside a cell at its own k, IC2 (kind 2) also at k + 1
+__host__ __device__ constexpr int sweep_a(int kind) { return kind == 2 ? 2 : 1; }
+
+// A (value, epoch) word of the exchange between tiles, moved as 16 bytes.
+struct alignas(16) SweepWord { unsigned long long v, epoch; };
+
+// Tiles of a grid and the march-order storage of a cell array.
+struct SweepGeo {
+  int nx, ny, nz, ti, tj;
+  int skew;         // of the storage rows (0 on short columns)
+  int rows;         // rows of a tile's storage
+  __host__ static SweepGeo make(int nx, int ny, int nz, int a) {
+    SweepGeo g;
+    g.nx = nx; g.ny = ny; g.nz = nz;
+    g.ti = (nx + kSweepTile - 1) / kSweepTile;
+    g.tj = (ny + kSweepTile - 1) / kSweepTile;
+    g.skew = nz >= kSweepSkewMin ? a : 0;
+    g.rows = nz + 2 * g.skew * (kSweepTile - 1);
+    return g;
+  }
+  __host__ __device__ int tiles() const { return ti * tj; }
+  __host__ __device__ size_t size() const { return (size_t)tiles() * rows * kSweepCols; }
+  // storage index of cell (i, j, 0); cell (i, j, k) is kSweepCols * k further
+  __device__ __forceinline__ size_t off(int i, int j) const {
+    const int li = i % kSweepTile, lj = j % kSweepTile;
+    const size_t tile = (size_t)(i / kSweepTile) * tj + j / kSweepTile;
+    return (tile * rows + skew * (li + lj)) * kSweepCols + li * kSweepTile + lj;
+  }
+  // words of one exchanged value: the tiles' last columns along i, then along j
+  __host__ __device__ size_t words_i() const { return (size_t)ti * ny * nz; }
+  __host__ __device__ size_t words() const { return words_i() + (size_t)tj * nx * nz; }
+};
+
+// Shared state of the sweeps of one solver's workspace.
+struct SweepSync {
+  SweepWord *words;             // exchange, SweepGeo::words() per value
+  unsigned *ticket;             // [0] next tile, [1] finished tiles (both 0 between launches)
+  int *stuck;                   // set when a poll ran out
+  unsigned long long epoch;     // of this launch, larger than any before it
+};
+
+// Incomplete Cholesky factor in march order. y = 1 / c rounded, for the
+// division by c (NaN where KnownDiv's range does not hold).
+struct IcFactor {
+  double *c, *y, *w, *s, *b, *tw, *ts;
+};
+
+// Operands of the Gauss-Seidel sweeps of one solve in march order.
+struct GsOps {
+  double *b, *ci, *w, *e, *s, *n, *bt, *t, *x;
+};
+
+}  // namespace pbg
