@@ -1163,19 +1163,11 @@ Ic3Factor RefKrylovWork::ic3(size_t n) {
   return {mc.p, mw.p, ms.p, mb.p, mtw.p, mts.p, mnw.p};
 }
 
-IcFactor RefKrylovWork::ic(int kind, const SweepGeo &g) {
-  const size_t n = g.size();
-  auto fit = [](DBuf<double> &b, size_t m) { if (b.n < m) b.alloc(m); };
-  fit(z, (size_t)g.nx * g.ny * g.nz);
-  for (DBuf<double> *a : {&zm, &mc, &my, &mw, &ms, &mb}) fit(*a, n);
-  if (kind == 2) { fit(mtw, n); fit(mts, n); }
-  return {mc.p, my.p, mw.p, ms.p, mb.p, mtw.p, mts.p};
-}
-
-GsOps RefKrylovWork::gs(const SweepGeo &g) {
-  for (DBuf<double> &b : go)
-    if (b.n < g.size()) b.alloc(g.size());
-  return {go[0].p, go[1].p, go[2].p, go[3].p, go[4].p, go[5].p, go[6].p, go[7].p, go[8].p};
+// the operands of the sweeps in march order, `planes` a cell
+double *RefKrylovWork::march(const SweepGeo &g, int planes) {
+  const size_t n = g.all_rows() * planes * kSweepCols;
+  if (mo.n < n) mo.alloc(n);
+  return mo.p;
 }
 
 // Exchange words and tickets; new memory is zeroed, which no epoch equals.
@@ -1215,10 +1207,11 @@ static int ic3_planes(const MatView<double> &A) { return 5 * (A.nx - 1) + 2 * (A
 // the factor of kind (1 IC0, 2 IC2) on every solve, as the reference forms it
 static void ic_form(const MatView<double> &A, int kind, RefKrylovWork &w, cudaStream_t s) {
   const SweepGeo g = SweepGeo::make(A.nx, A.ny, A.nz, sweep_a(kind));
-  const IcFactor M = w.ic(kind, g);
+  double *M = w.march(g, ic_planes(kind));
+  if (w.z.n < (size_t)A.ncell()) w.z.alloc((size_t)A.ncell());
   w.sweep_alloc(g.words() * (kind == 2 ? 2 : 1), s);
-  if (kind == 2) k_ic_factor<2><<<g.tiles(), kSweepCols, 0, s>>>(g, A, M, w.sweep());
-  else k_ic_factor<1><<<g.tiles(), kSweepCols, 0, s>>>(g, A, M, w.sweep());
+  if (kind == 2) k_ic_factor<2><<<g.tiles(), kSweepThreads, 0, s>>>(g, A, M, w.sweep());
+  else k_ic_factor<1><<<g.tiles(), kSweepThreads, 0, s>>>(g, A, M, w.sweep());
   note_launch();
 }
 
@@ -1239,7 +1232,8 @@ void enqueue_ref_setup(const MatView<double> &A, double *x, const double *b, con
     if (solver == 4 && !A.per) {  // the sweeps' operands in march order
       const SweepGeo sg = SweepGeo::make(A.nx, A.ny, A.nz, sweep_a(1));
       w.sweep_alloc(sg.words(), s);
-      k_gs_pack<<<grid_for((long long)sg.size()), kThreads, 0, s>>>(sg, A, w.ci, b, x, w.gs(sg)); note_launch();
+      k_gs_pack<<<grid_for((long long)sg.all_rows() * kSweepCols), kThreads, 0, s>>>(sg, A, w.ci, b, x,
+                                                                                 w.march(sg, kGsPlanes)); note_launch();
     }
     k_it_init<<<g, kThreads, 0, s>>>(A, x, b, w.r.p, st, red.slot_part(0), red.slot_count(0),
                                      solver == 4 ? 1 : 0); note_launch();
@@ -1280,14 +1274,14 @@ static void ic_apply(const MatView<double> &A, int prec, RefKrylovWork &w, const
     return;
   }
   const SweepGeo g = SweepGeo::make(A.nx, A.ny, A.nz, sweep_a(prec));
-  const IcFactor M = w.ic(prec, g);
+  double *M = w.march(g, ic_planes(prec));
   const int n = g.tiles();
   if (prec == 2) {
-    k_ic_sweep<2, false><<<n, kSweepCols, 0, s>>>(g, M, r, w.zm.p, z, w.sweep(), st);
-    k_ic_sweep<2, true><<<n, kSweepCols, 0, s>>>(g, M, r, w.zm.p, z, w.sweep(), st);
+    k_ic_sweep<2, false><<<n, kSweepThreads, 0, s>>>(g, M, r, z, w.sweep(), st);
+    k_ic_sweep<2, true><<<n, kSweepThreads, 0, s>>>(g, M, r, z, w.sweep(), st);
   } else {
-    k_ic_sweep<1, false><<<n, kSweepCols, 0, s>>>(g, M, r, w.zm.p, z, w.sweep(), st);
-    k_ic_sweep<1, true><<<n, kSweepCols, 0, s>>>(g, M, r, w.zm.p, z, w.sweep(), st);
+    k_ic_sweep<1, false><<<n, kSweepThreads, 0, s>>>(g, M, r, z, w.sweep(), st);
+    k_ic_sweep<1, true><<<n, kSweepThreads, 0, s>>>(g, M, r, z, w.sweep(), st);
   }
   note_launch(); note_launch();
 }
@@ -1306,7 +1300,7 @@ void enqueue_ref_iters(const MatView<double> &A, double *x, int solver, int coun
     const SweepGeo sg = SweepGeo::make(A.nx, A.ny, A.nz, sweep_a(1));
     for (int it = 0; it < count; ++it) {
       if (gs && !A.per) {
-        k_gs_sweep<<<sg.tiles(), kSweepCols, 0, s>>>(sg, w.gs(sg), x, w.sweep(), st); note_launch();
+        k_gs_sweep<<<sg.tiles(), kSweepThreads, 0, s>>>(sg, w.march(sg, kGsPlanes), x, w.sweep(), st); note_launch();
       } else if (gs) {
         // the halo the exchange fills before each sweep
         if (w.xold.n < (size_t)N) w.xold.alloc(N);

@@ -31,9 +31,8 @@ struct RefKrylovWork {
   DBuf<double> mcd;                               // 1 / c (the diagonal preconditioner)
   DBuf<double> xold;                              // Gauss-Seidel: x before the sweep (periodic)
   const double *rhs = nullptr, *ci = nullptr;     // Jacobi / Gauss-Seidel operands of a solve
-  DBuf<double> z, mc, mw, ms, mb, mtw, mts, mnw;  // IC preconditioner
-  DBuf<double> my, zm;                            // IC0/IC2: 1 / mc and z in march order
-  DBuf<double> go[9];                             // Gauss-Seidel operands in march order
+  DBuf<double> z, mc, mw, ms, mb, mtw, mts, mnw;  // IC preconditioner: z, and IC3's factor
+  DBuf<double> mo;                                // sweeps: operands in march order
   DBuf<SweepWord> words;                          // sweeps: exchange between tiles
   DBuf<unsigned> ticket;                          // sweeps: tickets [0..1], the stuck flag [2]
   unsigned long long epoch = 0;                   // sweeps: the last launch's epoch
@@ -41,8 +40,7 @@ struct RefKrylovWork {
   ~RefKrylovWork();
   void ensure(size_t n, int solver);
   Ic3Factor ic3(size_t n);
-  IcFactor ic(int kind, const SweepGeo &g);
-  GsOps gs(const SweepGeo &g);
+  double *march(const SweepGeo &g, int planes);
   void sweep_alloc(size_t words_needed, cudaStream_t s);
   SweepSync sweep() {
     return {words.p, ticket.p, reinterpret_cast<int *>(ticket.p + 2), ++epoch};

@@ -16,15 +16,18 @@ __device__ __forceinline__ void sweep_st(SweepWord *p, double v, unsigned long l
                :: "l"(p), "l"((unsigned long long)__double_as_longlong(v)), "l"(epoch) : "memory");
 }
 
-// a / c with c's stored reciprocal (KnownDiv with its range check kept in y)
+// a / c with c's stored reciprocal y: KnownDiv with its range checks on the
+// exponents, beside the dependent operations instead of before them. A zero
+// dividend comes out right for +0 only; everything else outside the range,
+// and a NaN y, takes the division itself.
 __device__ __forceinline__ double sweep_div(double a, double c, double y) {
-  const double m = fabs(a);
-  if (m > 0x1p-900 && m < 0x1p900 && y == y) {
-    const double q0 = __dmul_rn(a, y);
-    return __fma_rn(__fma_rn(-q0, c, a), y, q0);
-  }
-  if (m == 0.0 && y == y) return __dmul_rn(a, c);
-  return __ddiv_rn(a, c);
+  const unsigned ea = ((unsigned)__double2hiint(a) >> 20) & 0x7ffu;
+  const unsigned ey = ((unsigned)__double2hiint(y) >> 20) & 0x7ffu;
+  const bool in = ea - (1023u - 899u) < 1799u || __double_as_longlong(a) == 0;   // 2^-899 <= |a| < 2^900
+  const double q0 = __dmul_rn(a, y);
+  double q = __fma_rn(__fma_rn(-q0, c, a), y, q0);
+  if (!in || ey == 0x7ffu) q = __ddiv_rn(a, c);
+  return q;
 }
 
 __device__ __forceinline__ double msub(double s, double a, double b) { return __dsub_rn(s, __dmul_rn(a, b)); }
@@ -42,31 +45,36 @@ __device__ __forceinline__ void sweep_finish(const SweepSync &y, int tiles) {
   if (atomicAdd(&y.ticket[1], 1u) == (unsigned)tiles - 1) { y.ticket[0] = 0; y.ticket[1] = 0; }
 }
 
-// The word p of this launch's epoch: w as loaded early, polled until valid.
-// A poll that runs out (or one that did elsewhere) sets *stuck and goes on
-// with zero, so that every block ends; the host reports the failure.
-__device__ __forceinline__ double sweep_wait(SweepWord w, const SweepWord *p, const SweepSync &y, bool &dead) {
-  if (w.epoch != y.epoch) {
-    for (int n = 1; !dead; ++n) {
-      w = sweep_ld(p);
-      if (w.epoch == y.epoch) break;
-      if (n >= kSweepPoll) { atomicExch(y.stuck, 1); dead = true; }
-      else if ((n & 1023) == 0 && *(volatile int *)y.stuck) dead = true;
-    }
-    if (w.epoch != y.epoch) return 0.0;
+// Waits until word p carries this launch's epoch and returns it. A poll that
+// runs out (or one that did elsewhere) sets *stuck and gives up with zero, so
+// that every block ends; the host reports the failure.
+__device__ __noinline__ SweepWord sweep_poll(const SweepWord *p, const SweepSync &y, bool &dead) {
+  SweepWord a = {0ull, 0ull};
+  for (int m = 1; !dead; ++m) {
+    a = sweep_ld(p);
+    if (a.epoch == y.epoch) break;
+    if (m >= kSweepPoll) { atomicExch(y.stuck, 1); dead = true; }
+    else if ((m & 1023) == 0 && *(volatile int *)y.stuck) dead = true;
+    a.v = 0ull;
   }
-  return __longlong_as_double((long long)w.v);
+  return a;
 }
 
-// Position of a thread in the march. In a backward sweep i, j and k run
+// 8 bytes to shared memory, completion by groups: the loads of later steps
+// stay in flight while an earlier step's are waited for
+__device__ __forceinline__ void sweep_copy(double *dst, const double *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;"
+               :: "r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+
+// Position of a column in the march. In a backward sweep i, j and k run
 // down: li, lj, kk and the tile indices count in march direction.
 template <bool BWD>
 struct SweepPos {
   int I, J, li, lj, i, j;
   bool col, hasW, hasS;   // the column, and those before it along i and along j, exist
-  __device__ __forceinline__ SweepPos(const SweepGeo &g, int tile) {
+  __device__ __forceinline__ SweepPos(const SweepGeo &g, int tile, int li_, int lj_) : li(li_), lj(lj_) {
     I = tile / g.tj; J = tile - I * g.tj;
-    li = threadIdx.x / kSweepTile; lj = threadIdx.x % kSweepTile;
     const int mi = I * kSweepTile + li, mj = J * kSweepTile + lj;
     i = BWD ? g.ti * kSweepTile - 1 - mi : mi;
     j = BWD ? g.tj * kSweepTile - 1 - mj : mj;
@@ -77,94 +85,206 @@ struct SweepPos {
   __device__ __forceinline__ int at(const SweepGeo &g, int kk) const { return BWD ? g.nz - 1 - kk : kk; }
 };
 
-// z = M^-1 r, one of its two triangular sweeps: forward
-// z = (r - lower terms) / c from r (natural order) into zm (march order),
-// backward z = (zm - upper terms) / c into z (natural order)
+// The march of one tile. Warps 0 and 1 hold a column a thread and do the
+// arithmetic (Body); warp 2 brings the columns beside the tile from the
+// exchange into the halo of the shared ring, a block of kSweepAhead steps
+// before they are read; warp 3 publishes the tile's last columns, one step
+// after they are formed. So a step of the arithmetic warps is shared loads,
+// the dependent operations and a barrier, whatever the exchange does. The
+// operands of a step are copied to shared memory asynchronously kSweepAhead
+// steps early (loads into registers would wait for each other: a warp has
+// few load counters). NV values a cell travel; a column beside a cell is
+// read at the cell's kk + LOOK.
+template <int NV, int A, int LOOK, bool BWD, class Body, class... Arg>
+__device__ __forceinline__ void sweep_march(const SweepGeo &g, const SweepSync &y, const Arg &...arg) {
+  constexpr int P = kSweepAhead, E = kSweepTile + 1, SLOT = NV * E * E, NP = Body::planes;
+  __shared__ double ring[2 * P][SLOT];   // values formed at a step; halo: values read at the next
+  __shared__ double stage[P][NP][kSweepCols];
+  const int tile = sweep_ticket(y);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nz = g.nz;
+  const int T = (nz + 2 * A * (kSweepTile - 1) + LOOK + P - 1) / P * P;
+  // a step: arithmetic warps and warp 3; a block of steps: those and warp 2
+  auto step_barrier = [] { asm volatile("bar.sync 1, %0;" ::"n"(kSweepCols + 32) : "memory"); };
+  auto block_barrier = [] { asm volatile("bar.sync 2, %0;" ::"n"(kSweepCols + 32) : "memory"); };
+  // lanes 0-7 of warps 2 and 3: the columns along i's edge, 8-15: along j's
+  const bool along_i = lane < kSweepTile, used = lane < 2 * kSweepTile;
+  const int m = lane % kSweepTile, last = kSweepTile - 1;
+  if (warp == 2) {
+    const SweepPos<BWD> q(g, tile, along_i ? 0 : m, along_i ? m : 0);
+    const bool on = used && (along_i ? q.hasW : q.hasS);
+    const SweepWord *p = along_i ? y.words + ((size_t)(q.I - 1) * g.ny + q.j) * nz
+                                 : y.words + g.words_i() + ((size_t)(q.J - 1) * g.nx + q.i) * nz;
+    const int at = along_i ? m + 1 : (m + 1) * E;
+    int ke = -A * m;   // the beside column's k of the block's first read
+    bool dead = false;
+    for (int t0 = 0; t0 < T; t0 += P, ke += P) {
+      // halo for the reads of steps t0 .. t0 + P - 1, in the slots before them
+      const int slot0 = (t0 + 2 * P - 1) % (2 * P);
+      SweepWord w[P][NV];
+      auto fetch = [&] {
+        bool ok = true;
+#pragma unroll
+        for (int u = 0; u < P; ++u)
+#pragma unroll
+          for (int v = 0; v < NV; ++v)
+            if (on && (unsigned)(ke + u) < (unsigned)nz) w[u][v] = sweep_ld(p + ke + u + v * g.words());
+#pragma unroll
+        for (int u = 0; u < P; ++u)
+#pragma unroll
+          for (int v = 0; v < NV; ++v)
+            if (on && (unsigned)(ke + u) < (unsigned)nz && w[u][v].epoch != y.epoch) ok = false;
+        return ok;
+      };
+      if (!fetch()) {   // caught up with the neighbour: wait for the block's last word first
+        sweep_poll(p + min(ke + P, nz) - 1 + (NV - 1) * g.words(), y, dead);
+        fetch();
+      }
+#pragma unroll
+      for (int u = 0; u < P; ++u)
+#pragma unroll
+        for (int v = 0; v < NV; ++v)
+          if (on && (unsigned)(ke + u) < (unsigned)nz) {
+            if (w[u][v].epoch != y.epoch) w[u][v] = sweep_poll(p + ke + u + v * g.words(), y, dead);
+            ring[(slot0 + u) % (2 * P)][v * E * E + at] = __longlong_as_double((long long)w[u][v].v);
+          }
+      block_barrier();
+    }
+  } else if (warp == 3) {
+    const SweepPos<BWD> q(g, tile, along_i ? last : m, along_i ? m : last);
+    const int start = -A * (last + m) - LOOK;
+    const bool on = used && q.col;
+    const int at = (q.li + 1) * E + q.lj + 1;
+    SweepWord *p = (along_i ? y.words + ((size_t)q.I * g.ny + q.j) * nz
+                            : y.words + g.words_i() + ((size_t)q.J * g.nx + q.i) * nz) + start;
+    for (int t0 = 0, h = 0; t0 < T; t0 += P, h ^= P) {
+#pragma unroll
+      for (int u = 0; u < P; ++u) {
+        step_barrier();
+        if (on && (unsigned)(start + t0 + u) < (unsigned)nz)
+#pragma unroll
+          for (int v = 0; v < NV; ++v) sweep_st(p + u + v * g.words(), ring[h + u][v * E * E + at], y.epoch);
+      }
+      p += P;
+    }
+  } else {
+    const SweepPos<BWD> q(g, tile, (int)threadIdx.x / kSweepTile, (int)threadIdx.x % kSweepTile);
+    const int start = -A * (q.li + q.lj) - LOOK, at = (q.li + 1) * E + q.lj + 1;
+    double *mine = &stage[0][0][threadIdx.x];
+    Body b(g, q, start, arg...);
+    auto load = [&](int u, int kk) {
+      if (q.col && (unsigned)kk < (unsigned)nz) b.load(u, kk, mine + u * (NP * kSweepCols));
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    auto fetch = [&](int u) {   // the operands of the step of slot u into registers
+      asm volatile("cp.async.wait_group %0;" ::"n"(P - 1) : "memory");
+      b.fetch(mine + u * (NP * kSweepCols));
+    };
+#pragma unroll
+    for (int u = 0; u < P; ++u) load(u, start + u);
+    b.ahead();
+    fetch(0);
+    double *cur = &ring[0][at], *oth = &ring[P][at];   // this block's slots and the other half
+    for (int kk = start, t0 = 0; t0 < T; t0 += P, kk += P) {
+      block_barrier();
+#pragma unroll
+      for (int u = 0; u < P; ++u) {
+        const double *prev = u > 0 ? cur + (u - 1) * SLOT : oth + (P - 1) * SLOT;
+        double w[NV], s[NV], o[NV];
+#pragma unroll
+        for (int v = 0; v < NV; ++v) { w[v] = prev[v * E * E - E]; s[v] = prev[v * E * E - 1]; }
+        b.before(w, s);
+        if (q.col && (unsigned)(kk + u) < (unsigned)nz) {
+          b.step(u, kk + u, w, s, o);
+#pragma unroll
+          for (int v = 0; v < NV; ++v) cur[u * SLOT + v * E * E] = o[v];
+        }
+        b.after(w, s);
+        load(u, kk + u + P);
+        fetch((u + 1) % P);
+        step_barrier();
+      }
+      b.next();
+      double *tmp = cur; cur = oth; oth = tmp;
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+  }
+  sweep_finish(y, g.tiles());
+}
+
+// Body of a triangular sweep of z = M^-1 r: forward z = (r - lower terms) / c
+// from r (natural order) into the factor's z plane, backward
+// z = (that - upper terms) / c into z (natural order)
 // (preconditioner_solve.cpp:14-110). Terms with a neighbour outside the
 // domain are skipped (the reference multiplies them by its zero halo).
 template <int KIND, bool BWD>
-__global__ void __launch_bounds__(kSweepCols) k_ic_sweep(SweepGeo g, IcFactor M, const double *__restrict__ r,
-                                                         double *__restrict__ zm, double *__restrict__ z,
-                                                         SweepSync y, const KrylovState *st) {
-  if (st->done) return;
-  constexpr int A = sweep_a(KIND), P = kSweepAhead, LOOK = KIND == 2 ? 1 : 0;
-  __shared__ double ring[2][kSweepCols];
-  const SweepPos<BWD> q(g, sweep_ticket(y));
-  const int me = threadIdx.x, skew = A * (q.li + q.lj) + LOOK, nz = g.nz;
-  const long long nat = ((long long)q.i * g.ny + q.j) * nz;
+struct IcBody {
+  static constexpr int P = kSweepAhead, NP = ic_planes(KIND), C = kSweepCols, planes = NP;
+  static constexpr int S = (BWD ? -1 : 1) * NP * C, D = BWD ? -1 : 1;   // a step in march and natural order
   // coefficient rows: the cell's own (forward), or those of the neighbour
   // whose lower entry is this cell's upper one (backward)
-  const size_t oO = q.col ? g.off(q.i, q.j) : 0;
-  const size_t oW = BWD && q.hasW ? g.off(q.i + 1, q.j) : oO;
-  const size_t oS = BWD && q.hasS ? g.off(q.i, q.j + 1) : oO;
-  constexpr int back = BWD ? kSweepCols : 0;
-  // columns read from, and published to, the tiles beside this one
-  const bool exW = q.hasW && q.li == 0, exS = q.hasS && q.lj == 0;
-  const bool putI = q.col && q.li == kSweepTile - 1, putJ = q.col && q.lj == kSweepTile - 1;
-  SweepWord *pi = y.words + ((size_t)q.I * g.ny + q.j) * nz;
-  SweepWord *pj = y.words + g.words_i() + ((size_t)q.J * g.nx + q.i) * nz;
-  const SweepWord *wi = pi - (size_t)g.ny * nz, *wj = pj - (size_t)g.nx * nz;
-  double cw[P], ctw[P], cs[P], cts[P], cb[P], cc[P], cy[P], cr[P];
-  SweepWord eW[P], eS[P];
-  auto load = [&](int u, int t) {
-    const int kk = t - skew, ke = kk + LOOK;
-    if (q.col && kk >= 0 && kk < nz) {
-      const int k = q.at(g, kk);
-      const size_t ko = (size_t)k * kSweepCols;
-      cc[u] = M.c[oO + ko];
-      cy[u] = M.y[oO + ko];
-      cr[u] = BWD ? zm[oO + ko] : r[nat + k];
-      if (q.hasW) cw[u] = M.w[oW + ko];
-      if (q.hasS) cs[u] = M.s[oS + ko];
-      if (kk > 0) cb[u] = M.b[oO + ko + back];
-      if constexpr (KIND == 2) {
-        if (kk + 1 < nz && q.hasW) ctw[u] = M.tw[oW + ko - back];
-        if (kk + 1 < nz && q.hasS) cts[u] = M.ts[oS + ko - back];
-      }
-    }
-    if (exW && ke >= 0 && ke < nz) eW[u] = sweep_ld(wi + ke);
-    if (exS && ke >= 0 && ke < nz) eS[u] = sweep_ld(wj + ke);
-  };
-#pragma unroll
-  for (int u = 0; u < P; ++u) load(u, u);
-  const int T = nz + 2 * A * (kSweepTile - 1) + LOOK;
-  double zB = 0.0, zW0 = 0.0, zS0 = 0.0;
-  bool dead = false;
-  for (int t0 = 0; t0 < T; t0 += P) {
-#pragma unroll
-    for (int u = 0; u < P; ++u) {
-      const int t = t0 + u;
-      if (t >= T) break;
-      const int kk = t - skew, ke = kk + LOOK;
-      double zW1 = 0.0, zS1 = 0.0;   // the columns beside, at kk + LOOK
-      if (ke >= 0 && ke < nz) {
-        if (exW) zW1 = sweep_wait(eW[u], wi + ke, y, dead);
-        else if (q.hasW) zW1 = ring[(t - 1) & 1][me - kSweepTile];
-        if (exS) zS1 = sweep_wait(eS[u], wj + ke, y, dead);
-        else if (q.hasS) zS1 = ring[(t - 1) & 1][me - 1];
-      }
-      if constexpr (LOOK == 0) { zW0 = zW1; zS0 = zS1; }
-      if (q.col && kk >= 0 && kk < nz) {
-        double sum = cr[u];
-        if (q.hasW) sum = msub(sum, cw[u], zW0);
-        if (KIND == 2 && q.hasW && kk + 1 < nz) sum = msub(sum, ctw[u], zW1);
-        if (q.hasS) sum = msub(sum, cs[u], zS0);
-        if (KIND == 2 && q.hasS && kk + 1 < nz) sum = msub(sum, cts[u], zS1);
-        if (kk > 0) sum = msub(sum, cb[u], zB);
-        zB = sweep_div(sum, cc[u], cy[u]);
-        ring[t & 1][me] = zB;
-        if (putI) sweep_st(pi + kk, zB, y.epoch);
-        if (putJ) sweep_st(pj + kk, zB, y.epoch);
-        const int k = q.at(g, kk);
-        if (BWD) z[nat + k] = zB;
-        else zm[oO + (size_t)k * kSweepCols] = zB;
-      }
-      if constexpr (LOOK == 1) { zW0 = zW1; zS0 = zS1; }
-      load(u, t + P);
-      __syncthreads();
+  const double *lO, *lW, *lS, *lr;
+  double *zO, *lz;
+  int nz;
+  bool hasW, hasS;
+  double cw, ctw, cs, cts, cb, cc, cy, cr;
+  double zB, zW0, zS0;
+  __device__ __forceinline__ IcBody(const SweepGeo &g, const SweepPos<BWD> &q, int start, double *M, const double *r,
+                                    double *z)
+      : nz(g.nz), hasW(q.hasW), hasS(q.hasS), zB(0.0), zW0(0.0), zS0(0.0) {
+    const long long row = (long long)q.at(g, start) * (NP * C);
+    const long long nat = ((long long)q.i * g.ny + q.j) * nz + q.at(g, start);
+    lO = zO = M + ((long long)(q.col ? g.off(q.i, q.j, NP) : 0) + row);
+    lW = BWD && hasW ? M + ((long long)g.off(q.i + 1, q.j, NP) + row) : lO;
+    lS = BWD && hasS ? M + ((long long)g.off(q.i, q.j + 1, NP) + row) : lO;
+    lr = r + nat;
+    lz = z + nat;
+  }
+  __device__ __forceinline__ void load(int u, int kk, double *d) {
+    const int o = u * S;
+    sweep_copy(d + kIcC * C, lO + o + kIcC * C);
+    sweep_copy(d + kIcY * C, lO + o + kIcY * C);
+    sweep_copy(d + kIcZ * C, BWD ? lO + o + kIcZ * C : lr + u);
+    if (!BWD || hasW) sweep_copy(d + kIcW * C, lW + o + kIcW * C);
+    if (!BWD || hasS) sweep_copy(d + kIcS * C, lS + o + kIcS * C);
+    if (!BWD || kk > 0) sweep_copy(d + kIcB * C, lO + o + kIcB * C - (BWD ? S : 0));
+    if constexpr (KIND == 2) {
+      if (!BWD || (hasW && kk + 1 < nz)) sweep_copy(d + kIcTw * C, lW + o + kIcTw * C + (BWD ? S : 0));
+      if (!BWD || (hasS && kk + 1 < nz)) sweep_copy(d + kIcTs * C, lS + o + kIcTs * C + (BWD ? S : 0));
     }
   }
-  sweep_finish(y, g.tiles());
+  __device__ __forceinline__ void fetch(const double *d) {
+    cc = d[kIcC * C]; cy = d[kIcY * C]; cr = d[kIcZ * C];
+    cw = d[kIcW * C]; cs = d[kIcS * C]; cb = d[kIcB * C];
+    if constexpr (KIND == 2) { ctw = d[kIcTw * C]; cts = d[kIcTs * C]; }
+  }
+  __device__ __forceinline__ void ahead() { lO += P * S; lW += P * S; lS += P * S; lr += P * D; }
+  __device__ __forceinline__ void next() { ahead(); zO += P * S; lz += P * D; }
+  __device__ __forceinline__ void before(const double *w, const double *s) {
+    if constexpr (KIND == 1) { zW0 = w[0]; zS0 = s[0]; }
+  }
+  __device__ __forceinline__ void after(const double *w, const double *s) {
+    if constexpr (KIND == 2) { zW0 = w[0]; zS0 = s[0]; }
+  }
+  __device__ __forceinline__ void step(int u, int kk, const double *w, const double *s, double *o) {
+    double sum = cr;
+    if (hasW) sum = msub(sum, cw, zW0);
+    if (KIND == 2 && hasW && kk + 1 < nz) sum = msub(sum, ctw, w[0]);
+    if (hasS) sum = msub(sum, cs, zS0);
+    if (KIND == 2 && hasS && kk + 1 < nz) sum = msub(sum, cts, s[0]);
+    if (kk > 0) sum = msub(sum, cb, zB);
+    zB = sweep_div(sum, cc, cy);
+    o[0] = zB;
+    if (BWD) lz[u * D] = zB;
+    else zO[u * S + kIcZ * C] = zB;
+  }
+};
+
+template <int KIND, bool BWD>
+__global__ void __launch_bounds__(kSweepThreads) k_ic_sweep(SweepGeo g, double *M, const double *__restrict__ r,
+                                                            double *__restrict__ z, SweepSync y,
+                                                            const KrylovState *st) {
+  if (st->done) return;
+  sweep_march<1, sweep_a(KIND), KIND == 2 ? 1 : 0, BWD, IcBody<KIND, BWD>>(g, y, M, r, z);
 }
 
 // IncompleteCholesky0/2::form (preconditioner_form.cpp:16-98) in march
@@ -177,97 +297,71 @@ __global__ void __launch_bounds__(kSweepCols) k_ic_sweep(SweepGeo g, IcFactor M,
 // so only c and b travel between columns. Entries whose p lies outside the
 // domain are zero.
 template <int KIND>
-__global__ void __launch_bounds__(kSweepCols) k_ic_factor(SweepGeo g, MatView<double> A, IcFactor M, SweepSync y) {
-  constexpr int W = sweep_a(KIND), P = kSweepAhead, LOOK = KIND == 2 ? 1 : 0;
-  __shared__ double rc[2][kSweepCols], rb[2][kSweepCols];
-  const SweepPos<false> q(g, sweep_ticket(y));
-  const int me = threadIdx.x, skew = W * (q.li + q.lj) + LOOK, nz = g.nz;
-  const long long nat = ((long long)q.i * g.ny + q.j) * nz;
-  const size_t oO = q.col ? g.off(q.i, q.j) : 0;
-  const bool exW = q.hasW && q.li == 0, exS = q.hasS && q.lj == 0;
-  const bool putI = q.col && q.li == kSweepTile - 1, putJ = q.col && q.lj == kSweepTile - 1;
-  SweepWord *pi = y.words + ((size_t)q.I * g.ny + q.j) * nz;
-  SweepWord *pj = y.words + g.words_i() + ((size_t)q.J * g.nx + q.i) * nz;
-  const SweepWord *wi = pi - (size_t)g.ny * nz, *wj = pj - (size_t)g.nx * nz;
-  const size_t vb = g.words();   // the words of b follow those of c
-  double ac[P], aw[P], as[P], ab[P];
-  SweepWord eW[P], eWb[P], eS[P], eSb[P];
-  auto load = [&](int u, int t) {
-    const int kk = t - skew, ke = kk + LOOK;
-    if (q.col && kk >= 0 && kk < nz) {
-      ac[u] = A.c[nat + kk]; aw[u] = A.w[nat + kk]; as[u] = A.s[nat + kk]; ab[u] = A.b[nat + kk];
-    }
-    if (exW && ke >= 0 && ke < nz) { eW[u] = sweep_ld(wi + ke); if (KIND == 2) eWb[u] = sweep_ld(wi + vb + ke); }
-    if (exS && ke >= 0 && ke < nz) { eS[u] = sweep_ld(wj + ke); if (KIND == 2) eSb[u] = sweep_ld(wj + vb + ke); }
-  };
-  // c and b of a column beside this one at ke
-  auto beside = [&](const SweepWord &wc, const SweepWord &wb, const SweepWord *w, bool ex, int from, int t, int ke,
-                    bool &dead, double &c, double &b) {
-    if (ex) {
-      c = sweep_wait(wc, w + ke, y, dead);
-      if (KIND == 2) b = sweep_wait(wb, w + vb + ke, y, dead);
-    } else {
-      c = rc[(t - 1) & 1][from];
-      if (KIND == 2) b = rb[(t - 1) & 1][from];
-    }
-  };
-#pragma unroll
-  for (int u = 0; u < P; ++u) load(u, u);
-  const int T = nz + 2 * W * (kSweepTile - 1) + LOOK;
-  double cB = 0.0, twB = 0.0, tsB = 0.0;   // of the cell before along k
-  double cW0 = 0.0, cS0 = 0.0;
-  bool dead = false;
-  for (int t0 = 0; t0 < T; t0 += P) {
-#pragma unroll
-    for (int u = 0; u < P; ++u) {
-      const int t = t0 + u;
-      if (t >= T) break;
-      const int kk = t - skew, ke = kk + LOOK;
-      double cW1 = 0.0, bW1 = 0.0, cS1 = 0.0, bS1 = 0.0;
-      if (ke >= 0 && ke < nz) {
-        if (q.hasW) beside(eW[u], eWb[u], wi, exW, me - kSweepTile, t, ke, dead, cW1, bW1);
-        if (q.hasS) beside(eS[u], eSb[u], wj, exS, me - 1, t, ke, dead, cS1, bS1);
-      }
-      if constexpr (LOOK == 0) { cW0 = cW1; cS0 = cS1; }
-      if (q.col && kk >= 0 && kk < nz) {
-        const double w = q.hasW ? __ddiv_rn(-aw[u], cW0) : 0.0;
-        const double s = q.hasS ? __ddiv_rn(-as[u], cS0) : 0.0;
-        double tw = 0.0, ts = 0.0, b = 0.0;
-        if (KIND == 2 && q.hasW && kk + 1 < nz) tw = __ddiv_rn(__dmul_rn(-w, bW1), cW1);
-        if (KIND == 2 && q.hasS && kk + 1 < nz) ts = __ddiv_rn(__dmul_rn(-s, bS1), cS1);
-        if (kk > 0) {
-          double n = -ab[u];
-          if (KIND == 2) n = msub(msub(n, w, twB), s, tsB);
-          b = __ddiv_rn(n, cB);
-        }
-        double c = msub(ac[u], w, w);
-        if (KIND == 2) c = msub(c, tw, tw);
-        c = msub(c, s, s);
-        if (KIND == 2) c = msub(c, ts, ts);
-        c = __dsqrt_rn(msub(c, b, b));
-        rc[t & 1][me] = c;
-        rb[t & 1][me] = b;
-        if (putI) { sweep_st(pi + kk, c, y.epoch); if (KIND == 2) sweep_st(pi + vb + kk, b, y.epoch); }
-        if (putJ) { sweep_st(pj + kk, c, y.epoch); if (KIND == 2) sweep_st(pj + vb + kk, b, y.epoch); }
-        const size_t o = oO + (size_t)kk * kSweepCols;
-        M.c[o] = c;
-        M.y[o] = KnownDiv(c).recip();
-        M.w[o] = w; M.s[o] = s; M.b[o] = b;
-        if (KIND == 2) { M.tw[o] = tw; M.ts[o] = ts; }
-        cB = c; twB = tw; tsB = ts;
-      }
-      if constexpr (LOOK == 1) { cW0 = cW1; cS0 = cS1; }
-      load(u, t + P);
-      __syncthreads();
-    }
+struct IcFormBody {
+  static constexpr int P = kSweepAhead, NP = ic_planes(KIND), C = kSweepCols, planes = 4;
+  const double *ac, *aw, *as, *ab;
+  double *o_;
+  int nz;
+  bool hasW, hasS;
+  double rc, rw, rs, rb;
+  double cB, twB, tsB, cW0, cS0;
+  __device__ __forceinline__ IcFormBody(const SweepGeo &g, const SweepPos<false> &q, int start,
+                                        const MatView<double> &A, double *M)
+      : nz(g.nz), hasW(q.hasW), hasS(q.hasS), cB(0.0), twB(0.0), tsB(0.0), cW0(0.0), cS0(0.0) {
+    const long long nat = ((long long)q.i * g.ny + q.j) * nz + start;
+    ac = A.c + nat; aw = A.w + nat; as = A.s + nat; ab = A.b + nat;
+    o_ = M + ((long long)(q.col ? g.off(q.i, q.j, NP) : 0) + (long long)start * (NP * C));
   }
-  sweep_finish(y, g.tiles());
+  __device__ __forceinline__ void load(int u, int, double *d) {
+    sweep_copy(d, ac + u); sweep_copy(d + C, aw + u); sweep_copy(d + 2 * C, as + u); sweep_copy(d + 3 * C, ab + u);
+  }
+  __device__ __forceinline__ void fetch(const double *d) { rc = d[0]; rw = d[C]; rs = d[2 * C]; rb = d[3 * C]; }
+  __device__ __forceinline__ void ahead() { ac += P; aw += P; as += P; ab += P; }
+  __device__ __forceinline__ void next() { ahead(); o_ += P * NP * C; }
+  __device__ __forceinline__ void before(const double *w, const double *s) {
+    if constexpr (KIND == 1) { cW0 = w[0]; cS0 = s[0]; }
+  }
+  __device__ __forceinline__ void after(const double *w, const double *s) {
+    if constexpr (KIND == 2) { cW0 = w[0]; cS0 = s[0]; }
+  }
+  // w, s: c and b of the columns beside at kk + LOOK
+  __device__ __forceinline__ void step(int u, int kk, const double *wv, const double *sv, double *out) {
+    const double w = hasW ? __ddiv_rn(-rw, cW0) : 0.0;
+    const double s = hasS ? __ddiv_rn(-rs, cS0) : 0.0;
+    double tw = 0.0, ts = 0.0, b = 0.0;
+    if constexpr (KIND == 2) {
+      if (hasW && kk + 1 < nz) tw = __ddiv_rn(__dmul_rn(-w, wv[1]), wv[0]);
+      if (hasS && kk + 1 < nz) ts = __ddiv_rn(__dmul_rn(-s, sv[1]), sv[0]);
+    }
+    if (kk > 0) {
+      double n = -rb;
+      if (KIND == 2) n = msub(msub(n, w, twB), s, tsB);
+      b = __ddiv_rn(n, cB);
+    }
+    double c = msub(rc, w, w);
+    if (KIND == 2) c = msub(c, tw, tw);
+    c = msub(c, s, s);
+    if (KIND == 2) c = msub(c, ts, ts);
+    c = __dsqrt_rn(msub(c, b, b));
+    out[0] = c;
+    if constexpr (KIND == 2) out[1] = b;
+    double *o = o_ + u * (NP * C);
+    o[kIcC * C] = c;
+    o[kIcY * C] = KnownDiv(c).recip();
+    o[kIcW * C] = w; o[kIcS * C] = s; o[kIcB * C] = b;
+    if constexpr (KIND == 2) { o[kIcTw * C] = tw; o[kIcTs * C] = ts; }
+    cB = c; twB = tw; tsB = ts;
+  }
+};
+
+template <int KIND>
+__global__ void __launch_bounds__(kSweepThreads) k_ic_factor(SweepGeo g, MatView<double> A, double *M, SweepSync y) {
+  sweep_march<KIND == 2 ? 2 : 1, sweep_a(KIND), KIND == 2 ? 1 : 0, false, IcFormBody<KIND>>(g, y, A, M);
 }
 
-
 __global__ void k_gs_pack(SweepGeo g, MatView<double> A, const double *__restrict__ ci,
-                          const double *__restrict__ b, const double *__restrict__ x, GsOps o) {
-  const size_t n = g.size();
+                          const double *__restrict__ b, const double *__restrict__ x, double *o) {
+  const size_t n = g.all_rows() * kSweepCols;
   for (size_t m = blockIdx.x * (size_t)blockDim.x + threadIdx.x; m < n; m += (size_t)gridDim.x * blockDim.x) {
     const int c = (int)(m % kSweepCols);
     const size_t row = m / kSweepCols;
@@ -277,8 +371,10 @@ __global__ void k_gs_pack(SweepGeo g, MatView<double> A, const double *__restric
     if (i >= g.nx || j >= g.ny || k < 0 || k >= g.nz) continue;
     const long long p = ((long long)i * g.ny + j) * g.nz + k;
     const Nb<double> a = coeffs(A, p, Pos{i, j, k});
-    o.b[m] = b[p]; o.ci[m] = ci[p]; o.x[m] = x[p];
-    o.w[m] = a.w; o.e[m] = a.e; o.s[m] = a.s; o.n[m] = a.n; o.bt[m] = a.b; o.t[m] = a.t;
+    double *w = o + row * (kGsPlanes * kSweepCols) + c;
+    const double v[kGsPlanes] = {b[p], ci[p], a.w, a.e, a.s, a.n, a.b, a.t, x[p]};
+#pragma unroll
+    for (int f = 0; f < kGsPlanes; ++f) w[f * kSweepCols] = v[f];
   }
 }
 
@@ -288,73 +384,60 @@ __global__ void k_gs_pack(SweepGeo g, MatView<double> A, const double *__restric
 // old values are loaded before their cells' new ones are formed: those wait,
 // directly or through the exchange, for this cell's own result. A neighbour
 // outside the domain counts as zero.
-__global__ void __launch_bounds__(kSweepCols) k_gs_sweep(SweepGeo g, GsOps o, double *__restrict__ x, SweepSync y,
-                                                         const KrylovState *st) {
-  if (st->done) return;
-  constexpr int P = kSweepAhead;
-  __shared__ double ring[2][kSweepCols];
-  const SweepPos<false> q(g, sweep_ticket(y));
-  const int me = threadIdx.x, skew = q.li + q.lj, nz = g.nz;
-  const long long nat = ((long long)q.i * g.ny + q.j) * nz;
-  const size_t oO = q.col ? g.off(q.i, q.j) : 0;
-  const bool hasE = q.col && q.i + 1 < g.nx, hasN = q.col && q.j + 1 < g.ny;
-  const size_t oE = hasE ? g.off(q.i + 1, q.j) : oO, oN = hasN ? g.off(q.i, q.j + 1) : oO;
-  const bool exW = q.hasW && q.li == 0, exS = q.hasS && q.lj == 0;
-  const bool putI = q.col && q.li == kSweepTile - 1, putJ = q.col && q.lj == kSweepTile - 1;
-  SweepWord *pi = y.words + ((size_t)q.I * g.ny + q.j) * nz;
-  SweepWord *pj = y.words + g.words_i() + ((size_t)q.J * g.nx + q.i) * nz;
-  const SweepWord *wi = pi - (size_t)g.ny * nz, *wj = pj - (size_t)g.nx * nz;
-  double *xs = o.x;
-  double rb[P], rci[P], rw[P], re[P], rs[P], rn[P], rbt[P], rt[P], xe[P], xn[P], xt[P];
-  SweepWord eW[P], eS[P];
-  auto load = [&](int u, int t) {
-    const int kk = t - skew;
-    if (!q.col || kk < 0 || kk >= nz) return;
-    const size_t m = oO + (size_t)kk * kSweepCols;
-    rb[u] = o.b[m]; rci[u] = o.ci[m];
-    rw[u] = o.w[m]; re[u] = o.e[m]; rs[u] = o.s[m]; rn[u] = o.n[m]; rbt[u] = o.bt[m]; rt[u] = o.t[m];
-    xe[u] = hasE ? __ldcg(xs + oE + (size_t)kk * kSweepCols) : 0.0;
-    xn[u] = hasN ? __ldcg(xs + oN + (size_t)kk * kSweepCols) : 0.0;
-    xt[u] = kk + 1 < nz ? __ldcg(xs + m + kSweepCols) : 0.0;
-    if (exW) eW[u] = sweep_ld(wi + kk);
-    if (exS) eS[u] = sweep_ld(wj + kk);
-  };
-#pragma unroll
-  for (int u = 0; u < P; ++u) load(u, u);
-  const int T = nz + 2 * (kSweepTile - 1);
-  double xB = 0.0;
-  bool dead = false;
-  for (int t0 = 0; t0 < T; t0 += P) {
-#pragma unroll
-    for (int u = 0; u < P; ++u) {
-      const int t = t0 + u;
-      if (t >= T) break;
-      const int kk = t - skew;
-      if (q.col && kk >= 0 && kk < nz) {
-        double xW = 0.0, xS = 0.0;
-        if (exW) xW = sweep_wait(eW[u], wi + kk, y, dead);
-        else if (q.hasW) xW = ring[(t - 1) & 1][me - kSweepTile];
-        if (exS) xS = sweep_wait(eS[u], wj + kk, y, dead);
-        else if (q.hasS) xS = ring[(t - 1) & 1][me - 1];
-        double v = rb[u];
-        v = __dadd_rn(v, __dmul_rn(rw[u], xW));
-        v = __dadd_rn(v, __dmul_rn(re[u], xe[u]));
-        v = __dadd_rn(v, __dmul_rn(rs[u], xS));
-        v = __dadd_rn(v, __dmul_rn(rn[u], xn[u]));
-        v = __dadd_rn(v, __dmul_rn(rbt[u], xB));
-        v = __dadd_rn(v, __dmul_rn(rt[u], xt[u]));
-        xB = __dmul_rn(rci[u], v);
-        ring[t & 1][me] = xB;
-        if (putI) sweep_st(pi + kk, xB, y.epoch);
-        if (putJ) sweep_st(pj + kk, xB, y.epoch);
-        xs[oO + (size_t)kk * kSweepCols] = xB;
-        x[nat + kk] = xB;
-      }
-      load(u, t + P);
-      __syncthreads();
-    }
+struct GsBody {
+  static constexpr int P = kSweepAhead, C = kSweepCols, S = kGsPlanes * C, planes = kGsPlanes + 2;
+  const double *lO, *lE, *lN;
+  double *xO, *lx;
+  int nz;
+  bool hasW, hasS, hasE, hasN;
+  double rb, rci, rw, re, rs, rn, rbt, rt, xe, xn, xt;
+  double xB;
+  __device__ __forceinline__ GsBody(const SweepGeo &g, const SweepPos<false> &q, int start, double *M, double *x)
+      : nz(g.nz), hasW(q.hasW), hasS(q.hasS), hasE(q.col && q.i + 1 < g.nx), hasN(q.col && q.j + 1 < g.ny), xB(0.0) {
+    const long long row = (long long)start * S;
+    lO = M + ((long long)(q.col ? g.off(q.i, q.j, kGsPlanes) : 0) + row);
+    lE = hasE ? M + ((long long)g.off(q.i + 1, q.j, kGsPlanes) + row) : lO;
+    lN = hasN ? M + ((long long)g.off(q.i, q.j + 1, kGsPlanes) + row) : lO;
+    xO = const_cast<double *>(lO) + kGsX * C;
+    lx = x + (((long long)q.i * g.ny + q.j) * nz + start);
   }
-  sweep_finish(y, g.tiles());
+  // planes of a stage: the cell's eight operands, then the old x at i + 1, j + 1 and k + 1
+  __device__ __forceinline__ void load(int u, int kk, double *d) {
+    const double *l = lO + u * S;
+#pragma unroll
+    for (int f = 0; f < kGsX; ++f) sweep_copy(d + f * C, l + f * C);
+    if (hasE) sweep_copy(d + kGsX * C, lE + u * S + kGsX * C);
+    if (hasN) sweep_copy(d + (kGsX + 1) * C, lN + u * S + kGsX * C);
+    if (kk + 1 < nz) sweep_copy(d + (kGsX + 2) * C, l + kGsX * C + S);
+  }
+  __device__ __forceinline__ void fetch(const double *d) {
+    rb = d[kGsB * C]; rci = d[kGsCi * C];
+    rw = d[kGsW * C]; re = d[kGsE * C]; rs = d[kGsS * C]; rn = d[kGsN * C]; rbt = d[kGsBt * C]; rt = d[kGsT * C];
+    xe = d[kGsX * C]; xn = d[(kGsX + 1) * C]; xt = d[(kGsX + 2) * C];
+  }
+  __device__ __forceinline__ void ahead() { lO += P * S; lE += P * S; lN += P * S; }
+  __device__ __forceinline__ void next() { ahead(); xO += P * S; lx += P; }
+  __device__ __forceinline__ void before(const double *, const double *) {}
+  __device__ __forceinline__ void after(const double *, const double *) {}
+  __device__ __forceinline__ void step(int u, int kk, const double *w, const double *s, double *o) {
+    double v = rb;
+    v = __dadd_rn(v, __dmul_rn(rw, hasW ? w[0] : 0.0));
+    v = __dadd_rn(v, __dmul_rn(re, hasE ? xe : 0.0));
+    v = __dadd_rn(v, __dmul_rn(rs, hasS ? s[0] : 0.0));
+    v = __dadd_rn(v, __dmul_rn(rn, hasN ? xn : 0.0));
+    v = __dadd_rn(v, __dmul_rn(rbt, xB));
+    v = __dadd_rn(v, __dmul_rn(rt, kk + 1 < nz ? xt : 0.0));
+    xB = __dmul_rn(rci, v);
+    o[0] = xB;
+    xO[u * S] = xB;
+    lx[u] = xB;
+  }
+};
+
+__global__ void __launch_bounds__(kSweepThreads) k_gs_sweep(SweepGeo g, double *M, double *__restrict__ x, SweepSync y,
+                                                            const KrylovState *st) {
+  if (st->done) return;
+  sweep_march<1, 1, 0, false, GsBody>(g, y, M, x);
 }
 
 }  // namespace pbg

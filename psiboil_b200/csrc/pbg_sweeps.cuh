@@ -10,8 +10,8 @@
 // order gives each cell exactly the values of the sequential sweep, and the
 // arithmetic per cell is the reference's, in its order (no contraction).
 //
-// One block of 64 threads owns the 8 x 8 columns of a tile of the (i, j)
-// plane and marches along k: at step t thread (li, lj) is at
+// One block owns the 8 x 8 columns of a tile of the (i, j) plane, a thread
+// each, and marches along k: at step t thread (li, lj) is at
 // k = t - a (li + lj), so the values it needs from the columns beside it
 // were formed in the step before and come from shared memory. Values crossing a tile's edge go through global memory as 16-byte
 // (value, epoch) words written and read whole: a word is valid when it
@@ -25,8 +25,8 @@
 // plus about a microsecond for each tile edge on the way. One launch per
 // plane, the form before this, paid a launch for every step. All operands
 // that the sweeps own are stored in march order (SweepGeo::off), so that a
-// step's 64 loads are two contiguous rows, and are loaded kSweepAhead steps
-// early into registers.
+// step reads contiguous rows at constant offsets from one pointer, and are
+// loaded kSweepAhead steps early into registers.
 #pragma once
 
 #include "pbg_common.cuh"
@@ -35,7 +35,8 @@
 namespace pbg {
 
 constexpr int kSweepTile = 8;                            // columns of a tile per direction
-constexpr int kSweepCols = kSweepTile * kSweepTile;      // threads of a block
+constexpr int kSweepCols = kSweepTile * kSweepTile;      // columns of a tile, a thread each
+constexpr int kSweepThreads = kSweepCols + 64;           // and two warps for the exchange
 constexpr int kSweepAhead = 6;                           // steps an operand is loaded early
 constexpr int kSweepPoll = 1 << 22;                      // polls of one word before giving up
 // rows from which the march-order storage is skewed: below it the skew's
@@ -64,12 +65,14 @@ struct SweepGeo {
     return g;
   }
   __host__ __device__ int tiles() const { return ti * tj; }
-  __host__ __device__ size_t size() const { return (size_t)tiles() * rows * kSweepCols; }
-  // storage index of cell (i, j, 0); cell (i, j, k) is kSweepCols * k further
-  __device__ __forceinline__ size_t off(int i, int j) const {
+  __host__ __device__ size_t all_rows() const { return (size_t)tiles() * rows; }
+  // Storage: a row holds `planes` operands of its 64 cells one after the
+  // other. Index of operand 0 of cell (i, j, 0); the cell (i, j, k) is k
+  // rows further, the next operand kSweepCols further.
+  __device__ __forceinline__ size_t off(int i, int j, int planes) const {
     const int li = i % kSweepTile, lj = j % kSweepTile;
     const size_t tile = (size_t)(i / kSweepTile) * tj + j / kSweepTile;
-    return (tile * rows + skew * (li + lj)) * kSweepCols + li * kSweepTile + lj;
+    return (tile * rows + skew * (li + lj)) * planes * kSweepCols + li * kSweepTile + lj;
   }
   // words of one exchanged value: the tiles' last columns along i, then along j
   __host__ __device__ size_t words_i() const { return (size_t)ti * ny * nz; }
@@ -84,15 +87,12 @@ struct SweepSync {
   unsigned long long epoch;     // of this launch, larger than any before it
 };
 
-// Incomplete Cholesky factor in march order. y = 1 / c rounded, for the
-// division by c (NaN where KnownDiv's range does not hold).
-struct IcFactor {
-  double *c, *y, *w, *s, *b, *tw, *ts;
-};
-
-// Operands of the Gauss-Seidel sweeps of one solve in march order.
-struct GsOps {
-  double *b, *ci, *w, *e, *s, *n, *bt, *t, *x;
-};
+// Operands of a cell in march order. Incomplete Cholesky: the factor's c, the
+// rounded 1 / c for the division by it (NaN where KnownDiv's range does not
+// hold), w, s, b, the forward sweep's z, and for IC2 tw and ts.
+// Gauss-Seidel: right-hand side, ci, the six couplings and x.
+enum : int { kIcC, kIcY, kIcW, kIcS, kIcB, kIcZ, kIcTw, kIcTs };
+enum : int { kGsB, kGsCi, kGsW, kGsE, kGsS, kGsN, kGsBt, kGsT, kGsX, kGsPlanes };
+__host__ __device__ constexpr int ic_planes(int kind) { return kind == 2 ? 8 : 6; }
 
 }  // namespace pbg
