@@ -85,16 +85,15 @@ struct SweepPos {
   __device__ __forceinline__ int at(const SweepGeo &g, int kk) const { return BWD ? g.nz - 1 - kk : kk; }
 };
 
-// The march of one tile. Warps 0 and 1 hold a column a thread and do the
-// arithmetic (Body); warp 2 brings the columns beside the tile from the
-// exchange into the halo of the shared ring, a block of kSweepAhead steps
-// before they are read; warp 3 publishes the tile's last columns, one step
-// after they are formed. So a step of the arithmetic warps is shared loads,
-// the dependent operations and a barrier, whatever the exchange does. The
-// operands of a step are copied to shared memory asynchronously kSweepAhead
-// steps early (loads into registers would wait for each other: a warp has
-// few load counters). NV values a cell travel; a column beside a cell is
-// read at the cell's kk + LOOK.
+// The march of one tile. Warps 0 and 1 hold a column a thread and do nothing
+// but the dependent arithmetic of a step (Body::step). Warp 2 brings the
+// columns beside the tile from the exchange into the halo of the shared
+// ring, a block of kSweepAhead steps before they are read; warp 3 publishes
+// the tile's last columns, one step after they are formed; warps 4 and 5
+// copy the operands of later steps to shared memory (asynchronously: loads
+// into registers would wait for each other, a warp has few load counters)
+// and store the results one step after they are formed. NV values a cell
+// travel; a column beside a cell is read at the cell's kk + LOOK.
 template <int NV, int A, int LOOK, bool BWD, class Body, class... Arg>
 __device__ __forceinline__ void sweep_march(const SweepGeo &g, const SweepSync &y, const Arg &...arg) {
   constexpr int P = kSweepAhead, E = kSweepTile + 1, SLOT = NV * E * E, NP = Body::planes;
@@ -103,8 +102,8 @@ __device__ __forceinline__ void sweep_march(const SweepGeo &g, const SweepSync &
   const int tile = sweep_ticket(y);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nz = g.nz;
   const int T = (nz + 2 * A * (kSweepTile - 1) + LOOK + P - 1) / P * P;
-  // a step: arithmetic warps and warp 3; a block of steps: those and warp 2
-  auto step_barrier = [] { asm volatile("bar.sync 1, %0;" ::"n"(kSweepCols + 32) : "memory"); };
+  // every step: all but warp 2; a block of steps: warp 2 and the arithmetic warps
+  auto step_barrier = [] { asm volatile("bar.sync 1, %0;" ::"n"(kSweepThreads - 32) : "memory"); };
   auto block_barrier = [] { asm volatile("bar.sync 2, %0;" ::"n"(kSweepCols + 32) : "memory"); };
   // lanes 0-7 of warps 2 and 3: the columns along i's edge, 8-15: along j's
   const bool along_i = lane < kSweepTile, used = lane < 2 * kSweepTile;
@@ -156,7 +155,8 @@ __device__ __forceinline__ void sweep_march(const SweepGeo &g, const SweepSync &
     const int at = (q.li + 1) * E + q.lj + 1;
     SweepWord *p = (along_i ? y.words + ((size_t)q.I * g.ny + q.j) * nz
                             : y.words + g.words_i() + ((size_t)q.J * g.nx + q.i) * nz) + start;
-    for (int t0 = 0, h = 0; t0 < T; t0 += P, h ^= P) {
+    step_barrier();
+    for (int t0 = 0, h = 0; t0 < T; t0 += P, h = P - h) {
 #pragma unroll
       for (int u = 0; u < P; ++u) {
         step_barrier();
@@ -167,46 +167,63 @@ __device__ __forceinline__ void sweep_march(const SweepGeo &g, const SweepSync &
       p += P;
     }
   } else {
-    const SweepPos<BWD> q(g, tile, (int)threadIdx.x / kSweepTile, (int)threadIdx.x % kSweepTile);
+    const int col = threadIdx.x % kSweepCols;
+    const SweepPos<BWD> q(g, tile, col / kSweepTile, col % kSweepTile);
     const int start = -A * (q.li + q.lj) - LOOK, at = (q.li + 1) * E + q.lj + 1;
-    double *mine = &stage[0][0][threadIdx.x];
-    Body b(g, q, start, arg...);
-    auto load = [&](int u, int kk) {
-      if (q.col && (unsigned)kk < (unsigned)nz) b.load(u, kk, mine + u * (NP * kSweepCols));
-      asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    auto fetch = [&](int u) {   // the operands of the step of slot u into registers
-      asm volatile("cp.async.wait_group %0;" ::"n"(P - 1) : "memory");
-      b.fetch(mine + u * (NP * kSweepCols));
-    };
-#pragma unroll
-    for (int u = 0; u < P; ++u) load(u, start + u);
-    b.ahead();
-    fetch(0);
     double *cur = &ring[0][at], *oth = &ring[P][at];   // this block's slots and the other half
-    for (int kk = start, t0 = 0; t0 < T; t0 += P, kk += P) {
-      block_barrier();
+    Body b(g, q, start, arg...);
+    if (warp < 2) {
+      const double *mine = &stage[0][0][col];
+      step_barrier();
+      for (int kk = start, t0 = 0; t0 < T; t0 += P, kk += P) {
+        block_barrier();
 #pragma unroll
-      for (int u = 0; u < P; ++u) {
-        const double *prev = u > 0 ? cur + (u - 1) * SLOT : oth + (P - 1) * SLOT;
-        double w[NV], s[NV], o[NV];
+        for (int u = 0; u < P; ++u) {
+          const double *prev = u > 0 ? cur + (u - 1) * SLOT : oth + (P - 1) * SLOT;
+          double w[NV], s[NV], o[NV];
 #pragma unroll
-        for (int v = 0; v < NV; ++v) { w[v] = prev[v * E * E - E]; s[v] = prev[v * E * E - 1]; }
-        b.before(w, s);
-        if (q.col && (unsigned)(kk + u) < (unsigned)nz) {
-          b.step(u, kk + u, w, s, o);
+          for (int v = 0; v < NV; ++v) { w[v] = prev[v * E * E - E]; s[v] = prev[v * E * E - 1]; }
+          b.fetch(mine + u * (NP * kSweepCols));
+          b.before(w, s);
+          if (q.col && (unsigned)(kk + u) < (unsigned)nz) {
+            b.step(u, kk + u, w, s, o);
 #pragma unroll
-          for (int v = 0; v < NV; ++v) cur[u * SLOT + v * E * E] = o[v];
+            for (int v = 0; v < NV; ++v) cur[u * SLOT + v * E * E] = o[v];
+          }
+          b.after(w, s);
+          step_barrier();
         }
-        b.after(w, s);
-        load(u, kk + u + P);
-        fetch((u + 1) % P);
-        step_barrier();
+        b.next();
+        double *tmp = cur; cur = oth; oth = tmp;
       }
-      b.next();
-      double *tmp = cur; cur = oth; oth = tmp;
+    } else {
+      double *mine = &stage[0][0][col];
+      auto load = [&](int u, int kk) {
+        if (q.col && (unsigned)kk < (unsigned)nz) b.load(u, kk, mine + u % P * (NP * kSweepCols));
+        asm volatile("cp.async.commit_group;" ::: "memory");
+      };
+      auto store = [&](int u, int kk, const double *slot) {
+        if (q.col && (unsigned)kk < (unsigned)nz) b.store(u, slot[0]);
+      };
+#pragma unroll
+      for (int u = 0; u < P - 1; ++u) load(u, start + u);
+      asm volatile("cp.async.wait_group %0;" ::"n"(P - 2) : "memory");
+      step_barrier();
+      for (int kk = start, t0 = 0; t0 < T; t0 += P, kk += P) {
+#pragma unroll
+        for (int u = 0; u < P; ++u) {
+          // the step after the last loaded one, into the slot of the step before this one
+          load(u + P - 1, kk + u + P - 1);
+          store(u - 1, kk + u - 1, u > 0 ? cur + (u - 1) * SLOT : oth + (P - 1) * SLOT);
+          asm volatile("cp.async.wait_group %0;" ::"n"(P - 2) : "memory");
+          step_barrier();
+        }
+        b.next();
+        double *tmp = cur; cur = oth; oth = tmp;
+      }
+      store(-1, start + T - 1, oth + (P - 1) * SLOT);
+      asm volatile("cp.async.wait_all;" ::: "memory");
     }
-    asm volatile("cp.async.wait_all;" ::: "memory");
   }
   sweep_finish(y, g.tiles());
 }
@@ -257,8 +274,13 @@ struct IcBody {
     cw = d[kIcW * C]; cs = d[kIcS * C]; cb = d[kIcB * C];
     if constexpr (KIND == 2) { ctw = d[kIcTw * C]; cts = d[kIcTs * C]; }
   }
-  __device__ __forceinline__ void ahead() { lO += P * S; lW += P * S; lS += P * S; lr += P * D; }
-  __device__ __forceinline__ void next() { ahead(); zO += P * S; lz += P * D; }
+  __device__ __forceinline__ void next() {
+    lO += P * S; lW += P * S; lS += P * S; lr += P * D; zO += P * S; lz += P * D;
+  }
+  __device__ __forceinline__ void store(int u, double z) {
+    if (BWD) lz[u * D] = z;
+    else zO[u * S + kIcZ * C] = z;
+  }
   __device__ __forceinline__ void before(const double *w, const double *s) {
     if constexpr (KIND == 1) { zW0 = w[0]; zS0 = s[0]; }
   }
@@ -274,8 +296,6 @@ struct IcBody {
     if (kk > 0) sum = msub(sum, cb, zB);
     zB = sweep_div(sum, cc, cy);
     o[0] = zB;
-    if (BWD) lz[u * D] = zB;
-    else zO[u * S + kIcZ * C] = zB;
   }
 };
 
@@ -316,8 +336,8 @@ struct IcFormBody {
     sweep_copy(d, ac + u); sweep_copy(d + C, aw + u); sweep_copy(d + 2 * C, as + u); sweep_copy(d + 3 * C, ab + u);
   }
   __device__ __forceinline__ void fetch(const double *d) { rc = d[0]; rw = d[C]; rs = d[2 * C]; rb = d[3 * C]; }
-  __device__ __forceinline__ void ahead() { ac += P; aw += P; as += P; ab += P; }
-  __device__ __forceinline__ void next() { ahead(); o_ += P * NP * C; }
+  __device__ __forceinline__ void next() { ac += P; aw += P; as += P; ab += P; o_ += P * NP * C; }
+  __device__ __forceinline__ void store(int, double) {}   // the arithmetic warps hold the factor
   __device__ __forceinline__ void before(const double *w, const double *s) {
     if constexpr (KIND == 1) { cW0 = w[0]; cS0 = s[0]; }
   }
@@ -415,8 +435,8 @@ struct GsBody {
     rw = d[kGsW * C]; re = d[kGsE * C]; rs = d[kGsS * C]; rn = d[kGsN * C]; rbt = d[kGsBt * C]; rt = d[kGsT * C];
     xe = d[kGsX * C]; xn = d[(kGsX + 1) * C]; xt = d[(kGsX + 2) * C];
   }
-  __device__ __forceinline__ void ahead() { lO += P * S; lE += P * S; lN += P * S; }
-  __device__ __forceinline__ void next() { ahead(); xO += P * S; lx += P; }
+  __device__ __forceinline__ void next() { lO += P * S; lE += P * S; lN += P * S; xO += P * S; lx += P; }
+  __device__ __forceinline__ void store(int u, double v) { xO[u * S] = v; lx[u] = v; }
   __device__ __forceinline__ void before(const double *, const double *) {}
   __device__ __forceinline__ void after(const double *, const double *) {}
   __device__ __forceinline__ void step(int u, int kk, const double *w, const double *s, double *o) {
@@ -429,8 +449,6 @@ struct GsBody {
     v = __dadd_rn(v, __dmul_rn(rt, kk + 1 < nz ? xt : 0.0));
     xB = __dmul_rn(rci, v);
     o[0] = xB;
-    xO[u * S] = xB;
-    lx[u] = xB;
   }
 };
 
