@@ -462,7 +462,7 @@ class BatchEngine : public BatchEngineBase {
     C.cnt = dcnt_.p;
     C.S = S_;
     C.kc_max = shape_.kc_max;
-    C.omega = (T)0.8;
+    C.om = {(T)kOmegaA, (T)kOmegaB, (T)kOverCorr};
     return C;
   }
 

@@ -110,7 +110,7 @@ struct BCtx {
   unsigned *cnt;            // [kBMaxLev * S] arrival counters (zero between launches)
   int S;
   int kc_max;               // levels 1..kc_max run a K-cycle, deeper ones one visit
-  T omega;
+  CycleW<T> om;
 };
 
 // Tiles of level l, grid-strided, with the next tile's record loaded one
@@ -491,17 +491,17 @@ __device__ __forceinline__ const T *b_rhs(const BProb<T> &P, int l, bool kc) {
 // Two damped-Jacobi sweeps from zero (k_jac2) into xb; kc: rhs b - a1 q1,
 // formed on the fly and stored to r1.
 template <typename T>
-__device__ __forceinline__ void cell_jac2(const BLev<T> &V, const T *r, uint32_t p, T a1, bool kc, T om) {
+__device__ __forceinline__ void cell_jac2(const BLev<T> &V, const T *r, uint32_t p, T a1, bool kc, CycleW<T> om) {
   const EMat<T> &A = V.A;
   auto rv = [&](uint32_t s) -> T { return kc ? V.b[s] - a1 * V.q1[s] : r[s]; };
-  auto x1 = [&](uint32_t s) -> T { return om * rv(s) * A.dinv[s]; };
+  auto x1 = [&](uint32_t s) -> T { return om.a * rv(s) * A.dinv[s]; };
   const Pos q = A.g.pos(p);
   const T rp = rv(p);
   if (kc) V.r1[p] = rp;
   const T d = A.dinv[p];
-  const T xp = om * rp * d;
+  const T xp = om.a * rp * d;
   const T on = offdiag(A, p, q, x1);
-  V.xb[p] = xp + om * ((rp + on) * d - xp);
+  V.xb[p] = xp + om.b * ((rp + on) * d - xp);
 }
 
 // Row of the dense coarsest solve: one warp, FP64 sums (lane 0 writes).
@@ -514,8 +514,9 @@ __device__ __forceinline__ void warp_dense_row(const double *Ainv, int n, const 
   if (lane == 0) x[row] = (T)acc;
 }
 
-// xa = xb + P e, then one sweep (k_prolong_jac); e from level l+1: eH
-// (dense solution or single visit) or c1 z1 + c2 z2 (two).
+// xa = xb + P e, then one sweep (k_prolong_jac); e from level l+1: c1 eH
+// (dense solution or single visit) or c1 z1 + c2 z2 (two), the factor `over`
+// in c1 and c2.
 template <typename T>
 __device__ __forceinline__ void cell_prolong_jac(const BLev<T> &V, const BLev<T> &Hl, const T *r, const T *eH,
                                                  bool two, T c1, T c2, T om, uint32_t p) {
@@ -525,7 +526,7 @@ __device__ __forceinline__ void cell_prolong_jac(const BLev<T> &V, const BLev<T>
   const int sx = A.nx > 1 ? 1 : 0, sy = A.ny > 1 ? 1 : 0, sz = A.nz > 1 ? 1 : 0;
   auto e = [&](int i, int j, int k) -> T {
     const uint32_t Pc = (uint32_t)(i >> sx) * H.nynz + (uint32_t)(j >> sy) * (uint32_t)H.nz + (uint32_t)(k >> sz);
-    return two ? c1 * eH[Pc] + c2 * z2H[Pc] : eH[Pc];
+    return two ? c1 * eH[Pc] + c2 * z2H[Pc] : c1 * eH[Pc];
   };
   const T *xi = V.xb;
   const Pos q = A.g.pos(p);
@@ -600,17 +601,17 @@ __device__ __forceinline__ bool b_tile_level(const BState &S, const BProb<T> &P,
 // Coarse correction read by the prolongation on level l (from level l+1)
 template <typename T>
 __device__ __forceinline__ void b_coarse(const BProb<T> &P, const BState &S, int l, int kc_max,
-                                         const T *&eH, bool &two, T &c1, T &c2) {
+                                         T over, const T *&eH, bool &two, T &c1, T &c2) {
   const BLev<T> &Hl = P.L[l + 1];
   const bool hdense = P.nlev - 1 == l + 1;
   two = !hdense && (l + 1) <= kc_max;
   eH = hdense ? Hl.x : Hl.z1;
-  c1 = 1;
+  c1 = over;
   c2 = 0;
   if (two) {
     const KScal &k = S.ks[l + 1];
-    c1 = (T)(k.a1 - k.a2 * k.beta);
-    c2 = (T)k.a2;
+    c1 = over * (T)(k.a1 - k.a2 * k.beta);
+    c2 = over * (T)k.a2;
   }
 }
 
@@ -621,18 +622,18 @@ __device__ __forceinline__ void b_coarse(const BProb<T> &P, const BState &S, int
 
 // two damped-Jacobi sweeps from zero into xb (level 0 has no K-cycle rhs)
 template <typename T>
-__device__ __forceinline__ void vgroup_jac2(const BLev<T> &V, const T *r, T om, uint32_t p) {
+__device__ __forceinline__ void vgroup_jac2(const BLev<T> &V, const T *r, CycleW<T> om, uint32_t p) {
   constexpr int W = VecTraits<T>::V;
   const EMat<T> &A = V.A;
   const Pos q = A.g.pos(p);
   const CoefV<T> Cf = load_coef(A, p, q);
   const Vec<T> d = ldv(A.dinv, p), rp = ldv(r, p);
-  const HoodV<T> X = load_hood(A, p, q, FJac0<T>{r, A.dinv, om});
+  const HoodV<T> X = load_hood(A, p, q, FJac0<T>{r, A.dinv, om.a});
   Vec<T> o;
 #pragma unroll
   for (int m = 0; m < W; ++m) {
     const T xp = X.c.v[m];
-    o.v[m] = xp + om * ((rp.v[m] + offd(Cf, X, m)) * d.v[m] - xp);
+    o.v[m] = xp + om.b * ((rp.v[m] + offd(Cf, X, m)) * d.v[m] - xp);
   }
   stv(V.xb, p, o);
 }
@@ -692,7 +693,7 @@ __device__ __forceinline__ void vgroup_prolong_jac(const BProb<T> &P, const BLev
   auto e = [&](int i, int j, int k) -> T {
     if (k >= F) return T(0);
     const uint32_t Pc = (uint32_t)(i >> sx) * H.nynz + (uint32_t)(j >> sy) * (uint32_t)H.nz + (uint32_t)(k >> sz);
-    return two ? c1 * eH[Pc] + c2 * z2H[Pc] : eH[Pc];
+    return two ? c1 * eH[Pc] + c2 * z2H[Pc] : c1 * eH[Pc];
   };
   const T *xi = V.xb;
   const Pos q = A.g.pos(p);
@@ -753,10 +754,10 @@ __global__ void BPAD_BOUNDS kb_jac2(BCtx<T> C, int l, int kc) {
     const T a1 = kc ? (T)S.ks[l].a1 : T(0);
     const T *r = l == 0 ? P.r0 : P.L[l].b;
     if (kBPad<T> && l == 0) {
-      BGROUP_LOOP(tl, p) vgroup_jac2(P.L[0], r, C.omega, p);
+      BGROUP_LOOP(tl, p) vgroup_jac2(P.L[0], r, C.om, p);
       continue;
     }
-    BCELL_LOOP(tl, p) cell_jac2(P.L[l], r, p, a1, kc != 0, C.omega);
+    BCELL_LOOP(tl, p) cell_jac2(P.L[l], r, p, a1, kc != 0, C.om);
   }
 }
 
@@ -815,13 +816,13 @@ __global__ void BPAD_BOUNDS kb_prolong_jac(BCtx<T> C, int l, int kc) {
     const T *eH;
     bool two;
     T c1, c2;
-    b_coarse(P, S, l, C.kc_max, eH, two, c1, c2);
+    b_coarse(P, S, l, C.kc_max, C.om.over, eH, two, c1, c2);
     const T *r = b_rhs(P, l, kc != 0);
     if (kBPad<T> && l == 0) {
-      BGROUP_LOOP(tl, p) vgroup_prolong_jac(P, P.L[0], P.L[1], r, eH, two, c1, c2, C.omega, p);
+      BGROUP_LOOP(tl, p) vgroup_prolong_jac(P, P.L[0], P.L[1], r, eH, two, c1, c2, C.om.b, p);
       continue;
     }
-    BCELL_LOOP(tl, p) cell_prolong_jac(P.L[l], P.L[l + 1], r, eH, two, c1, c2, C.omega, p);
+    BCELL_LOOP(tl, p) cell_prolong_jac(P.L[l], P.L[l + 1], r, eH, two, c1, c2, C.om.b, p);
   }
 }
 
@@ -838,13 +839,13 @@ __global__ void BPAD_BOUNDS kb_jac(BCtx<T> C, int l, int kc) {
     T *z = l == 0 ? P.z0 : (kc ? V.z2 : V.z1);
     double v[2] = {0.0, 0.0};
     if (kBPad<T> && l == 0) {
-      BGROUP_LOOP(tl, p) vgroup_jac(P, V, r, C.omega, p, v);
+      BGROUP_LOOP(tl, p) vgroup_jac(P, V, r, C.om.a, p, v);
       double o[2];
       if (b_reduce<2>(C, 0, t, tl.slot, v, o)) { S.f.zr = o[0]; S.f.zq = o[1]; }
       continue;
     }
     BCELL_LOOP(tl, p) {
-      const T zz = cell_jac(V, r, z, C.omega, p);
+      const T zz = cell_jac(V, r, z, C.om.a, p);
       if (l == 0) {
         v[0] += (double)zz * (double)r[p];
         v[1] += (double)zz * (double)P.q0[p];
@@ -906,7 +907,7 @@ __device__ __forceinline__ void t_allreduce(double (&v)[K], double (*sm)[kBThrea
 // preconditioner application, 1 / 3 finish it. Leaves z1 (and z2) on level
 // top and its scalars in S.ks[top] as a1 = c1, a2 = c2, beta = 0.
 template <typename T>
-__device__ void t_kcycle(const BProb<T> &P, BState &S, int top, int kc_max, T om) {
+__device__ void t_kcycle(const BProb<T> &P, BState &S, int top, int kc_max, CycleW<T> om) {
   __shared__ double sm[3][kBThreadsMax / 32];
   __shared__ double bc[4];
   const int last = P.nlev - 1;
@@ -950,10 +951,10 @@ __device__ void t_kcycle(const BProb<T> &P, BState &S, int top, int kc_max, T om
       const bool hdense = l + 1 == last;
       const bool two = !hdense && (l + 1) <= kc_max;
       const T *eH = hdense ? H.x : H.z1;
-      const T c1 = hdense ? T(1) : (T)c1v[l + 1], c2 = hdense ? T(0) : (T)c2v[l + 1];
-      TCELL_LOOP(p, n) cell_prolong_jac(V, H, rr, eH, two, c1, c2, om, p);
+      const T c1 = hdense ? om.over : om.over * (T)c1v[l + 1], c2 = hdense ? T(0) : om.over * (T)c2v[l + 1];
+      TCELL_LOOP(p, n) cell_prolong_jac(V, H, rr, eH, two, c1, c2, om.b, p);
       __syncthreads();
-      TCELL_LOOP(p, n) cell_jac(V, rr, second ? V.z2 : V.z1, om, p);
+      TCELL_LOOP(p, n) cell_jac(V, rr, second ? V.z2 : V.z1, om.a, p);
       __syncthreads();
     }
     if (!second) {
@@ -994,7 +995,7 @@ __global__ void __launch_bounds__(kBThreadsMax) kb_tail(BCtx<T> C, int l) {
     BState &S = C.st[slot];
     const BProb<T> &P = C.prob[slot];
     if (!b_running(S) || P.tail != l) continue;
-    t_kcycle(P, S, l, C.kc_max, C.omega);
+    t_kcycle(P, S, l, C.kc_max, C.om);
   }
 }
 

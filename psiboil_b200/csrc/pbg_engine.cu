@@ -247,14 +247,14 @@ static bool graph_loop_enabled() {
 
 // Tuning knobs (environment): PBG_COARSE_MAX sets the size of the dense
 // coarsest level, PBG_KC_MAX the deepest level that runs a K-cycle,
-// PBG_OMEGA the damped-Jacobi weight (0 < omega < 1).
+// PBG_OMEGA one damped-Jacobi weight for every sweep (0 < omega < 1).
 EngineOpts::EngineOpts() {
   const char *c = getenv("PBG_COARSE_MAX");
   if (c && atoi(c) > 0) coarse_max = atoi(c);
   const char *k = getenv("PBG_KC_MAX");
   if (k && atoi(k) > 0) kc_max = atoi(k);
   const char *o = getenv("PBG_OMEGA");
-  if (o && atof(o) > 0.0 && atof(o) < 1.0) omega = atof(o);
+  if (o && atof(o) > 0.0 && atof(o) < 1.0) omega_a = omega_b = atof(o);
 }
 
 template struct EWork<double>;
@@ -451,7 +451,7 @@ template <typename T>
 void Engine::precond(int l, const T *r, T *z, bool dots, const T *u, double *out2, EWork<T> &w,
                      RedPool &red, const int *stop, cudaStream_t s, bool kc) {
   const int last = (int)L.size() - 1;
-  const T om = (T)opt.omega;
+  const CycleW<T> om{(T)opt.omega_a, (T)opt.omega_b, (T)opt.over};
   auto &v = w.L[l];
   if (l == last) {
     dense_solve<T>(r, z, stop, s);
@@ -496,17 +496,17 @@ void Engine::precond(int l, const T *r, T *z, bool dots, const T *u, double *out
              (const T *)v.xb.p, H.ny, H.nz, eH, z2H, ksH, v.xa.p, om, stop);
   if (dots && vec && l == 0) {
     // u is the q of the previous FCG iteration, picked by parity on the device
-    launch_pdl(kv_jac<T, true>, gv, kThreads, s, A, rr, (const T *)v.xa.p, z, om, (const T *)w.q0.p,
+    launch_pdl(kv_jac<T, true>, gv, kThreads, s, A, rr, (const T *)v.xa.p, z, om.a, (const T *)w.q0.p,
                (const T *)w.q0b.p, (const FcgScal *)w.fs.p, out2, red.slot_part(0), red.slot_count(0), stop);
   } else if (dots) {
-    launch_pdl(k_jac_dots<T>, g, kThreads, s, A, rr, (const T *)v.xa.p, z, om, u, out2, red.slot_part(0),
+    launch_pdl(k_jac_dots<T>, g, kThreads, s, A, rr, (const T *)v.xa.p, z, om.a, u, out2, red.slot_part(0),
                red.slot_count(0), stop);
   } else if (vec) {
-    launch_pdl(kv_jac<T, false>, gv, kThreads, s, A, rr, (const T *)v.xa.p, z, om, (const T *)nullptr,
+    launch_pdl(kv_jac<T, false>, gv, kThreads, s, A, rr, (const T *)v.xa.p, z, om.a, (const T *)nullptr,
                (const T *)nullptr, (const FcgScal *)nullptr, (double *)nullptr, (double *)nullptr,
                (unsigned *)nullptr, stop);
   } else {
-    launch_pdl(k_jac<T>, g, kThreads, s, A, rr, (const T *)v.xa.p, z, om, stop);
+    launch_pdl(k_jac<T>, g, kThreads, s, A, rr, (const T *)v.xa.p, z, om.a, stop);
   }
 }
 

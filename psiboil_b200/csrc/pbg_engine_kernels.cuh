@@ -84,27 +84,27 @@ __global__ void __launch_bounds__(kThreads, 8) k_jac(EMat<T> A, const T *__restr
 }
 
 // Two damped-Jacobi sweeps from a zero guess in one pass:
-//   x1 = w D^-1 r;  x2 = x1 + w (D^-1 (r + sum_nb a_nb x1_nb) - x1)
+//   x1 = a D^-1 r;  x2 = x1 + b (D^-1 (r + sum_nb a_nb x1_nb) - x1)
 // with x1 at the neighbours formed from r and D^-1 there. When ks is set the
 // right-hand side is the K-cycle residual r = b2 - a1 q2, formed on the fly
 // and stored to r_out for the later passes of the same cycle.
 template <typename T>
 __global__ void __launch_bounds__(kThreads, 8)
     k_jac2(EMat<T> A, const T *__restrict__ r, const T *__restrict__ b2, const T *__restrict__ q2,
-           const KScal *ks, T *__restrict__ r_out, T *__restrict__ xo, T omega, const int *stop) {
+           const KScal *ks, T *__restrict__ r_out, T *__restrict__ xo, CycleW<T> om, const int *stop) {
   PBG_PDL_ENTRY();
   if (stop && *stop) return;
   const T a1 = ks ? (T)ks->a1 : T(0);
   auto rv = [&](uint32_t s) -> T { return ks ? b2[s] - a1 * q2[s] : r[s]; };
-  auto x1 = [&](uint32_t s) -> T { return omega * rv(s) * A.dinv[s]; };
+  auto x1 = [&](uint32_t s) -> T { return om.a * rv(s) * A.dinv[s]; };
   GRID_LOOP(p, A.g.n) {
     Pos q = A.g.pos(p);
     const T rp = rv(p);
     if (ks) r_out[p] = rp;
     const T d = A.dinv[p];
-    const T xp = omega * rp * d;
+    const T xp = om.a * rp * d;
     const T on = offdiag(A, p, q, x1);
-    xo[p] = xp + omega * ((rp + on) * d - xp);
+    xo[p] = xp + om.b * ((rp + on) * d - xp);
   }
 }
 
@@ -186,22 +186,22 @@ __global__ void __launch_bounds__(kThreads, 8) k_resid_restrict(EMat<T> A, const
 }
 
 // x' = xi + P e (prolongation of the coarse correction), then one sweep.
-// e is the coarse array eH, or — after a K-cycle — e = c1 z1H + c2 z2H with
-// c1 = a1 - a2 beta, c2 = a2 from the coarse level's scalars ksH.
+// e is `over` times the coarse array eH, or — after a K-cycle — times
+// (a1 - a2 beta) z1H + a2 z2H with the coarse level's scalars ksH.
 template <typename T>
 __global__ void __launch_bounds__(kThreads, 8)
     k_prolong_jac(EMat<T> A, const T *__restrict__ r, const T *__restrict__ xi, int Hny, int Hnz,
                   const T *__restrict__ eH, const T *__restrict__ z2H, const KScal *ksH,
-                  T *__restrict__ xo, T omega, const int *stop) {
+                  T *__restrict__ xo, CycleW<T> om, const int *stop) {
   PBG_PDL_ENTRY();
   if (stop && *stop) return;
   const int sx = A.nx > 1 ? 1 : 0, sy = A.ny > 1 ? 1 : 0, sz = A.nz > 1 ? 1 : 0;
   const uint32_t HnYZ = (uint32_t)Hny * Hnz;
-  T c1 = 1, c2 = 0;
-  if (ksH) { c1 = (T)(ksH->a1 - ksH->a2 * ksH->beta); c2 = (T)ksH->a2; }
+  T c1 = om.over, c2 = 0;
+  if (ksH) { c1 = om.over * (T)(ksH->a1 - ksH->a2 * ksH->beta); c2 = om.over * (T)ksH->a2; }
   auto e = [&](int i, int j, int k) -> T {
     const uint32_t P = (uint32_t)(i >> sx) * HnYZ + (uint32_t)(j >> sy) * Hnz + (uint32_t)(k >> sz);
-    return ksH ? c1 * eH[P] + c2 * z2H[P] : eH[P];
+    return ksH ? c1 * eH[P] + c2 * z2H[P] : c1 * eH[P];
   };
   GRID_LOOP(p, A.g.n) {
     Pos q = A.g.pos(p);
@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(kThreads, 8)
     if (q.k > 0) on += A.b[p] * (xi[p - 1] + e(q.i, q.j, q.k - 1));
     if (q.k < A.nz - 1) on += A.b[p + 1] * (xi[p + 1] + e(q.i, q.j, q.k + 1));
     T xp = xi[p] + e(q.i, q.j, q.k);
-    xo[p] = xp + omega * ((r[p] + on) * A.dinv[p] - xp);
+    xo[p] = xp + om.b * ((r[p] + on) * A.dinv[p] - xp);
   }
 }
 

@@ -174,7 +174,7 @@ template <typename T> constexpr int kVecWideBlocks = 148 * kVecWideSm<T>;
 template <typename T>
 __global__ void __launch_bounds__(kThreads, kVecWideSm<T>)
     kv_jac2(EMat<T> A, const T *__restrict__ r, const T *__restrict__ b2, const T *__restrict__ q2,
-            const KScal *ks, T *__restrict__ r_out, T *__restrict__ xo, T omega, const int *stop) {
+            const KScal *ks, T *__restrict__ r_out, T *__restrict__ xo, CycleW<T> om, const int *stop) {
   PBG_PDL_ENTRY();
   if (stop && *stop) return;
   constexpr int V = VecTraits<T>::V;
@@ -189,17 +189,17 @@ __global__ void __launch_bounds__(kThreads, kVecWideSm<T>)
     if (ks) {
       FKc<T> fr{b2, q2, a1};
       rp = fr.vec(p);
-      X = load_hood(A, p, q, FJac0Kc<T>{fr, A.dinv, omega});
+      X = load_hood(A, p, q, FJac0Kc<T>{fr, A.dinv, om.a});
       stv(r_out, p, rp);
     } else {
       rp = ldv(r, p);
-      X = load_hood(A, p, q, FJac0<T>{r, A.dinv, omega});
+      X = load_hood(A, p, q, FJac0<T>{r, A.dinv, om.a});
     }
     Vec<T> o;
 #pragma unroll
     for (int m = 0; m < V; ++m) {
       const T xp = X.c.v[m];
-      o.v[m] = xp + omega * ((rp.v[m] + offd(C, X, m)) * d.v[m] - xp);
+      o.v[m] = xp + om.b * ((rp.v[m] + offd(C, X, m)) * d.v[m] - xp);
     }
     stv(xo, p, o);
   }
@@ -253,15 +253,15 @@ template <typename T>
 __global__ void __launch_bounds__(kThreads, 4)
     kv_prolong_jac(EMat<T> A, const T *__restrict__ r, const T *__restrict__ xi, int Hny, int Hnz,
                    const T *__restrict__ eH, const T *__restrict__ z2H, const KScal *ksH,
-                   T *__restrict__ xo, T omega, const int *stop) {
+                   T *__restrict__ xo, CycleW<T> om, const int *stop) {
   PBG_PDL_ENTRY();
   if (stop && *stop) return;
   constexpr int V = VecTraits<T>::V;
   const int sx = A.nx > 1 ? 1 : 0, sy = A.ny > 1 ? 1 : 0;
   const uint32_t HnYZ = (uint32_t)Hny * Hnz;
-  T c1 = 1, c2 = 0;
-  if (ksH) { c1 = (T)(ksH->a1 - ksH->a2 * ksH->beta); c2 = (T)ksH->a2; }
-  auto e = [&](uint32_t P) -> T { return ksH ? c1 * eH[P] + c2 * z2H[P] : eH[P]; };
+  T c1 = om.over, c2 = 0;
+  if (ksH) { c1 = om.over * (T)(ksH->a1 - ksH->a2 * ksH->beta); c2 = om.over * (T)ksH->a2; }
+  auto e = [&](uint32_t P) -> T { return ksH ? c1 * eH[P] + c2 * z2H[P] : c1 * eH[P]; };
   // x + P e around the group: lane m's parent along k is (k+m)>>1 (nz > 1 here)
   VGRID_LOOP(gi, A.g.n / V) {
     const uint32_t p = gi * V;
@@ -290,7 +290,7 @@ __global__ void __launch_bounds__(kThreads, 4)
 #pragma unroll
     for (int m = 0; m < V; ++m) {
       const T xp = X.c.v[m];
-      o.v[m] = xp + omega * ((rp.v[m] + offd(C, X, m)) * d.v[m] - xp);
+      o.v[m] = xp + om.b * ((rp.v[m] + offd(C, X, m)) * d.v[m] - xp);
     }
     stv(xo, p, o);
   }
