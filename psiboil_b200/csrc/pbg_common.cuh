@@ -282,10 +282,10 @@ struct RedScratch {
 };
 constexpr int kRedVals = 4;   // values reduced by one kernel at most
 
-template <int NV>
+template <int NV, int First = 16>
 __device__ __forceinline__ void warp_sum(double (&v)[NV]) {
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1)
+  for (int off = First; off > 0; off >>= 1)
 #pragma unroll
     for (int q = 0; q < NV; ++q) v[q] += __shfl_down_sync(0xffffffffu, v[q], off);
 }
@@ -335,13 +335,16 @@ __device__ bool grid_reduce(double (&v)[NV], double *part, unsigned *count, doub
 #pragma unroll
     for (int q = 0; q < NV; ++q) sm[q][wid] = v[q];
   __syncthreads();
+  // the warps' sums by the lanes of warp 0 (a serial sum by one thread took
+  // as long as the whole pass of a small grid)
+  if (wid == 0) {
+#pragma unroll
+    for (int q = 0; q < NV; ++q) v[q] = lane < nw ? sm[q][lane] : 0.0;
+    warp_sum<NV, kThreads / 64>(v);
+  }
   if (threadIdx.x == 0) {
 #pragma unroll
-    for (int q = 0; q < NV; ++q) {
-      double s = 0.0;
-      for (int w = 0; w < nw; ++w) s += sm[q][w];
-      part[q * kMaxBlocks + blockIdx.x] = s;
-    }
+    for (int q = 0; q < NV; ++q) part[q * kMaxBlocks + blockIdx.x] = v[q];
     __threadfence();
     unsigned prev = atomicAdd(count, 1u);
     last = (prev == gridDim.x - 1);
@@ -361,13 +364,14 @@ __device__ bool grid_reduce(double (&v)[NV], double *part, unsigned *count, doub
 #pragma unroll
     for (int q = 0; q < NV; ++q) sm[q][wid] = acc[q];
   __syncthreads();
+  if (wid == 0) {
+#pragma unroll
+    for (int q = 0; q < NV; ++q) acc[q] = lane < nw ? sm[q][lane] : 0.0;
+    warp_sum<NV, kThreads / 64>(acc);
+  }
   if (threadIdx.x == 0) {
 #pragma unroll
-    for (int q = 0; q < NV; ++q) {
-      double s = 0.0;
-      for (int w = 0; w < nw; ++w) s += sm[q][w];
-      out[q] = s;
-    }
+    for (int q = 0; q < NV; ++q) out[q] = acc[q];
     *count = 0u;
     return true;
   }
