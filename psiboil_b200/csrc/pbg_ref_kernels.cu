@@ -6,6 +6,7 @@
 #include <cstring>
 
 #include "pbg_ref_kernels.cuh"
+#include "pbg_small_cg.cuh"
 #include "pbg_sweep_kernels.cuh"
 
 namespace pbg {
@@ -67,9 +68,11 @@ __device__ __forceinline__ double ref_bmax(const MatView<double> &A, long long p
   return v;
 }
 
-// element of Scalar::dot_voldiv_avg: x*y/dV/dV (scalar.h:317-326)
-__device__ __forceinline__ double voldiv(double x, double y, double dV) {
-  return __ddiv_rn(__ddiv_rn(__dmul_rn(x, y), dV), dV);
+// element of Scalar::dot_voldiv_avg: x*y/dV/dV (scalar.h:317-326). Two FP64
+// divisions a cell (125 cycles each) bounded the kernels that form this sum;
+// the corrected products give the same bits.
+__device__ __forceinline__ double voldiv(double x, double y, const KnownDiv &dV) {
+  return dV(dV(__dmul_rn(x, y)));
 }
 
 // res = sqrt(d/N/N)/scale (cg.cpp:68 and :115)
@@ -101,7 +104,8 @@ __global__ void k_resid_ref(MatView<double> A, const double *__restrict__ x,
 
 // out[0] = sum x*y, out[1] = sum x*y/dV/dV (deterministic tree order)
 __global__ void k_dot2(long long N, const double *__restrict__ x, const double *__restrict__ y,
-                       double dV, double *part, unsigned *count, double *out) {
+                       double dvol, double *part, unsigned *count, double *out) {
+  const KnownDiv dV(dvol);
   double v[2] = {0.0, 0.0};
   for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < N;
        p += (long long)gridDim.x * blockDim.x) {
@@ -190,7 +194,7 @@ __global__ void k_cg_init(MatView<double> A, const double *__restrict__ x,
                           const double *__restrict__ b, double *__restrict__ r,
                           KrylovState *st, double *part, unsigned *count, const double *__restrict__ mc) {
   const long long N = A.ncell();
-  const double dV = st->dV;
+  const KnownDiv dV(st->dV);
   double v[2] = {0.0, 0.0};
   for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < N;
        p += (long long)gridDim.x * blockDim.x) {
@@ -267,7 +271,8 @@ __global__ void __launch_bounds__(kThreads, 3) k_cg_xr(long long N, const double
   if (st->done) return;
   const int it = st->iter;
   const double *p_ = (it & 1) ? pA : pB;  // the buffer k_cg_pq wrote
-  const double alfa = st->alfa, dV = st->dV;
+  const double alfa = st->alfa;
+  const KnownDiv dV(st->dV);
   double v[2] = {0.0, 0.0};
   for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < N;
        p += (long long)gridDim.x * blockDim.x) {
@@ -506,7 +511,7 @@ __global__ void k_bi_init(MatView<double> A, const double *__restrict__ x, const
                           double *__restrict__ r, double *__restrict__ rt, KrylovState *st,
                           double *part, unsigned *count) {
   const long long N = A.ncell();
-  const double dV = st->dV;
+  const KnownDiv dV(st->dV);
   double v[1] = {0.0};
   for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < N;
        p += (long long)gridDim.x * blockDim.x) {
@@ -624,7 +629,8 @@ __global__ void k_bi_xr(long long N, double *__restrict__ x, double *__restrict_
                         KrylovState *st, double *hist, double *part, unsigned *count) {
   const int pend = st->pending_x;
   if (st->done && !pend) return;
-  const double alfa = st->alfa, omega = st->omega, dV = st->dV;
+  const double alfa = st->alfa, omega = st->omega;
+  const KnownDiv dV(st->dV);
   double v[1] = {0.0};
   for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < N;
        p += (long long)gridDim.x * blockDim.x) {
@@ -735,7 +741,8 @@ __global__ void k_cgs_xr(MatView<double> A, double *__restrict__ x, double *__re
                          unsigned *count) {
   if (st->done) return;
   const long long N = A.ncell();
-  const double alfa = st->alfa, dV = st->dV;
+  const double alfa = st->alfa;
+  const KnownDiv dV(st->dV);
   double v[1] = {0.0};
   for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < N;
        p += (long long)gridDim.x * blockDim.x) {
@@ -956,10 +963,11 @@ __global__ void k_ac_interp(int nx, int ny, int nz, double *__restrict__ phi, in
 // out[0] = sqrt(dot_voldiv_avg(res,res)), linf via an order-free max of
 // |res/dV| (non-negative doubles order like their bit patterns).
 __global__ void k_ac_resnorm(MatView<double> A, const double *__restrict__ phi,
-                             const double *__restrict__ fnew, double dV, double *out,
+                             const double *__restrict__ fnew, double dvol, double *out,
                              unsigned long long *linf_bits, double *part, unsigned *count,
                              double *seq) {
   const long long N = A.ncell();
+  const KnownDiv dV(dvol);
   double v[1] = {0.0};
   double mx = 0.0;
   for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < N;
@@ -967,7 +975,7 @@ __global__ void k_ac_resnorm(MatView<double> A, const double *__restrict__ phi,
     Pos q = pos_of(p, A.ny, A.nz);
     double rv = ref_bmax(A, p, q, phi, fnew[p]);
     v[0] += voldiv(rv, rv, dV);
-    mx = fmax(mx, fabs(__ddiv_rn(rv, dV)));
+    mx = fmax(mx, fabs(dV(rv)));
   }
   for (int off = 16; off > 0; off >>= 1) mx = fmax(mx, __shfl_down_sync(0xffffffffu, mx, off));
   if ((threadIdx.x & 31) == 0) atomicMax(linf_bits, (unsigned long long)__double_as_longlong(mx));
@@ -1009,7 +1017,7 @@ __global__ void k_it_init(MatView<double> A, const double *__restrict__ x,
                           const double *__restrict__ b, double *__restrict__ r, KrylovState *st,
                           double *part, unsigned *count, int gs) {
   const long long N = A.ncell();
-  const double dV = st->dV;
+  const KnownDiv dV(st->dV);
   double v[1] = {0.0};
   for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < N;
        p += (long long)gridDim.x * blockDim.x) {
@@ -1095,7 +1103,7 @@ __global__ void k_it_resid(MatView<double> A, const double *__restrict__ x,
   if (st->done) return;
   const int it = st->iter;
   const long long N = A.ncell();
-  const double dV = st->dV;
+  const KnownDiv dV(st->dV);
   double v[1] = {0.0};
   for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < N;
        p += (long long)gridDim.x * blockDim.x) {
@@ -1358,7 +1366,9 @@ RefKrylovResult ref_krylov_solve(const MatView<double> &A, double *x, const doub
                                  const KrylovParams &pr, int solver, RefKrylovWork &w,
                                  const RedPool &red, KrylovState *st, KrylovState *hst,
                                  double *hist, cudaStream_t s) {
-  enqueue_ref_setup(A, x, b, pr, solver, w, red, st, s);
+  const int small = small_cg_blocks(A, solver, pr.prec, pr.seq != nullptr);
+  if (small) enqueue_small_cg(A, x, b, pr, small, st, hist, s);
+  else enqueue_ref_setup(A, x, b, pr, solver, w, red, st, s);
   int enq = 0, chunk = 8;
   for (;;) {
     PBG_CUDA(cudaMemcpyAsync(hst, st, sizeof(KrylovState), cudaMemcpyDeviceToHost, s));
@@ -1475,6 +1485,10 @@ void RefAC::smooth(int l, int mi, double res_rat, double res_tol, int ms, RefKry
   pr.prec = own ? sol_prec : sm_prec;
   pr.ci = l == 0 ? sm_ci0 : nullptr;  // coarse levels: ci = 1/c (additive_coarsen_system.cpp)
   MatView<double> A = view(l);
+  if (const int small = small_cg_blocks(A, kind, pr.prec, seq != nullptr)) {
+    enqueue_small_cg(A, L[l].phi.p, L[l].fnew.p, pr, small, st, nullptr, s);
+    return;
+  }
   enqueue_ref_setup(A, L[l].phi.p, L[l].fnew.p, pr, kind, w, red, st, s);
   enqueue_ref_iters(A, L[l].phi.p, kind, mi, w, red, st, nullptr, s, seq != nullptr, pr.prec);
 }
