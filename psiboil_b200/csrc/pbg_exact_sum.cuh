@@ -20,17 +20,20 @@
 //   2. an approximate prefix of all earlier terms comes from a decoupled
 //      look-back over the chunks' published sums (bounded polling: a block
 //      that gives up only loses its hint);
-//   3. for the three exponents around the hint, e0..e0+2, each warp computes
-//      K = sum of rint(a/u) over its 32 terms, the minimum and maximum of its
-//      running integer prefix, and whether every term was tie-free and
-//      finite; the chunk's record composes its warps' records;
+//   3. for the exponent of the approximate sum before its first term, each
+//      warp computes K = sum of rint(a/u) over its 32 terms, the minimum and
+//      maximum of its running integer prefix, and whether every term was
+//      tie-free and finite; the chunk's record composes its warps' records
+//      where they share the exponent (32 zero terms fit any);
 //   4. the last chunk of each group of kExactGroup chunks to arrive composes
-//      the group's records for the exponents of the group's last chunk;
+//      the group's records in the same way;
 //   5. the last block of the launch walks the groups in order with the exact
-//      running sum (one warp per sum): a group, chunk or warp record that
-//      holds the current exponent and keeps s/u + prefix inside
-//      [2^52 + 1, 2^53 - 1] is applied as s += u K; a warp segment whose
-//      record does not is added term by term.
+//      running sum (one warp per sum): 32 records at a time, a scan of their
+//      K gives each record's running sum, and every record up to the first
+//      that does not hold the current exponent or does not keep s/u + prefix
+//      inside [2^52 + 1, 2^53 - 1] is applied at once, as s += u K. A group
+//      that stops the run is entered at its chunks, a chunk at its warps, and
+//      the 32 terms of a warp that stops it are added one by one.
 // Every step of the walk is either the sequential rounding itself or an
 // integer sum proven equal to it, so the result is the sequential sum bit
 // for bit whatever the hints were; bad hints only cost time.
@@ -47,11 +50,11 @@ constexpr int kExactGroup = 64;          // chunks per group record
 constexpr int kExactVals = 2;            // sums per reducing kernel at most
 constexpr int kExactPoll = 4096;         // look-back polls before a block gives up its hint
 
-// Record of one chunk or group for the exponents e0, e0+1, e0+2.
+// Record of a warp's terms, a chunk or a group at the exponent e.
+enum : int { kExactNone, kExactOk, kExactZero };   // kExactZero: every term is zero, fits any sum
 struct ExactRec {
-  long long K[3], mn[3], mx[3];
-  int e0;   // exponent of candidate 0
-  int ok;   // bit c: candidate c usable
+  long long K, mn, mx;
+  int e, ok;
 };
 
 // Header stored kExactHdrBytes before the terms (the `seq` pointer).
@@ -92,71 +95,59 @@ __device__ __forceinline__ unsigned ld_volatile_u32(const unsigned *p) {
 }
 
 // Record load through L2 (records written by other blocks of the launch).
-__device__ __forceinline__ void exact_load(ExactRec &d, const ExactRec *s) {
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    d.K[c] = __ldcg(&s->K[c]);
-    d.mn[c] = __ldcg(&s->mn[c]);
-    d.mx[c] = __ldcg(&s->mx[c]);
-  }
-  d.e0 = __ldcg(&s->e0);
+__device__ __forceinline__ ExactRec exact_load(const ExactRec *s) {
+  ExactRec d;
+  d.K = __ldcg(&s->K);
+  d.mn = __ldcg(&s->mn);
+  d.mx = __ldcg(&s->mx);
+  d.e = __ldcg(&s->e);
   d.ok = __ldcg(&s->ok);
+  return d;
 }
 
-// Applies a record to the running sum s when it is provably the sequential
-// result; returns false (s unchanged) otherwise.
-__device__ __forceinline__ bool exact_apply(double &s, const ExactRec &R) {
-  if (!(s != 0.0) || !isfinite(s)) return false;
-  const int e = ilogb(s);
-  if (e < -960 || e > 1000) return false;
-  const int c = e - R.e0;
-  if (c < 0 || c > 2 || !((R.ok >> c) & 1)) return false;
-  const long long LO = (1LL << 52) + 1, HI = (1LL << 53) - 1;
-  long long S = (long long)ldexp(fabs(s), 52 - e);  // exact, in [2^52, 2^53)
-  if (s < 0.0) S = -S;
-  const long long lo = S + R.mn[c], hi = S + R.mx[c];
-  if (s > 0.0) {
-    if (lo < LO || hi > HI) return false;
-  } else {
-    if (hi > -LO || lo < -HI) return false;
+constexpr long long kExact53 = 1LL << 53;
+
+// Composition of the records of a warp's lanes (lane < cnt, in lane order)
+// into one, the same in every lane. e: the exponent they must share.
+__device__ __forceinline__ ExactRec exact_compose(const ExactRec &r, int cnt, int e) {
+  const int lane = threadIdx.x & 31;
+  const bool in = lane < cnt, fits = !in || r.ok == kExactZero || (r.ok == kExactOk && r.e == e);
+  const long long k = in && r.ok == kExactOk ? r.K : 0;
+  long long incl = k;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const long long y = __shfl_up_sync(0xffffffffu, incl, off);
+    if (lane >= off) incl += y;
   }
-  S += R.K[c];
-  s = ldexp((double)S, e - 52);
-  return true;
+  const bool has = in && r.ok == kExactOk;
+  long long lo = has ? incl - k + r.mn : kExact53, hi = has ? incl - k + r.mx : -kExact53;
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+    const long long a = __shfl_xor_sync(0xffffffffu, lo, off), b = __shfl_xor_sync(0xffffffffu, hi, off);
+    lo = a < lo ? a : lo;
+    hi = b > hi ? b : hi;
+  }
+  ExactRec o;
+  o.K = __shfl_sync(0xffffffffu, incl, 31);
+  o.mn = lo;
+  o.mx = hi;
+  o.e = e;
+  const bool zero = __all_sync(0xffffffffu, !in || r.ok == kExactZero);
+  const bool good = __all_sync(0xffffffffu, fits) && lo > -kExact53 && hi < kExact53 && o.K > -kExact53 && o.K < kExact53;
+  o.ok = zero ? kExactZero : (good ? kExactOk : kExactNone);
+  return o;
 }
 
-// Running sum of the walk. While `in` holds, s = S * 2^(e-52) with |S| in
-// [2^52, 2^53): the record applications keep it there, so s is formed only
-// when a chunk is added term by term, or at the end.
+// Running sum of the walk, the same in every lane of its warp. While `in`
+// holds, s = S * 2^(e-52) with |S| in [2^52, 2^53): the record applications
+// keep it there, so s is formed only when terms are added one by one, or at
+// the end.
 struct ExactWalk {
   double s;
   long long S;
   int e;
   bool in;
 };
-
-__device__ __forceinline__ bool exact_walk_apply(ExactWalk &w, const ExactRec &R) {
-  if (!w.in) {
-    if (!(w.s != 0.0) || !isfinite(w.s)) return false;
-    const int e = ilogb(w.s);
-    if (e < -960 || e > 1000) return false;
-    long long S = (long long)ldexp(fabs(w.s), 52 - e);  // exact
-    w.S = w.s < 0.0 ? -S : S;
-    w.e = e;
-    w.in = true;
-  }
-  const int c = w.e - R.e0;
-  if (c < 0 || c > 2 || !((R.ok >> c) & 1)) return false;
-  const long long LO = (1LL << 52) + 1, HI = (1LL << 53) - 1;
-  const long long lo = w.S + R.mn[c], hi = w.S + R.mx[c];
-  if (w.S > 0) {
-    if (lo < LO || hi > HI) return false;
-  } else {
-    if (hi > -LO || lo < -HI) return false;
-  }
-  w.S += R.K[c];
-  return true;
-}
 
 __device__ __forceinline__ void exact_walk_flush(ExactWalk &w) {
   if (w.in) {
@@ -165,68 +156,82 @@ __device__ __forceinline__ void exact_walk_flush(ExactWalk &w) {
   }
 }
 
-// The walk of sum q by one warp: lane 0 carries the running sum through the
-// group records, descending into a group's chunk records, a chunk's warp
-// records and a warp segment's 32 terms only where a record does not apply.
-// The lanes load the records and terms (rec: 32 records, wrec: a chunk's
-// warp records, term: one chunk's terms). Returns the sum on lane 0.
+// Applies the records of lanes first .. cnt-1 in order up to the first that
+// is not provably the sequential result; returns its lane (cnt: all applied).
+__device__ __forceinline__ int exact_walk_run(ExactWalk &w, const ExactRec &r, int first, int cnt) {
+  const int lane = threadIdx.x & 31;
+  if (!w.in && w.s != 0.0 && isfinite(w.s)) {
+    const int e = ilogb(w.s);
+    if (e >= -960 && e <= 1000) {
+      const long long S = (long long)ldexp(fabs(w.s), 52 - e);  // exact
+      w.S = w.s < 0.0 ? -S : S;
+      w.e = e;
+      w.in = true;
+    }
+  }
+  const bool mine = lane >= first && lane < cnt;
+  const bool use = mine && r.ok == kExactOk && w.in && r.e == w.e;
+  const long long k = use ? r.K : 0;
+  long long incl = k;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const long long y = __shfl_up_sync(0xffffffffu, incl, off);
+    if (lane >= off) incl += y;
+  }
+  bool fits = mine && r.ok == kExactZero;
+  if (use) {
+    const long long LO = (1LL << 52) + 1, HI = kExact53 - 1;
+    const long long lo = w.S + (incl - k) + r.mn, hi = w.S + (incl - k) + r.mx;
+    fits = w.S > 0 ? (lo >= LO && hi <= HI) : (hi <= -LO && lo >= -HI);
+  }
+  const unsigned bad = __ballot_sync(0xffffffffu, mine && !fits);
+  const int stop = bad ? __ffs(bad) - 1 : cnt;
+  const long long sum = __shfl_sync(0xffffffffu, incl, stop > 0 ? stop - 1 : 0);
+  if (stop > first && w.in) w.S += sum;
+  return stop;
+}
+
+// The walk of sum q by one warp through the group records, down into a
+// group's chunk records, a chunk's warp records and a warp's 32 terms only
+// where a record does not apply. Returns the sum (every lane).
 static __device__ __noinline__ double exact_walk(const ExactHdr *H, const double *seq, long long n, long long nch,
-                                          int q, long long cap, long long capg, ExactRec *rec, ExactRec *wrec,
-                                          double *term) {
+                                          int q, long long cap, long long capg, double *term) {
   const int lane = threadIdx.x & 31;
   const long long ng = (nch + kExactGroup - 1) / kExactGroup;
+  const ExactRec none{0, 0, 0, 0, kExactNone};
   ExactWalk w{0.0, 0, 0, false};
-  long long gi = 0;
-  while (gi < ng) {
+  for (long long gi = 0; gi < ng; gi += 32) {
     const int nb = (int)((ng - gi) < 32 ? (ng - gi) : 32);
-    if (lane < nb) exact_load(rec[lane], &H->grec[q * capg + gi + lane]);
-    __syncwarp();
-    int k = 0;
-    if (lane == 0)
-      while (k < nb && exact_walk_apply(w, rec[k])) ++k;
-    k = __shfl_sync(0xffffffffu, k, 0);
-    __syncwarp();
-    gi += k;
-    if (k == nb) continue;
-    // group gi: its chunk records, 32 at a time
-    const long long c0 = gi * kExactGroup;
-    const int cs = (int)((nch - c0) < kExactGroup ? (nch - c0) : kExactGroup);
-    for (int h0 = 0; h0 < cs; h0 += 32) {
-      const int hb = (cs - h0) < 32 ? (cs - h0) : 32;
-      if (lane < hb) exact_load(rec[lane], &H->crec[q * cap + c0 + h0 + lane]);
-      __syncwarp();
-      int ci = 0;
-      while (ci < hb) {
-        int m = ci;
-        if (lane == 0)
-          while (m < hb && exact_walk_apply(w, rec[m])) ++m;
-        m = __shfl_sync(0xffffffffu, m, 0);
-        if (m >= hb) break;
-        // chunk c0 + h0 + m: its warp records, then the terms of a warp
-        // segment where one does not apply
-        const long long ch = c0 + h0 + m;
-        const long long e0 = ch * kExactChunkThreads;
-        const int len = (int)((n - e0) < kExactChunkThreads ? (n - e0) : kExactChunkThreads);
-        if (lane < kExactWarps) exact_load(wrec[lane], &H->wrec[(q * cap + ch) * kExactWarps + lane]);
-        for (int e = lane; e < len; e += 32) term[e] = __ldcg(&seq[q * n + e0 + e]);
-        __syncwarp();
-        if (lane == 0) {
-          for (int ww = 0; ww < kExactWarps && 32 * ww < len; ++ww) {
-            if (exact_walk_apply(w, wrec[ww])) continue;
+    const ExactRec G = lane < nb ? exact_load(&H->grec[q * capg + gi + lane]) : none;
+    for (int k = 0; (k = exact_walk_run(w, G, k, nb)) < nb; ++k) {
+      const long long c0 = (gi + k) * kExactGroup;
+      const int cs = (int)((nch - c0) < kExactGroup ? (nch - c0) : kExactGroup);
+      // both halves of the group's chunk records in flight at once
+      const ExactRec C0 = lane < cs ? exact_load(&H->crec[q * cap + c0 + lane]) : none;
+      const ExactRec C1 = lane + 32 < cs ? exact_load(&H->crec[q * cap + c0 + 32 + lane]) : none;
+      for (int h0 = 0; h0 < cs; h0 += 32) {
+        const int hb = (cs - h0) < 32 ? (cs - h0) : 32;
+        const ExactRec C = h0 == 0 ? C0 : C1;
+        for (int m = 0; (m = exact_walk_run(w, C, m, hb)) < hb; ++m) {
+          const long long ch = c0 + h0 + m;
+          const long long e0 = ch * kExactChunkThreads;
+          const int len = (int)((n - e0) < kExactChunkThreads ? (n - e0) : kExactChunkThreads);
+          const int nw = (len + 31) / 32;
+          const ExactRec W = lane < nw ? exact_load(&H->wrec[(q * cap + ch) * kExactWarps + lane]) : none;
+          __syncwarp();
+          for (int e = lane; e < len; e += 32) term[e] = __ldcg(&seq[q * n + e0 + e]);
+          __syncwarp();
+          for (int v = 0; (v = exact_walk_run(w, W, v, nw)) < nw; ++v) {
             exact_walk_flush(w);
-            double sv = w.s;
-            const int e1 = (32 * ww + 32) < len ? (32 * ww + 32) : len;
+            double sv = w.s;   // every lane the same additions
+            const int e1 = (32 * v + 32) < len ? (32 * v + 32) : len;
 #pragma unroll 8
-            for (int e = 32 * ww; e < e1; ++e) sv = __dadd_rn(sv, term[e]);
+            for (int e = 32 * v; e < e1; ++e) sv = __dadd_rn(sv, term[e]);
             w.s = sv;
           }
         }
-        __syncwarp();
-        ci = m + 1;
       }
-      __syncwarp();
     }
-    ++gi;
   }
   exact_walk_flush(w);
   return w.s;
@@ -252,9 +257,7 @@ __device__ bool exact_reduce(const double (&v)[NV], double *seq, long long n, un
   __shared__ double s_agg[NV][NW];
   __shared__ double s_hint[NV];
   __shared__ ExactRec s_wr[NV][kExactWarps];
-  __shared__ ExactRec s_rec;
   __shared__ bool s_last;
-  __shared__ ExactRec s_wrec[kExactVals][32];
   __shared__ double s_wterm[kExactVals][kExactChunkThreads];
   __shared__ double s_res[kExactVals];
 
@@ -336,168 +339,93 @@ __device__ bool exact_reduce(const double (&v)[NV], double *seq, long long n, un
   }
   __syncthreads();
 
-  // 3. records for the exponents around the hint: one per warp (32 terms,
-  // warp scans only), composed by thread 0 into the chunk's record
-  constexpr long long L53 = 1LL << 53;
+  // 3. one record per warp (32 terms) at the exponent of the approximate sum
+  // before it, composed by warp q into sum q's chunk record
 #pragma unroll
   for (int q = 0; q < NV; ++q) {
-    const double hint = s_hint[q];
-    int e0 = 0;
-    bool have = isfinite(hint) && hint != 0.0;
-    if (have) {
-      e0 = ilogb(hint) - 1;
-      have = e0 >= -960 && e0 + 2 <= 1000;
+    double before = s_hint[q];
+    for (int w = 0; w < wid; ++w) before += s_agg[q][w];
+    int e = 0;
+    bool good = isfinite(before) && before != 0.0;
+    if (good) {
+      e = ilogb(before);
+      good = e >= -960 && e <= 1000;
     }
-    ExactRec W;
-    W.e0 = e0;
-    W.ok = 0;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      long long k = 0;
-      bool good = false;
-      if (have) {
-        const double y = a[q] * ldexp(1.0, 52 - (e0 + c));
-        // finite, |y| <= 2^53 and not half-way between two integers
-        good = isfinite(y) && fabs(y) <= 9007199254740992.0 && fabs(y - trunc(y)) != 0.5;
-        k = good ? __double2ll_rn(y) : 0;
-      }
-      // inclusive prefix over the warp, its total and range
-      for (int off = 1; off < 32; off <<= 1) {
-        const long long v = __shfl_up_sync(0xffffffffu, k, off);
-        if (lane >= off) k += v;
-      }
-      long long mn = k, mx = k;
-      for (int off = 16; off > 0; off >>= 1) {
-        const long long a2 = __shfl_xor_sync(0xffffffffu, mn, off), b2 = __shfl_xor_sync(0xffffffffu, mx, off);
-        mn = a2 < mn ? a2 : mn;
-        mx = b2 > mx ? b2 : mx;
-      }
-      W.K[c] = __shfl_sync(0xffffffffu, k, 31);
-      W.mn[c] = mn;
-      W.mx[c] = mx;
-      if (__all_sync(0xffffffffu, good) && mn > -L53 && mx < L53) W.ok |= 1 << c;
+    long long k = 0;
+    if (good) {
+      const double y = a[q] * ldexp(1.0, 52 - e);
+      // finite, |y| <= 2^53 and not half-way between two integers
+      good = isfinite(y) && fabs(y) <= 9007199254740992.0 && fabs(y - trunc(y)) != 0.5;
+      k = good ? __double2ll_rn(y) : 0;
     }
-    if (lane == 0) {
+    const bool zero = __all_sync(0xffffffffu, a[q] == 0.0);
+    // inclusive prefix over the warp, its total and range
+    for (int off = 1; off < 32; off <<= 1) {
+      const long long y = __shfl_up_sync(0xffffffffu, k, off);
+      if (lane >= off) k += y;
+    }
+    long long mn = k, mx = k;
+    for (int off = 16; off > 0; off >>= 1) {
+      const long long a2 = __shfl_xor_sync(0xffffffffu, mn, off), b2 = __shfl_xor_sync(0xffffffffu, mx, off);
+      mn = a2 < mn ? a2 : mn;
+      mx = b2 > mx ? b2 : mx;
+    }
+    good = __all_sync(0xffffffffu, good) && mn > -kExact53 && mx < kExact53;
+    if (lane == 31) {
+      const ExactRec W{k, mn, mx, e, zero ? kExactZero : (good ? kExactOk : kExactNone)};
       s_wr[q][wid] = W;
       H->wrec[(q * cap + b) * kExactWarps + wid] = W;
     }
   }
   __syncthreads();
-  if (t < NV) {  // thread q composes sum q's chunk record from its warp records
-    const int q = t;
-    ExactRec R;
-    R.e0 = s_wr[q][0].e0;
-    R.ok = 7;
-    for (int c = 0; c < 3; ++c) {
-      long long K = 0, mn = 0x7fffffffffffffffLL, mx = -0x7fffffffffffffffLL;
-      for (int w = 0; w < kExactWarps; ++w) {
-        const ExactRec &Wr = s_wr[q][w];
-        if (!((Wr.ok >> c) & 1)) { R.ok &= ~(1 << c); break; }
-        const long long lo = K + Wr.mn[c], hi = K + Wr.mx[c];
-        mn = lo < mn ? lo : mn;
-        mx = hi > mx ? hi : mx;
-        K += Wr.K[c];
-      }
-      if (!((R.ok >> c) & 1) || mn <= -L53 || mx >= L53 || K <= -L53 || K >= L53) {
-        R.ok &= ~(1 << c);
-        K = mn = mx = 0;
-      }
-      R.K[c] = K;
-      R.mn[c] = mn;
-      R.mx[c] = mx;
-    }
-    if (!(isfinite(s_hint[q]) && s_hint[q] != 0.0)) R.ok = 0;
-    H->crec[q * cap + b] = R;
+  if (wid < NV) {
+    const int q = wid;
+    const ExactRec W = s_wr[q][lane < kExactWarps ? lane : 0];
+    const ExactRec R = exact_compose(W, kExactWarps, s_wr[q][kExactWarps - 1].e);
+    if (lane == 0) { H->crec[q * cap + b] = R; __threadfence(); }
   }
 
-  // 4. group records
+  // 4. group records, by the last chunk of the group
   const long long g = b / kExactGroup;
   const long long g0 = g * kExactGroup;
   const int gsize = (int)((nch - g0) < kExactGroup ? (nch - g0) : kExactGroup);
+  __syncthreads();
   if (t == 0) {
     __threadfence();
     unsigned prev = atomicAdd(&H->gcount[g], 1u);
     s_last = (prev == (unsigned)gsize - 1);
   }
   __syncthreads();
-  if (s_last && wid == 0) {
+  if (!s_last) return false;
+  if (wid < NV) {
     __threadfence();
-#pragma unroll
-    for (int q = 0; q < NV; ++q) {
-      const int E0 = __ldcg(&H->crec[q * cap + g0 + gsize - 1].e0);
-      long long K[3], mn[3], mx[3];
-      int okm = 7;
-#pragma unroll
-      for (int c = 0; c < 3; ++c) { K[c] = 0; mn[c] = 0x7fffffffffffffffLL; mx[c] = -0x7fffffffffffffffLL; }
-      // two chunks per lane, in order
-      for (int h = 0; h < 2; ++h) {
-        const int jj = 2 * lane + h;
-        if (jj >= gsize) continue;
-        const ExactRec *R = &H->crec[q * cap + g0 + jj];
-        const int e0 = __ldcg(&R->e0), ok = __ldcg(&R->ok);
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          const int cc = E0 + c - e0;
-          if (cc < 0 || cc > 2 || !((ok >> cc) & 1)) { okm &= ~(1 << c); continue; }
-          const long long rk = __ldcg(&R->K[cc]), rn = __ldcg(&R->mn[cc]), rx = __ldcg(&R->mx[cc]);
-          const long long lo = K[c] + rn, hi = K[c] + rx;
-          mn[c] = lo < mn[c] ? lo : mn[c];
-          mx[c] = hi > mx[c] ? hi : mx[c];
-          K[c] += rk;
-        }
-      }
-      // invalid candidates carry zeros so that the sums below stay bounded
-#pragma unroll
-      for (int c = 0; c < 3; ++c)
-        if (!((okm >> c) & 1)) { K[c] = 0; mn[c] = 0; mx[c] = 0; }
-      // exclusive scan of K over the lanes, then min/max of excl + lane range
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        long long incl = K[c];
-        for (int off = 1; off < 32; off <<= 1) {
-          long long y = __shfl_up_sync(0xffffffffu, incl, off);
-          if (lane >= off) incl += y;
-        }
-        const long long excl = incl - K[c];
-        long long lo = 2 * lane < gsize ? excl + mn[c] : 0x7fffffffffffffffLL;
-        long long hi = 2 * lane < gsize ? excl + mx[c] : -0x7fffffffffffffffLL;
-        for (int off = 16; off > 0; off >>= 1) {
-          long long a2 = __shfl_down_sync(0xffffffffu, lo, off), b2 = __shfl_down_sync(0xffffffffu, hi, off);
-          lo = a2 < lo ? a2 : lo;
-          hi = b2 > hi ? b2 : hi;
-        }
-        const long long total = __shfl_sync(0xffffffffu, incl, 31);
-        const bool allok = __all_sync(0xffffffffu, (2 * lane >= gsize) || ((okm >> c) & 1));
-        if (lane == 0) {
-          s_rec.K[c] = total;
-          s_rec.mn[c] = lo;
-          s_rec.mx[c] = hi;
-          const long long L = 1LL << 53;
-          bool good = allok && lo > -L && hi < L && total > -L && total < L;
-          if (c == 0) s_rec.ok = 0;
-          if (good) s_rec.ok |= 1 << c;
-        }
-      }
-      if (lane == 0) {
-        s_rec.e0 = E0;
-        H->grec[q * capg + g] = s_rec;
-      }
-      __syncwarp();
+    const int q = wid;
+    const ExactRec none{0, 0, 0, 0, kExactNone};
+    const int c0 = gsize < 32 ? gsize : 32, c1 = gsize - c0;
+    const ExactRec A = lane < c0 ? exact_load(&H->crec[q * cap + g0 + lane]) : none;
+    const ExactRec B = lane < c1 ? exact_load(&H->crec[q * cap + g0 + 32 + lane]) : none;
+    const int E = __shfl_sync(0xffffffffu, c1 > 0 ? B.e : A.e, (c1 > 0 ? c1 : c0) - 1);
+    const ExactRec RA = exact_compose(A, c0, E), RB = exact_compose(B, c1, E);
+    const ExactRec R = exact_compose(lane == 0 ? RA : RB, c1 > 0 ? 2 : 1, E);
+    if (lane == 0) {
+      H->grec[q * capg + g] = R;
+      if (q == 0) H->gcount[g] = 0u;
+      __threadfence();
     }
-    if (lane == 0) H->gcount[g] = 0u;
   }
+  __syncthreads();
 
   // 5. the last block walks the groups; warp q walks sum q
   if (t == 0) {
     __threadfence();
     unsigned prev = atomicAdd(count, 1u);
-    s_last = (prev == (unsigned)nch - 1);
+    s_last = (prev == (unsigned)((nch + kExactGroup - 1) / kExactGroup) - 1);   // the last group's block
   }
   __syncthreads();
   if (!s_last) return false;
   __threadfence();
   if (wid < NV) {
-    const double r = exact_walk(H, seq, n, nch, wid, cap, capg, s_wrec[wid], s_wr[wid], s_wterm[wid]);
+    const double r = exact_walk(H, seq, n, nch, wid, cap, capg, s_wterm[wid]);
     if (lane == 0) s_res[wid] = r;
   }
   __syncthreads();
