@@ -42,6 +42,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "pbg_word.cuh"
+
 namespace pbg {
 
 constexpr int kExactChunkThreads = 256;  // terms per chunk (the reducing block)
@@ -62,12 +64,11 @@ struct ExactHdr {
   ExactRec *wrec;      // [kExactVals][cap_chunks][kExactWarps] (32 terms each)
   ExactRec *crec;      // [kExactVals][cap_chunks]
   ExactRec *grec;      // [kExactVals][cap_groups]
-  double *agg;         // [kExactVals][cap_chunks] chunk sums (hints)
-  double *incl;        // [kExactVals][cap_chunks] inclusive prefixes (hints)
-  unsigned *flag;      // [cap_chunks] (gen << 2) | 1 sums published, 2 prefix published
+  TagWord *sum;        // [kExactVals][cap_chunks] hints: the chunk's sum, tag (gen << 2) | 1,
+                       // then the sum of all chunks up to it, tag (gen << 2) | 2
   unsigned *gcount;    // [cap_groups] chunk arrivals per group, zero between uses
   long long cap_chunks, cap_groups;
-  unsigned gen;        // launch generation of the look-back flags
+  unsigned gen;        // launch generation of the hints' tags
   unsigned pad;
 };
 constexpr size_t kExactHdrBytes = 256;
@@ -80,8 +81,8 @@ inline size_t exact_scratch_doubles(long long ncell) {
   const long long gr = (ch + kExactGroup - 1) / kExactGroup + 1;
   size_t bytes = kExactHdrBytes + sizeof(double) * (size_t)kExactVals * ncell;
   bytes += sizeof(ExactRec) * kExactVals * (size_t)(ch * (kExactWarps + 1) + gr);
-  bytes += sizeof(double) * 2 * kExactVals * (size_t)ch;
-  bytes += sizeof(unsigned) * (size_t)(ch + gr) + 1024;
+  bytes += sizeof(TagWord) * kExactVals * (size_t)ch;
+  bytes += sizeof(unsigned) * (size_t)gr + 1024;
   return (bytes + 7) / 8;
 }
 inline double *exact_seq(double *base) { return base + kExactHdrBytes / 8; }
@@ -106,6 +107,23 @@ __device__ __forceinline__ ExactRec exact_load(const ExactRec *s) {
 }
 
 constexpr long long kExact53 = 1LL << 53;
+
+// Exponent and integer significand of a normal double, and back: s = S *
+// 2^(e-52), 2^52 <= |S| < 2^53.
+__device__ __forceinline__ int exact_exp(double s) { return (int)((__double2hiint(s) >> 20) & 0x7ff) - 1023; }
+__device__ __forceinline__ long long exact_int(double s) {
+  const long long b = __double_as_longlong(s), m = (b & ((1LL << 52) - 1)) | (1LL << 52);
+  return b < 0 ? -m : m;
+}
+__device__ __forceinline__ double exact_double(long long S, int e) {
+  const long long m = S < 0 ? -S : S;
+  const long long b = (m & ((1LL << 52) - 1)) | ((long long)(e + 1023) << 52);
+  return __longlong_as_double(S < 0 ? b | (long long)0x8000000000000000ULL : b);
+}
+// 2^e, -1022 <= e <= 1023
+__device__ __forceinline__ double exact_pow2(int e) { return __longlong_as_double((long long)(e + 1023) << 52); }
+// the exponents the records cover (s normal, and its unit and 2^53 units too)
+__device__ __forceinline__ bool exact_in_range(int e) { return e >= -960 && e <= 960; }
 
 // Composition of the records of a warp's lanes (lane < cnt, in lane order)
 // into one, the same in every lane. e: the exponent they must share.
@@ -151,7 +169,7 @@ struct ExactWalk {
 
 __device__ __forceinline__ void exact_walk_flush(ExactWalk &w) {
   if (w.in) {
-    w.s = ldexp((double)w.S, w.e - 52);
+    w.s = exact_double(w.S, w.e);
     w.in = false;
   }
 }
@@ -160,14 +178,10 @@ __device__ __forceinline__ void exact_walk_flush(ExactWalk &w) {
 // is not provably the sequential result; returns its lane (cnt: all applied).
 __device__ __forceinline__ int exact_walk_run(ExactWalk &w, const ExactRec &r, int first, int cnt) {
   const int lane = threadIdx.x & 31;
-  if (!w.in && w.s != 0.0 && isfinite(w.s)) {
-    const int e = ilogb(w.s);
-    if (e >= -960 && e <= 1000) {
-      const long long S = (long long)ldexp(fabs(w.s), 52 - e);  // exact
-      w.S = w.s < 0.0 ? -S : S;
-      w.e = e;
-      w.in = true;
-    }
+  if (!w.in && exact_in_range(exact_exp(w.s))) {
+    w.S = exact_int(w.s);
+    w.e = exact_exp(w.s);
+    w.in = true;
   }
   const bool mine = lane >= first && lane < cnt;
   const bool use = mine && r.ok == kExactOk && w.in && r.e == w.e;
@@ -255,7 +269,8 @@ __device__ bool exact_reduce(const double (&v)[NV], double *seq, long long n, un
   const long long p = b * kExactChunkThreads + t;
 
   __shared__ double s_agg[NV][NW];
-  __shared__ double s_hint[NV];
+  __shared__ double s_hint[NV], s_part[NW];
+  __shared__ int s_look[2][NW];
   __shared__ ExactRec s_wr[NV][kExactWarps];
   __shared__ bool s_last;
   __shared__ double s_wterm[kExactVals][kExactChunkThreads];
@@ -269,7 +284,7 @@ __device__ bool exact_reduce(const double (&v)[NV], double *seq, long long n, un
     if (p < n) seq[q * n + p] = v[q];
   }
 
-  // 2. chunk sums and the look-back hint
+  // 2. chunk sums and the look-back for the hint
 #pragma unroll
   for (int q = 0; q < NV; ++q) {
     double x = a[q];
@@ -277,67 +292,51 @@ __device__ bool exact_reduce(const double (&v)[NV], double *seq, long long n, un
     if (lane == 0) s_agg[q][wid] = x;
   }
   __syncthreads();
-  if (wid == 0) {
-    double my[NV];
+  // 256 chunks before this one at a time, a thread each, back to the first
+  // that has published the sum of all up to it
 #pragma unroll
-    for (int q = 0; q < NV; ++q) {
-      double x = 0.0;
-      for (int w = 0; w < NW; ++w) x += s_agg[q][w];
-      my[q] = x;
-    }
-    if (lane == 0) {
-#pragma unroll
-      for (int q = 0; q < NV; ++q) H->agg[q * cap + b] = my[q];
-      __threadfence();
-      atomicExch(&H->flag[b], (gen << 2) | 1u);
-    }
-    __syncwarp();
-    double pre[NV];
-#pragma unroll
-    for (int q = 0; q < NV; ++q) pre[q] = 0.0;
+  for (int q = 0; q < NV; ++q) {
+    TagWord *W = H->sum + q * cap;
+    const unsigned long long t1 = ((unsigned long long)gen << 2) | 1u, t2 = t1 + 1;
+    double mine = 0.0;
+    for (int w = 0; w < NW; ++w) mine += s_agg[q][w];
+    if (t == 0 && b > 0) word_st(W + b, mine, t1);
+    double pre = 0.0;
     bool okh = true;
-    long long top = b - 1;
     int polls = 0;
-    while (top >= 0) {
-      const long long j = top - lane;
-      int st = 2;  // before the first chunk: an inclusive prefix of zero
-      if (j >= 0) {
-        unsigned f = ld_volatile_u32(&H->flag[j]);
-        st = ((f >> 2) == gen) ? (int)(f & 3u) : 0;
+    for (long long top = b - 1; top >= 0;) {
+      const long long j = top - t;
+      const TagWord x = j >= 0 ? word_ld(W + j) : TagWord{0ull, t2};
+      const unsigned incl = __ballot_sync(0xffffffffu, x.tag == t2);
+      const unsigned none = __ballot_sync(0xffffffffu, x.tag != t1 && x.tag != t2);
+      if (lane == 0) {
+        s_look[0][wid] = incl ? 32 * wid + __ffs(incl) - 1 : kExactChunkThreads;
+        s_look[1][wid] = none ? 32 * wid + __ffs(none) - 1 : kExactChunkThreads;
       }
-      const unsigned incl = __ballot_sync(0xffffffffu, st == 2);
-      const unsigned notr = __ballot_sync(0xffffffffu, st == 0);
-      const int fi = incl ? __ffs(incl) - 1 : 32;
-      const unsigned need = fi == 32 ? 0xffffffffu : ((2u << fi) - 1u);
-      if (notr & need) {
+      __syncthreads();
+      int fi = kExactChunkThreads, fn = kExactChunkThreads;
+#pragma unroll
+      for (int w = 0; w < NW; ++w) { fi = min(fi, s_look[0][w]); fn = min(fn, s_look[1][w]); }
+      double y = t <= fi ? __longlong_as_double((long long)x.v) : 0.0;
+      if (fn < fi) {   // a chunk between has not published yet
+        __syncthreads();
         if (++polls > kExactPoll) { okh = false; break; }
-        __nanosleep(32);
         continue;
       }
-      __threadfence();
-#pragma unroll
-      for (int q = 0; q < NV; ++q) {
-        double x = 0.0;
-        if (j >= 0 && lane < fi) x = __ldcg(&H->agg[q * cap + j]);
-        else if (j >= 0 && lane == fi) x = __ldcg(&H->incl[q * cap + j]);
-        for (int off = 16; off > 0; off >>= 1) x += __shfl_down_sync(0xffffffffu, x, off);
-        pre[q] += __shfl_sync(0xffffffffu, x, 0);
-      }
-      if (fi < 32) break;
-      top -= 32;
+      for (int off = 16; off > 0; off >>= 1) y += __shfl_down_sync(0xffffffffu, y, off);
+      if (lane == 0) s_part[wid] = y;
+      __syncthreads();
+      for (int w = 0; w < NW; ++w) pre += s_part[w];
+      if (fi < kExactChunkThreads) break;
+      top -= kExactChunkThreads;
+      __syncthreads();
     }
-    if (lane == 0) {
-#pragma unroll
-      for (int q = 0; q < NV; ++q) s_hint[q] = okh ? pre[q] : __longlong_as_double(0x7ff8000000000000LL);
-      if (okh) {
-#pragma unroll
-        for (int q = 0; q < NV; ++q) H->incl[q * cap + b] = pre[q] + my[q];
-        __threadfence();
-        atomicExch(&H->flag[b], (gen << 2) | 2u);
-      }
+    if (t == 0) {
+      s_hint[q] = okh ? pre : __longlong_as_double(0x7ff8000000000000LL);
+      if (okh) word_st(W + b, pre + mine, t2);
     }
+    __syncthreads();
   }
-  __syncthreads();
 
   // 3. one record per warp (32 terms) at the exponent of the approximate sum
   // before it, composed by warp q into sum q's chunk record
@@ -345,15 +344,11 @@ __device__ bool exact_reduce(const double (&v)[NV], double *seq, long long n, un
   for (int q = 0; q < NV; ++q) {
     double before = s_hint[q];
     for (int w = 0; w < wid; ++w) before += s_agg[q][w];
-    int e = 0;
-    bool good = isfinite(before) && before != 0.0;
-    if (good) {
-      e = ilogb(before);
-      good = e >= -960 && e <= 1000;
-    }
+    const int e = exact_exp(before);   // zero, infinite and NaN hints fall outside the range
+    bool good = exact_in_range(e);
     long long k = 0;
     if (good) {
-      const double y = a[q] * ldexp(1.0, 52 - e);
+      const double y = a[q] * exact_pow2(52 - e);
       // finite, |y| <= 2^53 and not half-way between two integers
       good = isfinite(y) && fabs(y) <= 9007199254740992.0 && fabs(y - trunc(y)) != 0.5;
       k = good ? __double2ll_rn(y) : 0;

@@ -136,16 +136,16 @@ void exact_scratch_init(double *base, long long ncell, cudaStream_t s) {
   h.wrec = reinterpret_cast<ExactRec *>(q); q += sizeof(ExactRec) * kExactVals * (size_t)ch * kExactWarps;
   h.crec = reinterpret_cast<ExactRec *>(q); q += sizeof(ExactRec) * kExactVals * (size_t)ch;
   h.grec = reinterpret_cast<ExactRec *>(q); q += sizeof(ExactRec) * kExactVals * (size_t)gr;
-  h.agg = reinterpret_cast<double *>(q); q += sizeof(double) * kExactVals * (size_t)ch;
-  h.incl = reinterpret_cast<double *>(q); q += sizeof(double) * kExactVals * (size_t)ch;
-  h.flag = reinterpret_cast<unsigned *>(q); q += sizeof(unsigned) * (size_t)ch;
+  q += (16 - reinterpret_cast<size_t>(q) % 16) % 16;
+  h.sum = reinterpret_cast<TagWord *>(q); q += sizeof(TagWord) * kExactVals * (size_t)ch;
   h.gcount = reinterpret_cast<unsigned *>(q); q += sizeof(unsigned) * (size_t)gr;
   h.cap_chunks = ch;
   h.cap_groups = gr;
   h.gen = 1;
   if ((size_t)(q - reinterpret_cast<char *>(base)) > exact_scratch_doubles(ncell) * sizeof(double))
     throw CudaError("exact-sum scratch layout exceeds its allocation");
-  PBG_CUDA(cudaMemsetAsync(h.flag, 0, sizeof(unsigned) * (size_t)(ch + gr), s));
+  PBG_CUDA(cudaMemsetAsync(h.sum, 0, sizeof(TagWord) * kExactVals * (size_t)ch, s));
+  PBG_CUDA(cudaMemsetAsync(h.gcount, 0, sizeof(unsigned) * (size_t)gr, s));
   PBG_CUDA(cudaMemcpyAsync(base, &h, sizeof(h), cudaMemcpyHostToDevice, s));
   PBG_CUDA(cudaStreamSynchronize(s));
 }

@@ -33,7 +33,7 @@ struct RefKrylovWork {
   const double *rhs = nullptr, *ci = nullptr;     // Jacobi / Gauss-Seidel operands of a solve
   DBuf<double> z, mc, mw, ms, mb, mtw, mts, mnw;  // IC preconditioner: z, and IC3's factor
   DBuf<double> mo;                                // sweeps: operands in march order
-  DBuf<SweepWord> words;                          // sweeps: exchange between tiles
+  DBuf<TagWord> words;                          // sweeps: exchange between tiles
   DBuf<unsigned> ticket;                          // sweeps: tickets [0..1], the stuck flag [2]
   unsigned long long epoch = 0;                   // sweeps: the last launch's epoch
   int *hstuck = nullptr;                          // pinned copy of the stuck flag

@@ -5,17 +5,6 @@
 
 namespace pbg {
 
-__device__ __forceinline__ SweepWord sweep_ld(const SweepWord *p) {
-  SweepWord w;
-  asm volatile("{\n\t.reg .b128 q;\n\tld.relaxed.gpu.global.b128 q, [%2];\n\tmov.b128 {%0, %1}, q;\n\t}"
-               : "=l"(w.v), "=l"(w.epoch) : "l"(p) : "memory");
-  return w;
-}
-__device__ __forceinline__ void sweep_st(SweepWord *p, double v, unsigned long long epoch) {
-  asm volatile("{\n\t.reg .b128 q;\n\tmov.b128 q, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], q;\n\t}"
-               :: "l"(p), "l"((unsigned long long)__double_as_longlong(v)), "l"(epoch) : "memory");
-}
-
 // a / c with c's stored reciprocal y: KnownDiv with its range checks on the
 // exponents, beside the dependent operations instead of before them. A zero
 // dividend comes out right for +0 only; everything else outside the range,
@@ -48,11 +37,11 @@ __device__ __forceinline__ void sweep_finish(const SweepSync &y, int tiles) {
 // Waits until word p carries this launch's epoch and returns it. A poll that
 // runs out (or one that did elsewhere) sets *stuck and gives up with zero, so
 // that every block ends; the host reports the failure.
-__device__ __noinline__ SweepWord sweep_poll(const SweepWord *p, const SweepSync &y, bool &dead) {
-  SweepWord a = {0ull, 0ull};
+__device__ __noinline__ TagWord sweep_poll(const TagWord *p, const SweepSync &y, bool &dead) {
+  TagWord a = {0ull, 0ull};
   for (int m = 1; !dead; ++m) {
-    a = sweep_ld(p);
-    if (a.epoch == y.epoch) break;
+    a = word_ld(p);
+    if (a.tag == y.epoch) break;
     if (m >= kSweepPoll) { atomicExch(y.stuck, 1); dead = true; }
     else if ((m & 1023) == 0 && *(volatile int *)y.stuck) dead = true;
     a.v = 0ull;
@@ -111,7 +100,7 @@ __device__ __forceinline__ void sweep_march(const SweepGeo &g, const SweepSync &
   if (warp == 2) {
     const SweepPos<BWD> q(g, tile, along_i ? 0 : m, along_i ? m : 0);
     const bool on = used && (along_i ? q.hasW : q.hasS);
-    const SweepWord *p = along_i ? y.words + ((size_t)(q.I - 1) * g.ny + q.j) * nz
+    const TagWord *p = along_i ? y.words + ((size_t)(q.I - 1) * g.ny + q.j) * nz
                                  : y.words + g.words_i() + ((size_t)(q.J - 1) * g.nx + q.i) * nz;
     const int at = along_i ? m + 1 : (m + 1) * E;
     int ke = -A * m;   // the beside column's k of the block's first read
@@ -119,19 +108,19 @@ __device__ __forceinline__ void sweep_march(const SweepGeo &g, const SweepSync &
     for (int t0 = 0; t0 < T; t0 += P, ke += P) {
       // halo for the reads of steps t0 .. t0 + P - 1, in the slots before them
       const int slot0 = (t0 + 2 * P - 1) % (2 * P);
-      SweepWord w[P][NV];
+      TagWord w[P][NV];
       auto fetch = [&] {
         bool ok = true;
 #pragma unroll
         for (int u = 0; u < P; ++u)
 #pragma unroll
           for (int v = 0; v < NV; ++v)
-            if (on && (unsigned)(ke + u) < (unsigned)nz) w[u][v] = sweep_ld(p + ke + u + v * g.words());
+            if (on && (unsigned)(ke + u) < (unsigned)nz) w[u][v] = word_ld(p + ke + u + v * g.words());
 #pragma unroll
         for (int u = 0; u < P; ++u)
 #pragma unroll
           for (int v = 0; v < NV; ++v)
-            if (on && (unsigned)(ke + u) < (unsigned)nz && w[u][v].epoch != y.epoch) ok = false;
+            if (on && (unsigned)(ke + u) < (unsigned)nz && w[u][v].tag != y.epoch) ok = false;
         return ok;
       };
       if (!fetch()) {   // caught up with the neighbour: wait for the block's last word first
@@ -143,7 +132,7 @@ __device__ __forceinline__ void sweep_march(const SweepGeo &g, const SweepSync &
 #pragma unroll
         for (int v = 0; v < NV; ++v)
           if (on && (unsigned)(ke + u) < (unsigned)nz) {
-            if (w[u][v].epoch != y.epoch) w[u][v] = sweep_poll(p + ke + u + v * g.words(), y, dead);
+            if (w[u][v].tag != y.epoch) w[u][v] = sweep_poll(p + ke + u + v * g.words(), y, dead);
             ring[(slot0 + u) % (2 * P)][v * E * E + at] = __longlong_as_double((long long)w[u][v].v);
           }
       block_barrier();
@@ -153,7 +142,7 @@ __device__ __forceinline__ void sweep_march(const SweepGeo &g, const SweepSync &
     const int start = -A * (last + m) - LOOK;
     const bool on = used && q.col;
     const int at = (q.li + 1) * E + q.lj + 1;
-    SweepWord *p = (along_i ? y.words + ((size_t)q.I * g.ny + q.j) * nz
+    TagWord *p = (along_i ? y.words + ((size_t)q.I * g.ny + q.j) * nz
                             : y.words + g.words_i() + ((size_t)q.J * g.nx + q.i) * nz) + start;
     step_barrier();
     for (int t0 = 0, h = 0; t0 < T; t0 += P, h = P - h) {
@@ -162,7 +151,7 @@ __device__ __forceinline__ void sweep_march(const SweepGeo &g, const SweepSync &
         step_barrier();
         if (on && (unsigned)(start + t0 + u) < (unsigned)nz)
 #pragma unroll
-          for (int v = 0; v < NV; ++v) sweep_st(p + u + v * g.words(), ring[h + u][v * E * E + at], y.epoch);
+          for (int v = 0; v < NV; ++v) word_st(p + u + v * g.words(), ring[h + u][v * E * E + at], y.epoch);
       }
       p += P;
     }

@@ -33,6 +33,7 @@
 
 #include "pbg_common.cuh"
 #include "pbg_session.h"
+#include "pbg_word.cuh"
 
 namespace pbg {
 
@@ -48,9 +49,6 @@ constexpr int kSweepSkewMin = 32;
 // weight a = b of the schedule: IC0 (kind 1) and Gauss-Seidel read the
 // columns beside a cell at its own k, IC2 (kind 2) also at k + 1
 __host__ __device__ constexpr int sweep_a(int kind) { return kind == 2 ? 2 : 1; }
-
-// A (value, epoch) word of the exchange between tiles, moved as 16 bytes.
-struct alignas(16) SweepWord { unsigned long long v, epoch; };
 
 // Tiles of a grid and the march-order storage of a cell array.
 struct SweepGeo {
@@ -83,7 +81,7 @@ struct SweepGeo {
 
 // Shared state of the sweeps of one solver's workspace.
 struct SweepSync {
-  SweepWord *words;             // exchange, SweepGeo::words() per value
+  TagWord *words;             // exchange, SweepGeo::words() per value
   unsigned *ticket;             // [0] next tile, [1] finished tiles (both 0 between launches)
   int *stuck;                   // set when a poll ran out
   unsigned long long epoch;     // of this launch, larger than any before it
