@@ -25,14 +25,31 @@ struct LevelOut {
 __global__ void k_level_finish(EMat<double> A, LevelOut o) {
   GRID_LOOP(p, A.g.n) {
     const double c = A.c[p];
-    o.d[p] = 1.0 / c;
+    const double d = c != 0.0 ? 1.0 / c : 0.0;   // a pad cell has no diagonal and stays zero
+    o.d[p] = d;
     if (o.c32) {
       const Pos q = A.g.pos(p);
       const double sum = offdiag(A, p, q, [](uint32_t) { return 1.0; });
       o.c32[p] = (float)(c - sum);
       o.w32[p] = (float)A.w[p]; o.s32[p] = (float)A.s[p]; o.b32[p] = (float)A.b[p];
-      o.d32[p] = (float)(1.0 / c);
+      o.d32[p] = (float)d;
     }
+  }
+}
+
+// Level 0 of the hierarchy in padded rows (RowPad) from the caller's: in 2-D
+// the j couplings become the row's.
+__global__ void k_pad_matrix(EMat<double> A, RowPad P, uint32_t rows, FastDiv dFP, double *__restrict__ c,
+                             double *__restrict__ w, double *__restrict__ s, double *__restrict__ b) {
+  GRID_LOOP(pp, rows * (uint32_t)P.FP) {
+    const uint32_t row = dFP.div(pp);
+    const int f = (int)(pp - row * (uint32_t)P.FP);
+    const bool in = f < P.F;
+    const uint32_t p = row * (uint32_t)P.F + (in ? f : 0);
+    c[pp] = in ? A.c[p] : 0.0;
+    w[pp] = in ? A.w[p] : 0.0;
+    s[pp] = in && !P.two_d ? A.s[p] : 0.0;
+    b[pp] = in ? (P.two_d ? A.s[p] : A.b[p]) : 0.0;
   }
 }
 
@@ -176,6 +193,12 @@ __global__ void __launch_bounds__(256) k_gj_block(int n, int k0, const double *_
 }
 
 
+// Grids whose rows are padded: below kPadMin the passes are bound by their
+// chains of loads whatever the rows, and the pad cells would be a larger
+// share of the level; above kPadMax the copy of the operator (32 bytes a
+// cell) could cost a grid its place in device memory.
+constexpr long long kPadMin = 4096, kPadMax = 1ll << 28;
+
 template <typename T>
 void EWork<T>::ensure(const std::vector<ELevel> &lv) {
   if (L.size() == lv.size() && x0.n == (size_t)lv[0].ncell()) return;
@@ -194,6 +217,9 @@ void EWork<T>::ensure(const std::vector<ELevel> &lv) {
   ks.alloc(lv.size());
   fs.alloc(1);
   PBG_CUDA(cudaMemset(fs.p, 0, sizeof(FcgScal)));
+  // the refinement's residual is written to the cells of padded rows only
+  PBG_CUDA(cudaMemset(L[0].b.p, 0, L[0].b.bytes()));
+  PBG_CUDA(cudaStreamSynchronize(0));
 }
 
 template <typename T>
@@ -340,18 +366,41 @@ void Engine::dense_solve(const T *r, T *z, const int *stop, cudaStream_t s) {
   launch_pdl(k_dense_solve<T, AT>, blocks, kThreads, s, ncoarse, (const AT *)ainv<T>(), r, z, stop);
 }
 
-void Engine::build(const EMat<double> &A0, cudaStream_t s, bool mixed) {
+void Engine::build(const EMat<double> &A0_, cudaStream_t s, bool mixed) {
   w64.drop_graph();
   w32.drop_graph();
   w64.L.clear();
   w32.L.clear();
   L.clear();
+  // levels of the grid itself, as pbg_levels and the results report them
+  report.clear();
+  report.push_back({A0_.nx, A0_.ny, A0_.nz});
+  for (;;) {
+    const Dims d = report.back();
+    if ((long long)d.nx * d.ny * d.nz <= opt.coarse_max || (d.nx == 1 && d.ny == 1 && d.nz == 1)) break;
+    report.push_back({d.nx > 1 ? (d.nx + 1) / 2 : 1, d.ny > 1 ? (d.ny + 1) / 2 : 1, d.nz > 1 ? (d.nz + 1) / 2 : 1});
+  }
+  A0 = A0_;
+  const int V = mixed ? VecTraits<float>::V : VecTraits<double>::V;
+  auto up = [V](int n) { return (n + V - 1) / V * V; };
+  pad = RowPad();
+  const bool padded = A0.ncell() >= kPadMin && A0.ncell() <= kPadMax;
+  pad.two_d = padded && A0.nz == 1 && A0.ny > 1;
+  pad.F = pad.two_d ? A0.ny : A0.nz;
+  pad.FP = padded ? up(pad.F) : pad.F;
   L.emplace_back();
   {
     ELevel &l0 = L[0];
-    l0.nx = A0.nx; l0.ny = A0.ny; l0.nz = A0.nz;
+    l0.nx = A0.nx; l0.ny = pad.two_d ? 1 : A0.ny; l0.nz = pad.FP;
     l0.d64.alloc(l0.ncell());
-    l0.m64 = make_emat<double>(A0.nx, A0.ny, A0.nz, A0.c, A0.w, A0.s, A0.b, l0.d64.p);
+    if (pad.any()) {
+      for (DBuf<double> *a : {&pc, &pw, &ps, &pb})
+        if (a->n != (size_t)l0.ncell()) a->alloc(l0.ncell());
+      l0.m64 = make_emat<double>(l0.nx, l0.ny, l0.nz, pc.p, pw.p, ps.p, pb.p, l0.d64.p);
+    } else {
+      for (DBuf<double> *a : {&pc, &pw, &ps, &pb}) a->release();
+      l0.m64 = make_emat<double>(A0.nx, A0.ny, A0.nz, A0.c, A0.w, A0.s, A0.b, l0.d64.p);
+    }
   }
   while (L.back().ncell() > opt.coarse_max &&
          (L.back().nx > 1 || L.back().ny > 1 || L.back().nz > 1)) {
@@ -360,6 +409,7 @@ void Engine::build(const EMat<double> &A0, cudaStream_t s, bool mixed) {
     c.nx = f.nx > 1 ? (f.nx + 1) / 2 : 1;
     c.ny = f.ny > 1 ? (f.ny + 1) / 2 : 1;
     c.nz = f.nz > 1 ? (f.nz + 1) / 2 : 1;
+    if (padded && c.ncell() >= kPadMin) c.nz = up(c.nz);   // rows of whole vectors here too
     long long n = c.ncell();
     c.c64.alloc(n); c.w64.alloc(n); c.s64.alloc(n); c.b64.alloc(n); c.d64.alloc(n);
     c.m64 = make_emat<double>(c.nx, c.ny, c.nz, c.c64.p, c.w64.p, c.s64.p, c.b64.p, c.d64.p);
@@ -404,6 +454,11 @@ void Engine::compute(cudaStream_t s) {
     if (have32) { o.c32 = lv.c32.p; o.w32 = lv.w32.p; o.s32 = lv.s32.p; o.b32 = lv.b32.p; o.d32 = lv.d32.p; }
     return o;
   };
+  if (pad.any()) {
+    const uint32_t rows = (uint32_t)(L[0].ncell() / pad.FP);
+    k_pad_matrix<<<grid_for(L[0].ncell()), kThreads, 0, s>>>(A0, pad, rows, FastDiv((uint32_t)pad.FP), pc.p, pw.p,
+                                                             ps.p, pb.p); note_launch();
+  }
   k_level_finish<<<grid_for(L[0].ncell()), kThreads, 0, s>>>(L[0].m64, out(L[0])); note_launch();
   for (size_t l = 1; l < L.size(); ++l) {
     ELevel &c = L[l];
@@ -437,9 +492,9 @@ void Engine::compute(cudaStream_t s) {
 
 // Numeric refresh for a changed fine matrix of the same shape at the same
 // addresses; false if the hierarchy has to be built anew.
-bool Engine::refresh(const EMat<double> &A0, bool mixed, cudaStream_t s) {
-  if (L.empty() || (mixed && !have32) || L[0].nx != A0.nx || L[0].ny != A0.ny || L[0].nz != A0.nz ||
-      L[0].m64.c != A0.c || L[0].m64.w != A0.w || L[0].m64.s != A0.s || L[0].m64.b != A0.b)
+bool Engine::refresh(const EMat<double> &A, bool mixed, cudaStream_t s) {
+  if (L.empty() || (mixed && !have32) || A0.nx != A.nx || A0.ny != A.ny || A0.nz != A.nz ||
+      A0.c != A.c || A0.w != A.w || A0.s != A.s || A0.b != A.b)
     return false;
   compute(s);
   return true;
@@ -683,13 +738,13 @@ void symmetrize(const MatView<double> &A, double *c, double *w, double *s, doubl
 // rounding into rT, and |r|^2, |b|^2 into dsc[0..1].
 template <typename T>
 void Engine::true_resid(const double *x, const double *b, T *rT, RedPool &red, cudaStream_t s) {
-  const EMat<double> A = L[0].m64;
+  const EMat<double> A = A0;
   const int g = grid_for(A.ncell());
   if (nonsym)
-    k_true_resid_ns<T><<<g, kThreads, 0, s>>>(top, A.g, x, b, nullptr, rT, dsc.p, red.slot_part(0),
+    k_true_resid_ns<T><<<g, kThreads, 0, s>>>(top, A.g, x, b, rT, pad, dsc.p, red.slot_part(0),
                                               red.slot_count(0));
   else
-    k_true_resid<T><<<g, kThreads, 0, s>>>(A, x, b, nullptr, rT, dsc.p, red.slot_part(0), red.slot_count(0));
+    k_true_resid<T><<<g, kThreads, 0, s>>>(A, x, b, rT, pad, dsc.p, red.slot_part(0), red.slot_count(0));
   note_launch();
 }
 
@@ -712,7 +767,7 @@ void Engine::restore_iterate(double *x, long long N, cudaStream_t s) {
 EngineResult Engine::solve_fp64(double *x, const double *b, double tol, int maxit, RedPool &red,
                                 cudaStream_t s, double *hist) {
   w64.ensure(L);
-  const EMat<double> A = L[0].m64;
+  const EMat<double> A = A0;
   const long long N = A.ncell();
   const int g = grid_for(N);
   FcgScal *hfs = (FcgScal *)hsc;
@@ -733,7 +788,7 @@ EngineResult Engine::solve_fp64(double *x, const double *b, double tol, int maxi
     res.iterations += its;
     res.sweeps++;
     keep_iterate(x, N, s);
-    k_add_corr<double><<<g, kThreads, 0, s>>>(N, x, w64.x0.p); note_launch();
+    k_add_corr<double><<<g, kThreads, 0, s>>>(A.g, x, w64.x0.p, pad); note_launch();
     true_resid<double>(x, b, rhs, red, s);
     PBG_CUDA(cudaMemcpyAsync(hsc + 32, dsc.p, 2 * sizeof(double), cudaMemcpyDeviceToHost, s));
     PBG_CUDA(cudaStreamSynchronize(s));
@@ -753,7 +808,7 @@ EngineResult Engine::solve_mixed(double *x, const double *b, double tol, double 
                                  int max_sweeps, int inner_maxit, RedPool &red, cudaStream_t s,
                                  double *hist) {
   w32.ensure(L);
-  const EMat<double> A = L[0].m64;
+  const EMat<double> A = A0;
   const long long N = A.ncell();
   const int g = grid_for(N);
   FcgScal *hfs = (FcgScal *)hsc;
@@ -775,7 +830,7 @@ EngineResult Engine::solve_mixed(double *x, const double *b, double tol, double 
     res.iterations += its;
     res.sweeps++;
     keep_iterate(x, N, s);
-    k_add_corr<float><<<g, kThreads, 0, s>>>(N, x, w32.x0.p); note_launch();
+    k_add_corr<float><<<g, kThreads, 0, s>>>(A.g, x, w32.x0.p, pad); note_launch();
     true_resid<float>(x, b, rhs, red, s);
     PBG_CUDA(cudaMemcpyAsync(hsc + 32, dsc.p, 2 * sizeof(double), cudaMemcpyDeviceToHost, s));
     PBG_CUDA(cudaStreamSynchronize(s));

@@ -100,9 +100,29 @@ struct EngineResult {
   double relres;             // FP64 true residual |b - A x| / |b|
 };
 
+// Rows of the hierarchy's storage. The 16-byte kernels need rows of a
+// multiple of V cells; a row is a k row in 3-D and a j row in 2-D (a 2-D grid
+// becomes (nx, 1, ny)). A grid whose rows are no such multiple is copied into
+// padded rows for the hierarchy, its pad cells without couplings, diagonal
+// and values; the solution and the right-hand side keep the caller's rows.
+struct RowPad {
+  int F = 0, FP = 0;   // cells of a row, and stored
+  int two_d = 0;
+  __host__ __device__ bool any() const { return two_d || F != FP; }
+  // stored index of cell p at q (3-D rows: i ny + j; 2-D rows: i)
+  __device__ __forceinline__ uint32_t at(uint32_t p, Pos q, int ny) const {
+    return p + (uint32_t)(FP - F) * (uint32_t)(two_d ? q.i : q.i * ny + q.j);
+  }
+};
+
 class Engine {
  public:
   std::vector<ELevel> L;
+  RowPad pad;                          // rows of level 0
+  EMat<double> A0{};                   // the operator in the caller's rows
+  DBuf<double> pc, pw, ps, pb;         // its copy in padded rows
+  struct Dims { int nx, ny, nz; };
+  std::vector<Dims> report;            // levels by the unpadded halving rule
   DBuf<double> Ainv;           // dense inverse of the coarsest operator
   DBuf<float> Ainv32;          // its FP32 copy (mixed path)
   DBuf<__half> Ainv16;         // row-scaled FP16 copy (mixed path, large coarsest levels)
@@ -131,7 +151,7 @@ class Engine {
   EngineResult solve_mixed(double *x, const double *b, double tol, double inner_tol,
                            int max_sweeps, int inner_maxit, RedPool &red, cudaStream_t s,
                            double *hist);
-  int nlevels() const { return (int)L.size(); }
+  int nlevels() const { return (int)report.size(); }
   template <typename T> EMat<T> mat(int l) const;
   template <typename T> const void *ainv() const;
   template <typename T> void dense_solve(const T *r, T *z, const int *stop, cudaStream_t s);

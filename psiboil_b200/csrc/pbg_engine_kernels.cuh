@@ -436,25 +436,28 @@ __global__ void __launch_bounds__(kThreads, 8) k_fcg_init(long long N, const T *
 }
 
 // ---------------------------------------------------------------- refinement
-// x64 += e (T), elementwise
+// x64 += e (T), elementwise; e in the hierarchy's rows
 template <typename T>
-__global__ void __launch_bounds__(kThreads, 8) k_add_corr(long long N, double *__restrict__ x, const T *__restrict__ e) {
+__global__ void __launch_bounds__(kThreads, 8) k_add_corr(Geo G, double *__restrict__ x, const T *__restrict__ e, RowPad pad) {
   PBG_PDL_ENTRY();
-  GRID_LOOP(p, N) x[p] += (double)e[p];
+  if (!pad.any()) {
+    GRID_LOOP(p, G.n) x[p] += (double)e[p];
+  } else {
+    GRID_LOOP(p, G.n) x[p] += (double)e[pad.at(p, G.pos(p), G.ny)];
+  }
 }
 
-// r = b - A x in FP64, r32 = (T) r, out[0] = |r|^2, out[1] = |b|^2
+// r = b - A x in FP64, rT = (T) r in the hierarchy's rows, out[0] = |r|^2,
+// out[1] = |b|^2
 template <typename T>
 __global__ void __launch_bounds__(kThreads, 8) k_true_resid(EMat<double> A, const double *__restrict__ x, const double *__restrict__ b,
-                             double *__restrict__ r, T *__restrict__ rT, double *out, double *part,
-                             unsigned *count) {
+                             T *__restrict__ rT, RowPad pad, double *out, double *part, unsigned *count) {
   PBG_PDL_ENTRY();
   double v[2] = {0.0, 0.0};
   GRID_LOOP(p, A.g.n) {
     Pos q = A.g.pos(p);
     double rv = b[p] - ax_at(A, p, q, x);
-    if (r) r[p] = rv;
-    if (rT) rT[p] = (T)rv;
+    rT[pad.at(p, q, A.ny)] = (T)rv;
     v[0] += rv * rv;
     v[1] += b[p] * b[p];
   }
@@ -467,8 +470,8 @@ __global__ void __launch_bounds__(kThreads, 8) k_true_resid(EMat<double> A, cons
 // its symmetric part: r = b - (c x - sum a_nb x_nb).
 template <typename T>
 __global__ void __launch_bounds__(kThreads, 8) k_true_resid_ns(MatView<double> A, Geo G, const double *__restrict__ x,
-                                const double *__restrict__ b, double *__restrict__ r,
-                                T *__restrict__ rT, double *out, double *part, unsigned *count) {
+                                const double *__restrict__ b, T *__restrict__ rT, RowPad pad, double *out,
+                                double *part, unsigned *count) {
   PBG_PDL_ENTRY();
   const uint32_t SI = G.nynz, SJ = (uint32_t)A.nz;
   double v[2] = {0.0, 0.0};
@@ -483,8 +486,7 @@ __global__ void __launch_bounds__(kThreads, 8) k_true_resid_ns(MatView<double> A
     if (q.k > 0) nb += a.b * x[p - 1];
     if (q.k < A.nz - 1) nb += a.t * x[p + 1];
     const double rv = b[p] - (A.c[p] * x[p] - nb);
-    if (r) r[p] = rv;
-    if (rT) rT[p] = (T)rv;
+    rT[pad.at(p, q, A.ny)] = (T)rv;
     v[0] += rv * rv;
     v[1] += b[p] * b[p];
   }
