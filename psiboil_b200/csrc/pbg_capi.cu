@@ -883,6 +883,7 @@ void ensure_engine(pbg_session *s, bool mixed, int coarse_max) {
   if (!s->eng) s->eng = std::make_unique<Engine>();
   if (coarse_max > 0 && coarse_max != s->eng->opt.coarse_max) {
     s->eng->opt.coarse_max = coarse_max;  // a different hierarchy: build anew
+    s->eng->opt.coarse_auto = false;
     s->eng->L.clear();
     s->eng_dirty = true;
   }

@@ -1,5 +1,6 @@
 // Host side of the engine solver (hierarchy set-up, K-cycle recursion,
 // flexible CG and the mixed-precision refinement loop).
+#include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -104,7 +105,8 @@ __global__ void k_dense_dmax(int n, const double *__restrict__ D, double *dmax) 
 }
 
 constexpr int kGjB = 32;     // pivots per block step
-constexpr int kGjRows = 32;  // rows per CTA (each reuses the pivot rows from L2)
+constexpr int kGjRows = 32;  // rows per CTA
+constexpr int kGjCols = 128; // columns per CTA, two threads a column
 
 // One blocked Gauss-Jordan exchange on the pivots k0 .. k0+kb-1 (out of
 // place, A -> B). With A11 the pivot block, G = A11^-1 (by scalar
@@ -116,6 +118,10 @@ constexpr int kGjRows = 32;  // rows per CTA (each reuses the pivot rows from L2
 // zero, which gives a generalised inverse of a consistent singular system
 // (in a positive semi-definite matrix a zero Schur pivot has a zero row
 // and column, so nothing else changes).
+// A step is bound by its pivot block (32 dependent exchanges with a barrier
+// pair each) and its launch; a CTA of 32 rows x 128 columns keeps the rest,
+// 128 multiply-adds a thread per pivot, below that. 32 rows x all columns
+// took 67 us a step at n = 512, this form 12.
 __global__ void __launch_bounds__(256) k_gj_block(int n, int k0, const double *__restrict__ A,
                                                   double *__restrict__ B, const double *dmax,
                                                   double rel_tol) {
@@ -131,64 +137,62 @@ __global__ void __launch_bounds__(256) k_gj_block(int n, int k0, const double *_
   }
   __syncthreads();
   for (int k = 0; k < kb; ++k) {
-    if (threadIdx.x < kb) { rowk[threadIdx.x] = G[k][threadIdx.x]; colk[threadIdx.x] = G[threadIdx.x][k]; }
+    if (threadIdx.x < kGjB) { rowk[threadIdx.x] = G[k][threadIdx.x]; colk[threadIdx.x] = G[threadIdx.x][k]; }
     __syncthreads();
     const double akk = rowk[k];
     const bool sk = !(akk > thr);
     const double piv = sk ? 0.0 : 1.0 / akk;
-    for (int e = threadIdx.x; e < kb * kb; e += blockDim.x) {
-      const int i = e / kb, j = e - i * kb;
+#pragma unroll
+    for (int u = 0; u < kGjB * kGjB / 256; ++u) {
+      const int e = threadIdx.x + 256 * u, i = e / kGjB, j = e % kGjB;
       double v;
       if (sk) v = (i == k || j == k) ? 0.0 : G[i][j];
       else if (i == k && j == k) v = piv;
       else if (i == k) v = rowk[j] * piv;
       else if (j == k) v = -colk[i] * piv;
       else v = G[i][j] - colk[i] * rowk[j] * piv;
-      G[i][j] = v;
+      if (i < kb && j < kb) G[i][j] = v;
     }
     __syncthreads();
   }
-  const int ntile = (n + kGjRows - 1) / kGjRows;
-  for (int t = blockIdx.x; t < ntile; t += gridDim.x) {
-    const int i0 = t * kGjRows;
-    // U: the row coefficients on the pivot rows; S: the rows' pivot-column entries
-    for (int e = threadIdx.x; e < kGjRows * kGjB; e += blockDim.x) {
-      const int ii = e / kGjB, l = e % kGjB, i = i0 + ii;
-      S[ii][l] = (i < n && l < kb) ? A[(size_t)i * n + k0 + l] : 0.0;
+  const int i0 = blockIdx.x * kGjRows;
+  // U: the row coefficients on the pivot rows; S: the rows' pivot-column entries
+  for (int e = threadIdx.x; e < kGjRows * kGjB; e += 256) {
+    const int ii = e / kGjB, l = e % kGjB, i = i0 + ii;
+    S[ii][l] = (i < n && l < kb) ? A[(size_t)i * n + k0 + l] : 0.0;
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < kGjRows * kGjB; e += 256) {
+    const int ii = e / kGjB, l = e % kGjB, i = i0 + ii;
+    double u = 0.0;
+    if (i < n && l < kb) {
+      if (i >= k0 && i < k0 + kb) u = G[i - k0][l];
+      else
+        for (int m = 0; m < kb; ++m) u += S[ii][m] * G[m][l];
     }
-    __syncthreads();
-    for (int e = threadIdx.x; e < kGjRows * kGjB; e += blockDim.x) {
-      const int ii = e / kGjB, l = e % kGjB, i = i0 + ii;
-      double u = 0.0;
-      if (i < n && l < kb) {
-        if (i >= k0 && i < k0 + kb) u = G[i - k0][l];
-        else
-          for (int m = 0; m < kb; ++m) u += S[ii][m] * G[m][l];
-      }
-      U[ii][l] = u;
-    }
-    __syncthreads();
-    for (int j = threadIdx.x; j < n; j += blockDim.x) {
-      const bool jin = j >= k0 && j < k0 + kb;
-      double a[kGjB];
+    U[ii][l] = u;
+  }
+  __syncthreads();
+  const int j = blockIdx.y * kGjCols + threadIdx.x % kGjCols;
+  const int half = threadIdx.x / kGjCols * (kGjRows / 2);
+  if (j >= n) return;
+  const bool jin = j >= k0 && j < k0 + kb;
+  double a[kGjB];
 #pragma unroll
-      for (int l = 0; l < kGjB; ++l) a[l] = (!jin && l < kb) ? A[(size_t)(k0 + l) * n + j] : 0.0;
-      for (int ii = 0; ii < kGjRows; ++ii) {
-        const int i = i0 + ii;
-        if (i >= n) break;
-        const bool iin = i >= k0 && i < k0 + kb;
-        double v;
-        if (jin) v = iin ? U[ii][j - k0] : -U[ii][j - k0];
-        else {
-          double acc = 0.0;
+  for (int l = 0; l < kGjB; ++l) a[l] = (!jin && l < kb) ? A[(size_t)(k0 + l) * n + j] : 0.0;
+  for (int ii = half; ii < half + kGjRows / 2; ++ii) {
+    const int i = i0 + ii;
+    if (i >= n) break;
+    const bool iin = i >= k0 && i < k0 + kb;
+    double v;
+    if (jin) v = iin ? U[ii][j - k0] : -U[ii][j - k0];
+    else {
+      double acc = 0.0;
 #pragma unroll
-          for (int l = 0; l < kGjB; ++l) acc += U[ii][l] * a[l];
-          v = iin ? acc : A[(size_t)i * n + j] - acc;
-        }
-        B[(size_t)i * n + j] = v;
-      }
+      for (int l = 0; l < kGjB; ++l) acc += U[ii][l] * a[l];
+      v = iin ? acc : A[(size_t)i * n + j] - acc;
     }
-    __syncthreads();
+    B[(size_t)i * n + j] = v;
   }
 }
 
@@ -198,6 +202,7 @@ __global__ void __launch_bounds__(256) k_gj_block(int n, int k0, const double *_
 // share of the level; above kPadMax the copy of the operator (32 bytes a
 // cell) could cost a grid its place in device memory.
 constexpr long long kPadMin = 4096, kPadMax = 1ll << 28;
+constexpr int kCoarseAuto = 1024;
 
 template <typename T>
 void EWork<T>::ensure(const std::vector<ELevel> &lv) {
@@ -276,7 +281,7 @@ static bool graph_loop_enabled() {
 // PBG_OMEGA one damped-Jacobi weight for every sweep (0 < omega < 1).
 EngineOpts::EngineOpts() {
   const char *c = getenv("PBG_COARSE_MAX");
-  if (c && atoi(c) > 0) coarse_max = atoi(c);
+  if (c && atoi(c) > 0) { coarse_max = atoi(c); coarse_auto = false; }
   const char *k = getenv("PBG_KC_MAX");
   if (k && atoi(k) > 0) kc_max = atoi(k);
   const char *o = getenv("PBG_OMEGA");
@@ -402,7 +407,12 @@ void Engine::build(const EMat<double> &A0_, cudaStream_t s, bool mixed) {
       l0.m64 = make_emat<double>(A0.nx, A0.ny, A0.nz, A0.c, A0.w, A0.s, A0.b, l0.d64.p);
     }
   }
-  while (L.back().ncell() > opt.coarse_max &&
+  // Unless the caller has chosen a size, the coarsest level is the first of at
+  // most kCoarseAuto cells: a level of 513 to 1024 cells is inverted rather
+  // than coarsened once more, whose visits (two of a level of 65 to 128 cells
+  // for each of its own) cost more than the larger inverse.
+  const long long dense = opt.coarse_auto ? std::max(opt.coarse_max, kCoarseAuto) : opt.coarse_max;
+  while (L.back().ncell() > dense &&
          (L.back().nx > 1 || L.back().ny > 1 || L.back().nz > 1)) {
     const ELevel &f = L.back();
     ELevel c;
@@ -473,7 +483,7 @@ void Engine::compute(cudaStream_t s) {
   k_dense_fill<<<grid_for(n), kThreads, 0, s>>>(L.back().m64, Dtmp.p); note_launch();
   k_dense_dmax<<<1, 1024, 0, s>>>(n, Dtmp.p, dsc.p + 7); note_launch();
   double *src = Dtmp.p, *dst = Ainv.p;
-  const int tiles = (n + kGjRows - 1) / kGjRows;
+  const dim3 tiles((n + kGjRows - 1) / kGjRows, (n + kGjCols - 1) / kGjCols);
   for (int k0 = 0; k0 < n; k0 += kGjB) {
     k_gj_block<<<tiles, 256, 0, s>>>(n, k0, src, dst, dsc.p + 7, 1e-10); note_launch();
     std::swap(src, dst);

@@ -91,6 +91,7 @@ struct EWork {
 struct EngineOpts {
   double omega_a = kOmegaA, omega_b = kOmegaB, over = kOverCorr;   // CycleW
   int coarse_max = 512;      // coarsest level size (dense direct solve)
+  bool coarse_auto = true;   // not chosen by the caller: up to 1024 where that ends the levels
   int kc_max = 99;           // levels 1..kc_max run a K-cycle, deeper levels one visit
   EngineOpts();
 };
