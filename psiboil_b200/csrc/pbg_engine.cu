@@ -619,23 +619,28 @@ int Engine::fcg(EWork<T> &w, const T *b, double tol, int maxit, RedPool &red, cu
                  (const T *)w.q0.p, fs, red.slot_part(0), red.slot_count(0));
     }
   };
-  if (!w.iter_graph) {
-    cudaGraph_t graph = nullptr;
+  // captured once: the loop where it is used, else the iteration alone
+  if (!w.iter_graph && !w.loop_graph) {
     const unsigned long long before = g_launch_count;
-    PBG_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-    try {
-      iteration(&fs->done);
-    } catch (...) {
-      cudaStreamEndCapture(s, &graph);  // leave the stream usable
-      if (graph) cudaGraphDestroy(graph);
-      throw;
-    }
-    PBG_CUDA(cudaStreamEndCapture(s, &graph));
-    w.iter_nodes = (size_t)(g_launch_count - before);
-    __atomic_sub_fetch(&g_launch_count, (unsigned long long)w.iter_nodes, __ATOMIC_RELAXED);
-    PBG_CUDA(cudaGraphInstantiate(&w.iter_graph, graph, 0));
-    cudaGraphDestroy(graph);
-    if (graph_loop_enabled()) {
+    auto counted = [&] {
+      w.iter_nodes = (size_t)(g_launch_count - before);
+      __atomic_sub_fetch(&g_launch_count, (unsigned long long)w.iter_nodes, __ATOMIC_RELAXED);
+    };
+    if (!graph_loop_enabled()) {
+      cudaGraph_t graph = nullptr;
+      PBG_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+      try {
+        iteration(&fs->done);
+      } catch (...) {
+        cudaStreamEndCapture(s, &graph);  // leave the stream usable
+        if (graph) cudaGraphDestroy(graph);
+        throw;
+      }
+      PBG_CUDA(cudaStreamEndCapture(s, &graph));
+      counted();
+      PBG_CUDA(cudaGraphInstantiate(&w.iter_graph, graph, 0));
+      cudaGraphDestroy(graph);
+    } else {
       // the same iteration as the body of a WHILE node: a gate kernel sets
       // its condition before the first pass, the last kernel of the body
       // after each pass
@@ -672,7 +677,7 @@ int Engine::fcg(EWork<T> &w, const T *b, double tol, int maxit, RedPool &red, cu
           throw;
         }
         PBG_CUDA(cudaStreamEndCapture(s, &body));
-        __atomic_sub_fetch(&g_launch_count, (unsigned long long)w.iter_nodes, __ATOMIC_RELAXED);
+        counted();
         PBG_CUDA(cudaGraphInstantiate(&w.loop_graph, lg, 0));
       } catch (...) {
         cudaGraphDestroy(lg);
