@@ -393,7 +393,7 @@ class BatchEngine : public BatchEngineBase {
     }
     sig_ = (unsigned long long)dtile | ((unsigned long long)dense_mask << 8) |
            ((unsigned long long)tail_mask << 24) | ((unsigned long long)dmax_ << 40);
-    const uint32_t tc = (uint32_t)shape_.tile_cells;
+    const uint32_t tmax = (uint32_t)shape_.tile_cells;
     for (int l = 0; l < kBMaxLev; ++l) {
       lbeg[l] = (int)tiles.size();
       for (int s = 0; s < S_; ++s) {
@@ -401,6 +401,11 @@ class BatchEngine : public BatchEngineBase {
         const Prob &P = get(slot_pid_[s]);
         if (P.nlev <= l) continue;
         const uint32_t n = (uint32_t)level_cells(P, l);
+        // 16 tiles of a level where its cells fill a block's threads: a
+        // small level in one or two tiles left the chip to a few blocks.
+        // The size depends on the level alone, and so do its sums.
+        const uint32_t NT = (uint32_t)shape_.threads;
+        const uint32_t tc = std::min(tmax, std::max(1u, n / (16 * NT)) * NT);
         tbeg[(size_t)l * S_ + s] = (int)tiles.size();
         int k = 0;
         for (uint32_t p0 = 0; p0 < n; p0 += tc, ++k) tiles.push_back({s, p0, std::min(tc, n - p0)});
@@ -492,7 +497,10 @@ class BatchEngine : public BatchEngineBase {
     if (kBPad<T> && l == 0) { kb_resid0<T><<<G, NT, 0, stream>>>(C); ++n; }
     kb_restrict<T><<<GH, NT, 0, stream>>>(C, l, kc); ++n;
     if (dense_mask & (1u << (l + 1))) { kb_dense<T><<<slot_grid(), NT, 0, stream>>>(C, l + 1); ++n; }
-    if (tail_mask & (1u << (l + 1))) { kb_tail<T><<<slot_grid(), NT, 0, stream>>>(C, l + 1); ++n; }
+    if (tail_mask & (1u << (l + 1))) {
+      PBG_CUDA(cudaFuncSetAttribute(kb_tail<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTailShared<T>));
+      kb_tail<T><<<slot_grid(), NT, kTailShared<T>, stream>>>(C, l + 1); ++n;
+    }
     if (l + 1 < dtile) seq_kcycle(C, l + 1, n);
     kb_prolong_jac<T><<<G, NT, 0, stream>>>(C, l, kc); ++n;
     kb_jac<T><<<G, NT, 0, stream>>>(C, l, kc); ++n;

@@ -907,7 +907,8 @@ __device__ __forceinline__ void t_allreduce(double (&v)[K], double (*sm)[kBThrea
 // preconditioner application, 1 / 3 finish it. Leaves z1 (and z2) on level
 // top and its scalars in S.ks[top] as a1 = c1, a2 = c2, beta = 0.
 template <typename T>
-__device__ void t_kcycle(const BProb<T> &P, BState &S, int top, int kc_max, CycleW<T> om) {
+__device__ void t_kcycle(const BProb<T> &P, const BLev<T> *L, const double *Ainv, BState &S, int top, int kc_max,
+                         CycleW<T> om) {
   __shared__ double sm[3][kBThreadsMax / 32];
   __shared__ double bc[4];
   const int last = P.nlev - 1;
@@ -918,7 +919,7 @@ __device__ void t_kcycle(const BProb<T> &P, BState &S, int top, int kc_max, Cycl
   int l = top;
   step[l] = 0;
   for (int guard = 0; guard < (1 << 24); ++guard) {
-    const BLev<T> &V = P.L[l];
+    const BLev<T> &V = L[l];
     const uint32_t n = V.A.g.n;
     const int s = step[l];
     const bool second = s >= 2;
@@ -927,7 +928,7 @@ __device__ void t_kcycle(const BProb<T> &P, BState &S, int top, int kc_max, Cycl
       const T a1 = second ? (T)ks[l].a1 : T(0);
       TCELL_LOOP(p, n) cell_jac2(V, V.b, p, a1, second, om);
       __syncthreads();
-      const BLev<T> &H = P.L[l + 1];
+      const BLev<T> &H = L[l + 1];
       for (uint32_t base = 0; base < H.A.g.n * 8u; base += blockDim.x) {
         const uint32_t u = base + threadIdx.x;
         const bool valid = u < H.A.g.n * 8u;
@@ -938,7 +939,7 @@ __device__ void t_kcycle(const BProb<T> &P, BState &S, int top, int kc_max, Cycl
       __syncthreads();
       step[l] = s + 1;
       if (l + 1 == last) {
-        for (int row = wid; row < P.ncoarse; row += nw) warp_dense_row(P.Ainv, P.ncoarse, H.b, H.x, row);
+        for (int row = wid; row < P.ncoarse; row += nw) warp_dense_row(Ainv, P.ncoarse, H.b, H.x, row);
         __syncthreads();
       } else {
         l = l + 1;
@@ -947,7 +948,7 @@ __device__ void t_kcycle(const BProb<T> &P, BState &S, int top, int kc_max, Cycl
       continue;
     }
     {
-      const BLev<T> &H = P.L[l + 1];
+      const BLev<T> &H = L[l + 1];
       const bool hdense = l + 1 == last;
       const bool two = !hdense && (l + 1) <= kc_max;
       const T *eH = hdense ? H.x : H.z1;
@@ -988,14 +989,62 @@ __device__ void t_kcycle(const BProb<T> &P, BState &S, int top, int kc_max, Cycl
   __syncthreads();
 }
 
+// Shared memory of a tail: the levels' operators and vectors and the dense
+// inverse, where they fit kTailShared (1024 cells and the levels below them
+// do); a tail of more cells works in global memory. A phase of a few hundred
+// cells is one chain of loads and a barrier: from shared memory it takes
+// about 0.5 us where from L2 it took 3.
+template <typename T> constexpr size_t kTailShared = (sizeof(T) == 4 ? 96 : 160) * 1024;
+constexpr int kTailArrays = 12;   // w s b c dinv, b q1 r1 xb xa z1 z2
+
 // K-cycles of level l for every slot whose tail starts there.
 template <typename T>
 __global__ void __launch_bounds__(kBThreadsMax) kb_tail(BCtx<T> C, int l) {
+  extern __shared__ __align__(16) unsigned char tail_sm[];
+  __shared__ BLev<T> lev[kBMaxLev];
   for (int slot = blockIdx.x; slot < C.S; slot += gridDim.x) {
     BState &S = C.st[slot];
     const BProb<T> &P = C.prob[slot];
     if (!b_running(S) || P.tail != l) continue;
-    t_kcycle(P, S, l, C.kc_max, C.om);
+    const int last = P.nlev - 1;
+    size_t need = (size_t)P.ncoarse * P.ncoarse * sizeof(double);
+    for (int q = l; q < last; ++q) need += (size_t)P.L[q].A.g.n * kTailArrays * sizeof(T);
+    need += 2 * (size_t)P.ncoarse * sizeof(T);
+    if (need > kTailShared<T>) {
+      t_kcycle(P, P.L, P.Ainv, S, l, C.kc_max, C.om);
+      continue;
+    }
+    double *inv = reinterpret_cast<double *>(tail_sm);
+    T *at = reinterpret_cast<T *>(inv + P.ncoarse * P.ncoarse);
+    for (int e = threadIdx.x; e < P.ncoarse * P.ncoarse; e += blockDim.x) inv[e] = P.Ainv[e];
+    for (int q = l; q < last; ++q) {
+      const BLev<T> &V = P.L[q];
+      const uint32_t n = V.A.g.n;
+      const T *src[6] = {V.A.w, V.A.s, V.A.b, V.A.c, V.A.dinv, V.b};
+      for (int f = 0; f < (q == l ? 6 : 5); ++f)
+        for (uint32_t e = threadIdx.x; e < n; e += blockDim.x) at[f * n + e] = src[f][e];
+      if (threadIdx.x == 0) {
+        BLev<T> W = V;
+        W.A.w = at; W.A.s = at + n; W.A.b = at + 2 * n; W.A.c = at + 3 * n; W.A.dinv = at + 4 * n;
+        W.b = at + 5 * n; W.q1 = at + 6 * n; W.r1 = at + 7 * n; W.xb = at + 8 * n; W.xa = at + 9 * n;
+        W.z1 = at + 10 * n; W.z2 = at + 11 * n;
+        lev[q] = W;
+      }
+      at += kTailArrays * n;
+    }
+    if (threadIdx.x == 0) {
+      lev[last] = P.L[last];
+      lev[last].b = at;
+      lev[last].x = at + P.ncoarse;
+    }
+    __syncthreads();
+    t_kcycle(P, lev, inv, S, l, C.kc_max, C.om);   // ends with a barrier
+    const uint32_t n = P.L[l].A.g.n;
+    for (uint32_t e = threadIdx.x; e < n; e += blockDim.x) {
+      P.L[l].z1[e] = lev[l].z1[e];
+      P.L[l].z2[e] = lev[l].z2[e];
+    }
+    __syncthreads();   // the next slot reuses the shared memory
   }
 }
 
