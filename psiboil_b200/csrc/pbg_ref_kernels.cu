@@ -261,9 +261,30 @@ __global__ void __launch_bounds__(kThreads, 3) k_cg_pq(MatView<double> A, const 
   }
 }
 
-// Seq = false: tree-order sums only (the split path), without the
-// exact-order reduction's code and shared memory
-template <bool Seq>
+// The end of a CG step from its two sums: residual, tests, next rho
+// (cg.cpp:112-175); one thread.
+__device__ __forceinline__ void cg_step_end(KrylovState *st, double *hist, int it, double rr, double rz, int ic) {
+  double res = res_of(rr, st);
+  st->res = res;
+  if (hist && it < st->hist_cap) hist[it] = res;
+  const bool minok = it >= st->mini - 1;
+  if ((res < st->res_tol && minok) || (res < st->res0 * st->res_rat && minok)) {
+    st->done = 1; st->converged = 1; st->status = ST_CONVERGED; st->iterations = it + 1;
+  } else if (stale_step_dev(st, res)) {
+    st->done = 1; st->status = ST_STALE; st->iterations = it + 1;
+  } else if (!(res == res)) {
+    st->done = 1; st->status = ST_NAN; st->iterations = it + 1;
+  } else {
+    if (!ic) {  // with an IC preconditioner k_cg_rho forms rho after the solve
+      st->rho_old = st->rho;
+      st->rho = rz;
+    }
+    st->iter = it + 1;
+    st->iterations = it + 1;
+    if (it + 1 >= st->maxit) { st->done = 1; st->status = ST_MAXITER; }
+  }
+}
+
 __global__ void __launch_bounds__(kThreads, 3) k_cg_xr(long long N, const double *__restrict__ mc, double *__restrict__ x,
                         double *__restrict__ r, const double *pA, const double *pB,
                         const double *__restrict__ qv, KrylovState *st, double *hist,
@@ -283,27 +304,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_cg_xr(long long N, const double
     v[1] += __dmul_rn(rv, __dmul_rn(rv, mc[p]));
   }
   double o[2];
-  if (grid_reduce<2>(v, part, count, o, Seq ? st->seq : nullptr, N)) {
-    double res = res_of(o[0], st);
-    st->res = res;
-    if (hist && it < st->hist_cap) hist[it] = res;
-    const bool minok = it >= st->mini - 1;
-    if ((res < st->res_tol && minok) || (res < st->res0 * st->res_rat && minok)) {
-      st->done = 1; st->converged = 1; st->status = ST_CONVERGED; st->iterations = it + 1;
-    } else if (stale_step_dev(st, res)) {
-      st->done = 1; st->status = ST_STALE; st->iterations = it + 1;
-    } else if (!(res == res)) {
-      st->done = 1; st->status = ST_NAN; st->iterations = it + 1;
-    } else {
-      if (!ic) {  // with an IC preconditioner k_cg_rho forms rho after the solve
-        st->rho_old = st->rho;
-        st->rho = o[1];
-      }
-      st->iter = it + 1;
-      st->iterations = it + 1;
-      if (it + 1 >= st->maxit) { st->done = 1; st->status = ST_MAXITER; }
-    }
-  }
+  if (grid_reduce<2>(v, part, count, o, st->seq, N)) cg_step_end(st, hist, it, o[0], o[1], ic);
 }
 
 // ---------------------------------------------------------------------------
@@ -384,6 +385,38 @@ __global__ void __launch_bounds__(kThreads, 4) k_cg_q(MatView<double> A, Geo G, 
     st->pq = o[0];
     st->alfa = __ddiv_rn(st->rho, o[0]);
   }
+}
+
+// x += alfa p, r -= alfa q and the two sums of k_cg_xr, two cells a thread
+// (nz, and so N, even): five 16-byte loads in flight where there were five of
+// 8 bytes.
+__global__ void __launch_bounds__(kThreads, 4) k_cg_xr2(long long N, const double *__restrict__ mc, double *__restrict__ x,
+                         double *__restrict__ r, const double *__restrict__ p, const double *__restrict__ qv,
+                         KrylovState *st, double *hist, double *part, unsigned *count) {
+  if (st->done) return;
+  const int it = st->iter;
+  const double alfa = st->alfa;
+  const KnownDiv dV(st->dV);
+  double v[2] = {0.0, 0.0};
+  const long long NP = N / 2;
+  for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < NP;
+       g += (long long)gridDim.x * blockDim.x) {
+    double2 xv = reinterpret_cast<const double2 *>(x)[g], rv = reinterpret_cast<const double2 *>(r)[g];
+    const double2 pv = reinterpret_cast<const double2 *>(p)[g], q2 = reinterpret_cast<const double2 *>(qv)[g];
+    const double2 mv = reinterpret_cast<const double2 *>(mc)[g];
+    xv.x = __dadd_rn(xv.x, __dmul_rn(alfa, pv.x));
+    xv.y = __dadd_rn(xv.y, __dmul_rn(alfa, pv.y));
+    rv.x = __dsub_rn(rv.x, __dmul_rn(alfa, q2.x));
+    rv.y = __dsub_rn(rv.y, __dmul_rn(alfa, q2.y));
+    reinterpret_cast<double2 *>(x)[g] = xv;
+    reinterpret_cast<double2 *>(r)[g] = rv;
+    v[0] += voldiv(rv.x, rv.x, dV);
+    v[0] += voldiv(rv.y, rv.y, dV);
+    v[1] += __dmul_rn(rv.x, __dmul_rn(rv.x, mv.x));
+    v[1] += __dmul_rn(rv.y, __dmul_rn(rv.y, mv.y));
+  }
+  double o[2];
+  if (grid_reduce<2>(v, part, count, o)) cg_step_end(st, hist, it, o[0], o[1], 0);
 }
 
 // ---------------------------------------------------------------------------
@@ -480,6 +513,7 @@ __global__ void k_ic3_bwd(MatView<double> A, Ic3Factor M, int h, double *z, cons
 }
 
 // rho = r.z (Scalar::dot, scalar.h:296-298) for the next CG step
+template <bool Seq>
 __global__ void k_cg_rho(long long N, const double *__restrict__ r, const double *__restrict__ z,
                          KrylovState *st, double *part, unsigned *count) {
   if (st->done) return;
@@ -488,7 +522,7 @@ __global__ void k_cg_rho(long long N, const double *__restrict__ r, const double
        p += (long long)gridDim.x * blockDim.x)
     v[0] += __dmul_rn(r[p], z[p]);
   double o[1];
-  if (grid_reduce<1>(v, part, count, o, st->seq, N)) {
+  if (grid_reduce<1>(v, part, count, o, Seq ? st->seq : nullptr, N)) {
     st->rho_old = st->rho;
     st->rho = o[0];
   }
@@ -507,6 +541,7 @@ __global__ void k_cg_rho(long long N, const double *__restrict__ r, const double
 // pending_x, which k_bi_xr applies and clears. With an incomplete Cholesky
 // preconditioner (diag == 0) the IC sweeps form p^ and s^ instead.
 // ---------------------------------------------------------------------------
+template <bool Seq>
 __global__ void k_bi_init(MatView<double> A, const double *__restrict__ x, const double *__restrict__ b,
                           double *__restrict__ r, double *__restrict__ rt, KrylovState *st,
                           double *part, unsigned *count) {
@@ -522,7 +557,7 @@ __global__ void k_bi_init(MatView<double> A, const double *__restrict__ x, const
     v[0] += voldiv(rv, rv, dV);
   }
   double o[1];
-  if (grid_reduce<1>(v, part, count, o, st->seq, N)) {
+  if (grid_reduce<1>(v, part, count, o, Seq ? st->seq : nullptr, N)) {
     double res = res_of(o[0], st);
     st->res0 = res;
     st->res = res;
@@ -541,6 +576,7 @@ __global__ void k_bi_init(MatView<double> A, const double *__restrict__ x, const
   }
 }
 
+template <bool Seq>
 __global__ void k_bi_rho(long long N, const double *__restrict__ rt, const double *__restrict__ r,
                          KrylovState *st, double *part, unsigned *count) {
   if (st->done) return;
@@ -549,7 +585,7 @@ __global__ void k_bi_rho(long long N, const double *__restrict__ rt, const doubl
        p += (long long)gridDim.x * blockDim.x)
     v[0] += __dmul_rn(rt[p], r[p]);
   double o[1];
-  if (grid_reduce<1>(v, part, count, o, st->seq, N)) {
+  if (grid_reduce<1>(v, part, count, o, Seq ? st->seq : nullptr, N)) {
     const int it = st->iter;
     st->rho = o[0];
     if (__dsqrt_rn(fabs(o[0])) < st->res_tol) {
@@ -580,6 +616,7 @@ __global__ void k_bi_p(long long N, const double *__restrict__ c, const double *
 }
 
 // y = A x and up to two dots with y: mode 0 -> rt.y (alfa), mode 1 -> y.s, y.y (omega)
+template <bool Seq>
 __global__ void k_bi_spmv(MatView<double> A, const double *__restrict__ x, double *__restrict__ y,
                           const double *__restrict__ o1, int mode, KrylovState *st,
                           double *part, unsigned *count) {
@@ -595,12 +632,13 @@ __global__ void k_bi_spmv(MatView<double> A, const double *__restrict__ x, doubl
     else { v[0] += __dmul_rn(yv, o1[p]); v[1] += __dmul_rn(yv, yv); }
   }
   double o[2];
-  if (grid_reduce<2>(v, part, count, o, st->seq, N)) {
+  if (grid_reduce<2>(v, part, count, o, Seq ? st->seq : nullptr, N)) {
     if (mode == 0) st->alfa = __ddiv_rn(st->rho, o[0]);
     else { st->aux0 = o[0]; st->aux1 = o[1]; st->omega = __ddiv_rn(o[0], o[1]); }
   }
 }
 
+template <bool Seq>
 __global__ void k_bi_s(long long N, const double *__restrict__ c, const double *__restrict__ r,
                        const double *__restrict__ v, double *__restrict__ s, double *__restrict__ sh,
                        KrylovState *st, double *part, unsigned *count, int diag) {
@@ -615,7 +653,7 @@ __global__ void k_bi_s(long long N, const double *__restrict__ c, const double *
     a[0] += __dmul_rn(sv, sv);
   }
   double o[1];
-  if (grid_reduce<1>(a, part, count, o, st->seq, N)) {
+  if (grid_reduce<1>(a, part, count, o, Seq ? st->seq : nullptr, N)) {
     if (__dsqrt_rn(o[0]) < st->res_tol) {
       st->pending_x = 1;  // x += alfa p^, then stop (bicgs.cpp:146-150)
       st->done = 1; st->status = ST_BREAKDOWN; st->iterations = st->iter + 1;
@@ -623,6 +661,7 @@ __global__ void k_bi_s(long long N, const double *__restrict__ c, const double *
   }
 }
 
+template <bool Seq>
 __global__ void k_bi_xr(long long N, double *__restrict__ x, double *__restrict__ r,
                         const double *__restrict__ ph, const double *__restrict__ sh,
                         const double *__restrict__ s, const double *__restrict__ t,
@@ -642,7 +681,7 @@ __global__ void k_bi_xr(long long N, double *__restrict__ x, double *__restrict_
     v[0] += voldiv(rv, rv, dV);
   }
   double o[1];
-  if (grid_reduce<1>(v, part, count, o, st->seq, N)) {
+  if (grid_reduce<1>(v, part, count, o, Seq ? st->seq : nullptr, N)) {
     if (pend) { st->pending_x = 0; return; }
     const int it = st->iter;
     double res = res_of(o[0], st);
@@ -679,6 +718,7 @@ __global__ void k_bi_xr(long long N, double *__restrict__ x, double *__restrict_
 // incomplete Cholesky preconditioner (diag == 0) the IC sweeps form p^
 // and u^ instead.
 // ---------------------------------------------------------------------------
+template <bool Seq>
 __global__ void k_cgs_rho(long long N, const double *__restrict__ rt, const double *__restrict__ r,
                           KrylovState *st, double *part, unsigned *count) {
   if (st->done) return;
@@ -687,7 +727,7 @@ __global__ void k_cgs_rho(long long N, const double *__restrict__ rt, const doub
        p += (long long)gridDim.x * blockDim.x)
     v[0] += __dmul_rn(rt[p], r[p]);
   double o[1];
-  if (grid_reduce<1>(v, part, count, o, st->seq, N)) {
+  if (grid_reduce<1>(v, part, count, o, Seq ? st->seq : nullptr, N)) {
     const int it = st->iter;
     st->rho = o[0];
     if (__dsqrt_rn(fabs(o[0])) < st->res_tol) {
@@ -736,6 +776,7 @@ __global__ void k_cgs_qs(long long N, const double *__restrict__ c, const double
   }
 }
 
+template <bool Seq>
 __global__ void k_cgs_xr(MatView<double> A, double *__restrict__ x, double *__restrict__ r,
                          const double *__restrict__ sh, KrylovState *st, double *hist, double *part,
                          unsigned *count) {
@@ -754,7 +795,7 @@ __global__ void k_cgs_xr(MatView<double> A, double *__restrict__ x, double *__re
     v[0] += voldiv(rv, rv, dV);
   }
   double o[1];
-  if (grid_reduce<1>(v, part, count, o, st->seq, N)) {
+  if (grid_reduce<1>(v, part, count, o, Seq ? st->seq : nullptr, N)) {
     const int it = st->iter;
     double res = res_of(o[0], st);
     st->res = res;
@@ -1013,6 +1054,7 @@ __device__ __forceinline__ double it_res(double d, const KrylovState *st, int gs
   return gs ? res_of(d, st) : __dsqrt_rn(d);
 }
 
+template <bool Seq>
 __global__ void k_it_init(MatView<double> A, const double *__restrict__ x,
                           const double *__restrict__ b, double *__restrict__ r, KrylovState *st,
                           double *part, unsigned *count, int gs) {
@@ -1027,7 +1069,7 @@ __global__ void k_it_init(MatView<double> A, const double *__restrict__ x,
     v[0] += gs ? voldiv(rv, rv, dV) : __dmul_rn(rv, rv);
   }
   double o[1];
-  if (grid_reduce<1>(v, part, count, o, st->seq, N)) {
+  if (grid_reduce<1>(v, part, count, o, Seq ? st->seq : nullptr, N)) {
     const double res = it_res(o[0], st, gs);
     st->res0 = res;
     st->res = res;
@@ -1097,6 +1139,7 @@ __global__ void k_gs_plane(MatView<double> A, const double *__restrict__ ci,
 
 // r = b - A x after a sweep, the residual measure and the exits
 // (jacobi.cpp:47-61, gaussseidel.cpp:63-105)
+template <bool Seq>
 __global__ void k_it_resid(MatView<double> A, const double *__restrict__ x,
                            const double *__restrict__ b, double *__restrict__ r, KrylovState *st,
                            double *hist, double *part, unsigned *count, int gs) {
@@ -1113,7 +1156,7 @@ __global__ void k_it_resid(MatView<double> A, const double *__restrict__ x,
     v[0] += gs ? voldiv(rv, rv, dV) : __dmul_rn(rv, rv);
   }
   double o[1];
-  if (grid_reduce<1>(v, part, count, o, st->seq, N)) {
+  if (grid_reduce<1>(v, part, count, o, Seq ? st->seq : nullptr, N)) {
     const double res = it_res(o[0], st, gs);
     st->res = res;
     if (hist && it < st->hist_cap) hist[it] = res;
@@ -1227,7 +1270,8 @@ void enqueue_ref_setup(const MatView<double> &A, double *x, const double *b, con
                        int solver, RefKrylovWork &w, const RedPool &red, KrylovState *st,
                        cudaStream_t s) {
   const long long N = A.ncell();
-  const int g = pr.seq ? grid_exact(N) : grid_for(N);
+  const bool exact = pr.seq != nullptr;   // kernels without the exact-order code keep their occupancy
+  const int g = exact ? grid_exact(N) : grid_for(N);
   w.ensure((size_t)N, solver);
   k_krylov_setup<<<1, 1, 0, s>>>(st, pr, N); note_launch();
   if (solver >= 3) {  // Jacobi, Gauss-Seidel: ci as stored with the matrix, else 1/c
@@ -1243,7 +1287,7 @@ void enqueue_ref_setup(const MatView<double> &A, double *x, const double *b, con
       k_gs_pack<<<grid_for((long long)sg.all_rows() * kSweepCols), kThreads, 0, s>>>(sg, A, w.ci, b, x,
                                                                                  w.march(sg, kGsPlanes)); note_launch();
     }
-    k_it_init<<<g, kThreads, 0, s>>>(A, x, b, w.r.p, st, red.slot_part(0), red.slot_count(0),
+    (exact ? k_it_init<true> : k_it_init<false>)<<<g, kThreads, 0, s>>>(A, x, b, w.r.p, st, red.slot_part(0), red.slot_count(0),
                                      solver == 4 ? 1 : 0); note_launch();
     PBG_CUDA(cudaGetLastError());
     return;
@@ -1266,7 +1310,7 @@ void enqueue_ref_setup(const MatView<double> &A, double *x, const double *b, con
   if (solver == 0)
     k_cg_init<<<g, kThreads, 0, s>>>(A, x, b, w.r.p, st, red.slot_part(0), red.slot_count(0), w.mcd.p);
   else
-    k_bi_init<<<g, kThreads, 0, s>>>(A, x, b, w.r.p, w.rt.p, st, red.slot_part(0), red.slot_count(0));
+    (exact ? k_bi_init<true> : k_bi_init<false>)<<<g, kThreads, 0, s>>>(A, x, b, w.r.p, w.rt.p, st, red.slot_part(0), red.slot_count(0));
   note_launch();
   PBG_CUDA(cudaGetLastError());
 }
@@ -1319,7 +1363,7 @@ void enqueue_ref_iters(const MatView<double> &A, double *x, int solver, int coun
       } else {
         k_jacobi_x<<<grid_for(N), kThreads, 0, s>>>(N, A.c, w.ci, w.r.p, x, st); note_launch();
       }
-      k_it_resid<<<g, kThreads, 0, s>>>(A, x, w.rhs, w.r.p, st, hist, P0, C0, gs); note_launch();
+      (exact ? k_it_resid<true> : k_it_resid<false>)<<<g, kThreads, 0, s>>>(A, x, w.rhs, w.r.p, st, hist, P0, C0, gs); note_launch();
     }
     PBG_CUDA(cudaGetLastError());
     return;
@@ -1328,34 +1372,38 @@ void enqueue_ref_iters(const MatView<double> &A, double *x, int solver, int coun
     if (solver == 0 && prec > 0) {
       // z = M^-1 r (forward and backward sweeps), rho = r.z, then the CG step
       ic_apply(A, prec, w, w.r.p, w.z.p, st, s);
-      k_cg_rho<<<g, kThreads, 0, s>>>(N, w.r.p, w.z.p, st, P0, C0); note_launch();
+      (exact ? k_cg_rho<true> : k_cg_rho<false>)<<<g, kThreads, 0, s>>>(N, w.r.p, w.z.p, st, P0, C0); note_launch();
       k_cg_pq<<<g, kThreads, 0, s>>>(A, w.r.p, w.pA.p, w.pB.p, w.q.p, st, P0, C0, w.z.p, w.mcd.p); note_launch();
-      k_cg_xr<true><<<g, kThreads, 0, s>>>(N, w.mcd.p, x, w.r.p, w.pA.p, w.pB.p, w.q.p, st, hist, P1, C1, 1); note_launch();
+      k_cg_xr<<<g, kThreads, 0, s>>>(N, w.mcd.p, x, w.r.p, w.pA.p, w.pB.p, w.q.p, st, hist, P1, C1, 1); note_launch();
     } else if (solver == 0 && !exact && A.nz % 2 == 0 && !A.per) {
       const int gq = grid_for(N / 2);
       k_cg_p<<<gq, kThreads, 0, s>>>(N, w.r.p, w.mcd.p, w.pA.p, st); note_launch();
       k_cg_q<<<gq, kThreads, 0, s>>>(A, Geo(A.nx, A.ny, A.nz), w.pA.p, w.q.p, st, P0, C0); note_launch();
-      k_cg_xr<false><<<g, kThreads, 0, s>>>(N, w.mcd.p, x, w.r.p, w.pA.p, w.pA.p, w.q.p, st, hist, P1, C1, 0); note_launch();
+      if (reinterpret_cast<uintptr_t>(x) % 16 == 0)   // x is the caller's
+        k_cg_xr2<<<gq, kThreads, 0, s>>>(N, w.mcd.p, x, w.r.p, w.pA.p, w.q.p, st, hist, P1, C1);
+      else
+        k_cg_xr<<<g, kThreads, 0, s>>>(N, w.mcd.p, x, w.r.p, w.pA.p, w.pA.p, w.q.p, st, hist, P1, C1, 0);
+      note_launch();
     } else if (solver == 0) {
       k_cg_pq<<<g, kThreads, 0, s>>>(A, w.r.p, w.pA.p, w.pB.p, w.q.p, st, P0, C0, nullptr, w.mcd.p); note_launch();
-      k_cg_xr<true><<<g, kThreads, 0, s>>>(N, w.mcd.p, x, w.r.p, w.pA.p, w.pB.p, w.q.p, st, hist, P1, C1, 0); note_launch();
+      k_cg_xr<<<g, kThreads, 0, s>>>(N, w.mcd.p, x, w.r.p, w.pA.p, w.pB.p, w.q.p, st, hist, P1, C1, 0); note_launch();
     } else if (solver == 1) {
-      k_bi_rho<<<g, kThreads, 0, s>>>(N, w.rt.p, w.r.p, st, P0, C0); note_launch();
+      (exact ? k_bi_rho<true> : k_bi_rho<false>)<<<g, kThreads, 0, s>>>(N, w.rt.p, w.r.p, st, P0, C0); note_launch();
       k_bi_p<<<g, kThreads, 0, s>>>(N, w.mcd.p, w.r.p, w.pA.p, w.v.p, w.ph.p, st, diag); note_launch();
       if (!diag) ic_apply(A, prec, w, w.pA.p, w.ph.p, st, s);
-      k_bi_spmv<<<g, kThreads, 0, s>>>(A, w.ph.p, w.v.p, w.rt.p, 0, st, P1, C1); note_launch();
-      k_bi_s<<<g, kThreads, 0, s>>>(N, w.mcd.p, w.r.p, w.v.p, w.s.p, w.sh.p, st, P0, C0, diag); note_launch();
+      (exact ? k_bi_spmv<true> : k_bi_spmv<false>)<<<g, kThreads, 0, s>>>(A, w.ph.p, w.v.p, w.rt.p, 0, st, P1, C1); note_launch();
+      (exact ? k_bi_s<true> : k_bi_s<false>)<<<g, kThreads, 0, s>>>(N, w.mcd.p, w.r.p, w.v.p, w.s.p, w.sh.p, st, P0, C0, diag); note_launch();
       if (!diag) ic_apply(A, prec, w, w.s.p, w.sh.p, st, s);
-      k_bi_spmv<<<g, kThreads, 0, s>>>(A, w.sh.p, w.t.p, w.s.p, 1, st, P1, C1); note_launch();
-      k_bi_xr<<<g, kThreads, 0, s>>>(N, x, w.r.p, w.ph.p, w.sh.p, w.s.p, w.t.p, st, hist, P0, C0); note_launch();
+      (exact ? k_bi_spmv<true> : k_bi_spmv<false>)<<<g, kThreads, 0, s>>>(A, w.sh.p, w.t.p, w.s.p, 1, st, P1, C1); note_launch();
+      (exact ? k_bi_xr<true> : k_bi_xr<false>)<<<g, kThreads, 0, s>>>(N, x, w.r.p, w.ph.p, w.sh.p, w.s.p, w.t.p, st, hist, P0, C0); note_launch();
     } else {
-      k_cgs_rho<<<g, kThreads, 0, s>>>(N, w.rt.p, w.r.p, st, P0, C0); note_launch();
+      (exact ? k_cgs_rho<true> : k_cgs_rho<false>)<<<g, kThreads, 0, s>>>(N, w.rt.p, w.r.p, st, P0, C0); note_launch();
       k_cgs_up<<<g, kThreads, 0, s>>>(N, w.mcd.p, w.r.p, w.q.p, w.u.p, w.pA.p, w.ph.p, st, diag); note_launch();
       if (!diag) ic_apply(A, prec, w, w.pA.p, w.ph.p, st, s);
-      k_bi_spmv<<<g, kThreads, 0, s>>>(A, w.ph.p, w.v.p, w.rt.p, 0, st, P1, C1); note_launch();
+      (exact ? k_bi_spmv<true> : k_bi_spmv<false>)<<<g, kThreads, 0, s>>>(A, w.ph.p, w.v.p, w.rt.p, 0, st, P1, C1); note_launch();
       k_cgs_qs<<<g, kThreads, 0, s>>>(N, w.mcd.p, w.u.p, w.v.p, w.q.p, w.s.p, w.sh.p, st, diag); note_launch();
       if (!diag) ic_apply(A, prec, w, w.s.p, w.sh.p, st, s);
-      k_cgs_xr<<<g, kThreads, 0, s>>>(A, x, w.r.p, w.sh.p, st, hist, P0, C0); note_launch();
+      (exact ? k_cgs_xr<true> : k_cgs_xr<false>)<<<g, kThreads, 0, s>>>(A, x, w.r.p, w.sh.p, st, hist, P0, C0); note_launch();
     }
   }
   PBG_CUDA(cudaGetLastError());
