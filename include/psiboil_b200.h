@@ -123,9 +123,11 @@ typedef struct {
    * results; computed in parallel, see pbg_seq_sum, about 15x the time of
    * a tree sum); 0 = deterministic tree sums */
   int exact_sums;
-  /* engine: cells of the dense coarsest level (0: 512). Larger (4096) saves
-   * launches in repeated solves with one matrix and costs a longer set-up
-   * after every matrix change (a dense inverse, O(cells^3)). */
+  /* engine: cells of the dense coarsest level at most, until a later call
+   * names another size; 0: as an earlier call on this session chose, else the
+   * first level of at most 1024. Larger (4096) saves launches in repeated
+   * solves with one matrix and costs a longer set-up after every matrix change
+   * (a dense inverse, O(cells^3)). */
   int coarse_max;
   /* Krylov preconditioner (CG, BiCGS, CGS), the reference's Prec codes
    * (preconditioner.h:15-29): 0 diagonal (Prec::di, default), 1 IC0, 2 IC2,

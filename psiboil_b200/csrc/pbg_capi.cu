@@ -881,9 +881,10 @@ void ensure_refac(pbg_session *s) {
 
 void ensure_engine(pbg_session *s, bool mixed, int coarse_max) {
   if (!s->eng) s->eng = std::make_unique<Engine>();
-  if (coarse_max > 0 && coarse_max != s->eng->opt.coarse_max) {
-    s->eng->opt.coarse_max = coarse_max;  // a different hierarchy: build anew
-    s->eng->opt.coarse_auto = false;
+  EngineOpts &o = s->eng->opt;
+  if (coarse_max > 0 && (o.coarse_auto || coarse_max != o.coarse_max)) {
+    o.coarse_max = coarse_max;  // a different hierarchy: build anew
+    o.coarse_auto = false;
     s->eng->L.clear();
     s->eng_dirty = true;
   }

@@ -1,0 +1,38 @@
+"""The engine's hierarchy as the caller sees it: which levels there are, what
+an explicit coarse_max does, and that a solve depends on its matrix and its
+options alone, not on the calls before it on the same session."""
+import numpy as np
+import pytest
+
+from test_gpu_sweeps import problem
+
+pytestmark = pytest.mark.gpu
+
+
+def solve(engine, E, P, **kw):
+    x = np.zeros(P.N)
+    assert E.solve(x, P.b.copy(), tol=1e-9, **kw)
+    assert np.linalg.norm(x) > 0.0
+    return x
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("before", [None, 0, 4096])
+def test_explicit_coarse_max_is_a_limit(engine, precision, before):
+    """20x16x18 coarsens to 720 and 100 cells: asked for at most 512 the
+    hierarchy goes down to 100, whatever an earlier call on the session asked
+    for (None: no earlier call; 0: the engine's choice)."""
+    P = problem((20, 16, 18), False)
+    with engine.Session(*P.dims, P.h) as s:
+        s.upload_matrix(P.A)
+        E = engine.Engine(s)
+        ref = solve(engine, E, P, precision=precision, coarse_max=511)
+        assert s.levels(1) == [(20, 16, 18), (10, 8, 9), (5, 4, 5)]
+    with engine.Session(*P.dims, P.h) as s:
+        s.upload_matrix(P.A)
+        E = engine.Engine(s)
+        if before is not None:
+            solve(engine, E, P, precision=precision, coarse_max=before)
+        x = solve(engine, E, P, precision=precision, coarse_max=512)
+        assert E.last.levels == 3
+        assert np.array_equal(x, ref)
