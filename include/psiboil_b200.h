@@ -338,7 +338,8 @@ int pbg_seq_sum(pbg_session *s, const double *a, const double *b, long long n, i
 
 /* Multigrid hierarchy sizes: count and per-level dims (3 ints per level).
  * kind 0: the reference AC hierarchy (Domain::coarsen rule), kind 1: the
- * engine's aggregation hierarchy. */
+ * engine's aggregation hierarchy (the levels it solves on, in cells of the
+ * grid: pad cells of its storage do not count). */
 int pbg_levels(pbg_session *s, int kind, int *count, int *dims, int cap);
 /* Coarse matrix of the reference AC hierarchy, level l (7 compact arrays
  * c,w,e,s,n,b,t concatenated, AC::coarsen_system). */

@@ -1202,7 +1202,7 @@ int pbg_levels(pbg_session *s, int kind, int *count, int *dims, int cap) {
       for (auto &l : s->refac->L) { d.push_back(l.nx); d.push_back(l.ny); d.push_back(l.nz); }
     } else {
       ensure_engine(s, false, 0);
-      for (auto &l : s->eng->report) { d.push_back(l.nx); d.push_back(l.ny); d.push_back(l.nz); }
+      for (auto &l : s->eng->L) { d.push_back(l.grid.nx); d.push_back(l.grid.ny); d.push_back(l.grid.nz); }
     }
     *count = (int)d.size() / 3;
     if (dims) for (int q = 0; q < (int)d.size() && q < 3 * cap; ++q) dims[q] = d[q];

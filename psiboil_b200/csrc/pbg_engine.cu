@@ -377,14 +377,6 @@ void Engine::build(const EMat<double> &A0_, cudaStream_t s, bool mixed) {
   w64.L.clear();
   w32.L.clear();
   L.clear();
-  // levels of the grid itself, as pbg_levels and the results report them
-  report.clear();
-  report.push_back({A0_.nx, A0_.ny, A0_.nz});
-  for (;;) {
-    const Dims d = report.back();
-    if ((long long)d.nx * d.ny * d.nz <= opt.coarse_max || (d.nx == 1 && d.ny == 1 && d.nz == 1)) break;
-    report.push_back({d.nx > 1 ? (d.nx + 1) / 2 : 1, d.ny > 1 ? (d.ny + 1) / 2 : 1, d.nz > 1 ? (d.nz + 1) / 2 : 1});
-  }
   A0 = A0_;
   const int V = mixed ? VecTraits<float>::V : VecTraits<double>::V;
   auto up = [V](int n) { return (n + V - 1) / V * V; };
@@ -396,6 +388,7 @@ void Engine::build(const EMat<double> &A0_, cudaStream_t s, bool mixed) {
   L.emplace_back();
   {
     ELevel &l0 = L[0];
+    l0.grid = {A0.nx, A0.ny, A0.nz};
     l0.nx = A0.nx; l0.ny = pad.two_d ? 1 : A0.ny; l0.nz = pad.FP;
     l0.d64.alloc(l0.ncell());
     if (pad.any()) {
@@ -412,13 +405,15 @@ void Engine::build(const EMat<double> &A0_, cudaStream_t s, bool mixed) {
   // than coarsened once more, whose visits (two of a level of 65 to 128 cells
   // for each of its own) cost more than the larger inverse.
   const long long dense = opt.coarse_auto ? std::max(opt.coarse_max, kCoarseAuto) : opt.coarse_max;
-  while (L.back().ncell() > dense &&
-         (L.back().nx > 1 || L.back().ny > 1 || L.back().nz > 1)) {
+  // Cells of the grid count, not pad cells: padding adds no level.
+  auto half = [](int n) { return (n + 1) / 2; };
+  while (L.back().grid.ncell() > dense) {
     const ELevel &f = L.back();
     ELevel c;
-    c.nx = f.nx > 1 ? (f.nx + 1) / 2 : 1;
-    c.ny = f.ny > 1 ? (f.ny + 1) / 2 : 1;
-    c.nz = f.nz > 1 ? (f.nz + 1) / 2 : 1;
+    c.grid = {half(f.grid.nx), half(f.grid.ny), half(f.grid.nz)};
+    c.nx = half(f.nx);
+    c.ny = half(f.ny);
+    c.nz = half(f.nz);
     if (padded && c.ncell() >= kPadMin) c.nz = up(c.nz);   // rows of whole vectors here too
     long long n = c.ncell();
     c.c64.alloc(n); c.w64.alloc(n); c.s64.alloc(n); c.b64.alloc(n); c.d64.alloc(n);

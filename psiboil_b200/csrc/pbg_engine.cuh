@@ -61,7 +61,11 @@ struct FcgScal {
 
 // One aggregation level of the engine hierarchy.
 struct ELevel {
-  int nx = 0, ny = 0, nz = 0;
+  struct Dims {
+    int nx = 0, ny = 0, nz = 0;
+    long long ncell() const { return (long long)nx * ny * nz; }
+  } grid;                              // in the caller's shape, without pad cells
+  int nx = 0, ny = 0, nz = 0;          // of the storage (RowPad)
   DBuf<double> c64, w64, s64, b64;     // level >= 1 (level 0 borrows the session's)
   DBuf<double> d64;                    // inverse diagonal (every level)
   DBuf<float> c32, w32, s32, b32, d32; // mixed precision copies
@@ -122,8 +126,6 @@ class Engine {
   RowPad pad;                          // rows of level 0
   EMat<double> A0{};                   // the operator in the caller's rows
   DBuf<double> pc, pw, ps, pb;         // its copy in padded rows
-  struct Dims { int nx, ny, nz; };
-  std::vector<Dims> report;            // levels by the unpadded halving rule
   DBuf<double> Ainv;           // dense inverse of the coarsest operator
   DBuf<float> Ainv32;          // its FP32 copy (mixed path)
   DBuf<__half> Ainv16;         // row-scaled FP16 copy (mixed path, large coarsest levels)
@@ -152,7 +154,7 @@ class Engine {
   EngineResult solve_mixed(double *x, const double *b, double tol, double inner_tol,
                            int max_sweeps, int inner_maxit, RedPool &red, cudaStream_t s,
                            double *hist);
-  int nlevels() const { return (int)report.size(); }
+  int nlevels() const { return (int)L.size(); }
   template <typename T> EMat<T> mat(int l) const;
   template <typename T> const void *ainv() const;
   template <typename T> void dense_solve(const T *r, T *z, const int *stop, cudaStream_t s);

@@ -36,3 +36,26 @@ def test_explicit_coarse_max_is_a_limit(engine, precision, before):
         x = solve(engine, E, P, precision=precision, coarse_max=512)
         assert E.last.levels == 3
         assert np.array_equal(x, ref)
+
+
+@pytest.mark.parametrize("dims,coarse_max,levels", [
+    ((20, 16, 18), 0, [(20, 16, 18), (10, 8, 9)]),                    # 720 cells are the coarsest
+    ((20, 16, 18), 100, [(20, 16, 18), (10, 8, 9), (5, 4, 5)]),
+    ((17, 33, 30), 0, [(17, 33, 30), (9, 17, 15), (5, 9, 8)]),        # padded rows
+    ((66, 71, 1), 0, [(66, 71, 1), (33, 36, 1), (17, 18, 1)]),        # 2-D, padded
+    ((24, 18, 17), 0, [(24, 18, 17), (12, 9, 9)]),                    # 972 cells, stored as 1080
+    ((31, 32, 35), 4096, [(31, 32, 35), (16, 16, 18), (8, 8, 9)]),
+    ((64, 64, 2), 0, [(64, 64, 2), (32, 32, 1)]),                     # thin
+    ((9, 5, 7), 0, [(9, 5, 7)]),
+])
+def test_levels_are_those_of_the_hierarchy(engine, dims, coarse_max, levels):
+    """pbg_levels and pbg_result.levels: the levels that are solved on, with
+    the extents of the caller's grid halved (no pad cells)."""
+    P = problem(dims, False)
+    with engine.Session(*dims, P.h) as s:
+        s.upload_matrix(P.A)
+        E = engine.Engine(s)
+        for precision in (0, 1):
+            solve(engine, E, P, precision=precision, coarse_max=coarse_max)
+            assert E.last.levels == len(levels)
+            assert s.levels(1) == levels
