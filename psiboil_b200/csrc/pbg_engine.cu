@@ -378,8 +378,10 @@ void Engine::build(const EMat<double> &A0_, cudaStream_t s, bool mixed) {
   w32.L.clear();
   L.clear();
   A0 = A0_;
-  const int V = mixed ? VecTraits<float>::V : VecTraits<double>::V;
-  auto up = [V](int n) { return (n + V - 1) / V * V; };
+  // Rows of whole FP32 vectors in both precisions: a hierarchy serves mixed and
+  // FP64 solves, and an FP64 solve's bits do not depend on which came first.
+  constexpr int V = VecTraits<float>::V;
+  auto up = [](int n) { return (n + V - 1) / V * V; };
   pad = RowPad();
   const bool padded = A0.ncell() >= kPadMin && A0.ncell() <= kPadMax;
   pad.two_d = padded && A0.nz == 1 && A0.ny > 1;

@@ -59,3 +59,18 @@ def test_levels_are_those_of_the_hierarchy(engine, dims, coarse_max, levels):
             solve(engine, E, P, precision=precision, coarse_max=coarse_max)
             assert E.last.levels == len(levels)
             assert s.levels(1) == levels
+
+
+@pytest.mark.parametrize("dims", [(16, 16, 18), (16, 18, 17), (30, 31, 6), (66, 70, 1)])
+def test_fp64_solve_does_not_depend_on_a_mixed_one_before(engine, dims):
+    """The hierarchy that a mixed solve leaves serves FP64 solves too: its
+    rows, and with them the bits, are the same for both."""
+    P = problem(dims, False)
+    with engine.Session(*dims, P.h) as s:
+        s.upload_matrix(P.A)
+        ref = solve(engine, engine.Engine(s), P, precision=engine.FP64)
+    with engine.Session(*dims, P.h) as s:
+        s.upload_matrix(P.A)
+        E = engine.Engine(s)
+        solve(engine, E, P, precision=engine.MIXED)
+        assert np.array_equal(solve(engine, E, P, precision=engine.FP64), ref)
