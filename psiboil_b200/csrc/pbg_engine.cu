@@ -204,6 +204,18 @@ __global__ void __launch_bounds__(256) k_gj_block(int n, int k0, const double *_
 constexpr long long kPadMin = 4096, kPadMax = 1ll << 28;
 constexpr int kCoarseAuto = 1024;
 
+// Stored cells of a row of n: whole FP32 vectors in both precisions (a
+// hierarchy serves mixed and FP64 solves, and an FP64 solve's bits do not
+// depend on which came first), where that adds at most a seventh. Measured
+// there: 7, 14, 22 and 30 cells a row mixed 2 to 7% faster, FP64 from 1.4%
+// slower to even. Above: 10, 13 and 17 cells mixed 2% faster, FP64 3 to 4.5%
+// slower; 5 and 6 cells 3 to 12% slower, and 2 cells 512x512 2.7 -> 3.1 ms.
+constexpr int kRowVec = VecTraits<float>::V;
+static int padded_row(int n) {
+  const int up = (n + kRowVec - 1) / kRowVec * kRowVec;
+  return 7ll * up <= 8ll * n ? up : n;
+}
+
 template <typename T>
 void EWork<T>::ensure(const std::vector<ELevel> &lv) {
   if (L.size() == lv.size() && x0.n == (size_t)lv[0].ncell()) return;
@@ -378,15 +390,12 @@ void Engine::build(const EMat<double> &A0_, cudaStream_t s, bool mixed) {
   w32.L.clear();
   L.clear();
   A0 = A0_;
-  // Rows of whole FP32 vectors in both precisions: a hierarchy serves mixed and
-  // FP64 solves, and an FP64 solve's bits do not depend on which came first.
-  constexpr int V = VecTraits<float>::V;
-  auto up = [](int n) { return (n + V - 1) / V * V; };
   pad = RowPad();
   const bool padded = A0.ncell() >= kPadMin && A0.ncell() <= kPadMax;
-  pad.two_d = padded && A0.nz == 1 && A0.ny > 1;
+  // rows along j only where the 16-byte kernels can run on them
+  pad.two_d = padded && A0.nz == 1 && padded_row(A0.ny) % kRowVec == 0;
   pad.F = pad.two_d ? A0.ny : A0.nz;
-  pad.FP = padded ? up(pad.F) : pad.F;
+  pad.FP = padded ? padded_row(pad.F) : pad.F;
   L.emplace_back();
   {
     ELevel &l0 = L[0];
@@ -416,7 +425,7 @@ void Engine::build(const EMat<double> &A0_, cudaStream_t s, bool mixed) {
     c.nx = half(f.nx);
     c.ny = half(f.ny);
     c.nz = half(f.nz);
-    if (padded && c.ncell() >= kPadMin) c.nz = up(c.nz);   // rows of whole vectors here too
+    if (padded && c.ncell() >= kPadMin) c.nz = padded_row(c.nz);   // rows of whole vectors here too
     long long n = c.ncell();
     c.c64.alloc(n); c.w64.alloc(n); c.s64.alloc(n); c.b64.alloc(n); c.d64.alloc(n);
     c.m64 = make_emat<double>(c.nx, c.ny, c.nz, c.c64.p, c.w64.p, c.s64.p, c.b64.p, c.d64.p);
