@@ -428,17 +428,19 @@ class BatchEngine : public BatchEngineBase {
     if (nt > tile_cap_) {
       PBG_CUDA(cudaStreamSynchronize(stream));
       drop_graphs();  // kernel arguments point at the old arrays
+      tile_cap_ = 0;   // stays so where an allocation fails
+      dtiles_.alloc(nt + nt / 2);
+      dpart_.alloc((nt + nt / 2) * 4);
       tile_cap_ = nt + nt / 2;
-      dtiles_.alloc(tile_cap_);
-      dpart_.alloc(tile_cap_ * 4);
     }
     const size_t bytes = sizeof(BTile) * tiles.size() + sizeof(int) * (lbeg.size() + 2 * tbeg.size());
     PBG_CUDA(cudaStreamSynchronize(stream));  // the staging buffer may feed an earlier copy
     if (bytes > htile_cap_) {
       if (htile_) cudaFreeHost(htile_);
       htile_ = nullptr;
+      htile_cap_ = 0;
+      PBG_CUDA(cudaMallocHost((void **)&htile_, bytes + bytes / 2));
       htile_cap_ = bytes + bytes / 2;
-      PBG_CUDA(cudaMallocHost((void **)&htile_, htile_cap_));
     }
     char *h = htile_;
     std::memcpy(h, tiles.data(), sizeof(BTile) * tiles.size());

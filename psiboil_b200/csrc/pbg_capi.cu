@@ -251,11 +251,10 @@ void d2h(pbg_session *s, void *host, const void *dev, size_t n, void *stage) {
 }
 
 void ensure_staging(pbg_session *s) {
-  if (!s->px) {
-    PBG_CUDA(cudaMallocHost((void **)&s->px, sizeof(double) * s->ncell()));
-    PBG_CUDA(cudaMallocHost((void **)&s->pb, sizeof(double) * s->ncell()));
-  }
-  if (s->dx.n == 0) { s->dx.alloc(s->ncell()); s->db.alloc(s->ncell()); }
+  if (!s->px) PBG_CUDA(cudaMallocHost((void **)&s->px, sizeof(double) * s->ncell()));
+  if (!s->pb) PBG_CUDA(cudaMallocHost((void **)&s->pb, sizeof(double) * s->ncell()));
+  s->dx.fit(s->ncell());
+  s->db.fit(s->ncell());
 }
 
 void invalidate(pbg_session *s) {
@@ -451,8 +450,8 @@ int pbg_matrix_upload(pbg_session *s, const double *c, const double *w, const do
     A.nx = s->nx; A.ny = s->ny; A.nz = s->nz;
     A.per = s->per;
     // same-size uploads keep the buffers (the engine then refreshes in place)
-    if (A.c.n != (size_t)N) { A.c.alloc(N); A.w.alloc(N); A.s.alloc(N); A.b.alloc(N); }
-    if (A.e.n != (size_t)N) { A.e.alloc(N); A.n.alloc(N); A.t.alloc(N); }
+    for (DBuf<double> *a : {&A.c, &A.w, &A.s, &A.b}) a->fit(N);
+    for (DBuf<double> *a : {&A.e, &A.n, &A.t}) a->fit(N);
     const double *src[7] = {c, w, e, sv, n, b, t};
     DBuf<double> *dst[7] = {&A.c, &A.w, &A.e, &A.s, &A.n, &A.b, &A.t};
     for (int q = 0; q < 7; ++q) upload_compact(s, src[q], dst[q]->p, si, sj, sk, offset, where);
@@ -536,7 +535,7 @@ int pbg_ci_upload(pbg_session *s, const double *ci, long long si, long long sj, 
   if (!s->have_matrix) return fail(PBG_ERR_STATE, "no matrix uploaded or assembled");
   return guard(s, [&]() -> int {
     const long long N = s->ncell();
-    if (s->ci.n != (size_t)N) s->ci.alloc(N);
+    s->ci.fit(N);
     if (where == PBG_HOST) {
       std::vector<double> h(N);
       gather(ci, h.data(), s->nx, s->ny, s->nz, si, sj, sk, offset);
@@ -583,13 +582,13 @@ int pbg_body_upload(pbg_session *s, const double *fV, const double *fS, int wher
       idx[p] = (int)(fs.size() / 6);
       for (int d = 0; d < 6; ++d) fs.push_back(f[(size_t)d * N + p]);
     }
-    s->ncut = (long long)(fs.size() / 6);
     s->boff.alloc(N);
     s->bidx.alloc(N);
     s->bfs.alloc(fs.empty() ? 6 : fs.size());
     PBG_CUDA(cudaMemcpy(s->boff.p, off.data(), N, cudaMemcpyHostToDevice));
     PBG_CUDA(cudaMemcpy(s->bidx.p, idx.data(), N * sizeof(int), cudaMemcpyHostToDevice));
     if (!fs.empty()) PBG_CUDA(cudaMemcpy(s->bfs.p, fs.data(), fs.size() * 8, cudaMemcpyHostToDevice));
+    s->ncut = (long long)(fs.size() / 6);   // the body counts from here on
     return PBG_OK;
   });
 }
@@ -611,7 +610,7 @@ int pbg_assemble_pressure(pbg_session *s, const double *rho, const uint8_t *soli
     }
     Mat64 &A = s->A;
     A.nx = s->nx; A.ny = s->ny; A.nz = s->nz; A.sym = true;
-    if (A.c.n != (size_t)N) { A.c.alloc(N); A.w.alloc(N); A.s.alloc(N); A.b.alloc(N); }
+    for (DBuf<double> *a : {&A.c, &A.w, &A.s, &A.b}) a->fit(N);
     A.e.release(); A.n.release(); A.t.release();
     k_assemble<<<grid_for(N), kThreads, 0, s->stream>>>(
         s->nx, s->ny, s->nz, s->h, make_int4(s->bc[0], s->bc[1], s->bc[2], s->bc[3]),
@@ -654,10 +653,11 @@ int pbg_assemble_mix(pbg_session *s, const double *col, double rho_a, double rho
     // a cut body's face fractions differ between the two cells of a face:
     // the seven-array form
     const bool sym = bd.idx == nullptr;
-    A.nx = s->nx; A.ny = s->ny; A.nz = s->nz; A.sym = sym;
-    if (A.c.n != (size_t)N) { A.c.alloc(N); A.w.alloc(N); A.s.alloc(N); A.b.alloc(N); }
+    A.nx = s->nx; A.ny = s->ny; A.nz = s->nz;
+    for (DBuf<double> *a : {&A.c, &A.w, &A.s, &A.b}) a->fit(N);
+    if (!sym) for (DBuf<double> *a : {&A.e, &A.n, &A.t}) a->fit(N);
+    A.sym = sym;   // seven arrays only once they are there
     if (sym) { A.e.release(); A.n.release(); A.t.release(); }
-    else if (A.e.n != (size_t)N) { A.e.alloc(N); A.n.alloc(N); A.t.alloc(N); }
     if (flow_vec(s, bd.idx != nullptr)) {
       km_assemble_mix<kAsmV><<<march_grid(s->nx, s->ny, s->nz, kAsmV), kThreads, 0, s->stream>>>(
           s->nx, s->ny, s->nz, march_kq(s->nz, kAsmV), march_len(s->nx, s->ny, s->nz, kAsmV),
@@ -831,7 +831,7 @@ int pbg_pressure_step(pbg_session *s, const double *col, double rho_a, double rh
     const double *cp = col;
     const uint8_t *sp = solid;
     double *pp = p;
-    if (s->frhs.n != (size_t)N) s->frhs.alloc(N);
+    s->frhs.fit(N);
     if (where == PBG_HOST) {
       if (col) {
         dcol.alloc(N);
@@ -896,7 +896,7 @@ void ensure_engine(pbg_session *s, bool mixed, int coarse_max) {
       // a cut body's matrix: the hierarchy from its symmetric part, the
       // refinement against the matrix itself
       const long long N = s->ncell();
-      if (s->symc.n != (size_t)N) { s->symc.alloc(N); s->symw.alloc(N); s->syms.alloc(N); s->symb.alloc(N); }
+      for (DBuf<double> *a : {&s->symc, &s->symw, &s->syms, &s->symb}) a->fit(N);
       symmetrize(A.view(), s->symc.p, s->symw.p, s->syms.p, s->symb.p, s->stream);
       m = make_emat<double>(A.nx, A.ny, A.nz, s->symc.p, s->symw.p, s->syms.p, s->symb.p, nullptr);
       s->eng->top = A.view();
@@ -906,7 +906,12 @@ void ensure_engine(pbg_session *s, bool mixed, int coarse_max) {
       s->eng_dirty = false;
       return;
     }
-    s->eng->build(m, s->stream, mixed || s->eng_mixed);
+    try {
+      s->eng->build(m, s->stream, mixed || s->eng_mixed);
+    } catch (...) {
+      s->eng->L.clear();   // no refresh of a part of a hierarchy
+      throw;
+    }
     s->eng_mixed = s->eng_mixed || mixed;
     s->eng_dirty = false;
   }

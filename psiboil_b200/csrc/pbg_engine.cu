@@ -220,6 +220,7 @@ template <typename T>
 void EWork<T>::ensure(const std::vector<ELevel> &lv) {
   if (L.size() == lv.size() && x0.n == (size_t)lv[0].ncell()) return;
   drop_graph();
+  x0.release();   // the last one allocated: its size says that all are there
   L.clear();
   L.resize(lv.size());
   for (size_t l = 0; l < lv.size(); ++l) {
@@ -229,7 +230,7 @@ void EWork<T>::ensure(const std::vector<ELevel> &lv) {
     if (l > 0) { v.z1.alloc(n); v.z2.alloc(n); v.q1.alloc(n); v.r1.alloc(n); v.v.alloc(n); }
   }
   size_t n0 = (size_t)lv[0].ncell();
-  x0.alloc(n0); r0.alloc(n0); z0.alloc(n0); pA.alloc(n0); pB.alloc(n0); q0.alloc(n0);
+  r0.alloc(n0); z0.alloc(n0); pA.alloc(n0); pB.alloc(n0); q0.alloc(n0);
   q0b.alloc(n0);
   ks.alloc(lv.size());
   fs.alloc(1);
@@ -237,6 +238,7 @@ void EWork<T>::ensure(const std::vector<ELevel> &lv) {
   // the refinement's residual is written to the cells of padded rows only
   PBG_CUDA(cudaMemset(L[0].b.p, 0, L[0].b.bytes()));
   PBG_CUDA(cudaStreamSynchronize(0));
+  x0.alloc(n0);
 }
 
 template <typename T>

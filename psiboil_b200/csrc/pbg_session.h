@@ -25,10 +25,23 @@ struct DBuf {
     return *this;
   }
   ~DBuf() { release(); }
+  // A failed allocation leaves the buffer empty (n = 0), so that a later call
+  // allocates again instead of taking it for whole, and no error behind for
+  // that call's launch checks.
   void alloc(size_t count) {
     release();
+    if (!count) return;
+    void *q = nullptr;
+    const cudaError_t e = cudaMalloc(&q, sizeof(T) * count);
+    if (e != cudaSuccess) {
+      (void)cudaGetLastError();
+      throw CudaError(std::string("cudaMalloc: ") + cudaGetErrorString(e));
+    }
+    p = static_cast<T *>(q);
     n = count;
-    if (count) PBG_CUDA(cudaMalloc((void **)&p, sizeof(T) * (count ? count : 1)));
+  }
+  void fit(size_t count) {
+    if (n != count) alloc(count);
   }
   void release() {
     if (p) cudaFree(p);
