@@ -1216,7 +1216,7 @@ Ic3Factor RefKrylovWork::ic3(size_t n) {
 
 // the operands of the sweeps in march order, `planes` a cell
 double *RefKrylovWork::march(const SweepGeo &g, int planes) {
-  const size_t n = g.all_rows() * planes * kSweepCols;
+  const size_t n = g.all_rows() * planes * g.cols;
   if (mo.n < n) mo.alloc(n);
   return mo.p;
 }
@@ -1261,8 +1261,9 @@ static void ic_form(const MatView<double> &A, int kind, RefKrylovWork &w, cudaSt
   double *M = w.march(g, ic_planes(kind));
   if (w.z.n < (size_t)A.ncell()) w.z.alloc((size_t)A.ncell());
   w.sweep_alloc(g.words() * (kind == 2 ? 2 : 1), s);
-  if (kind == 2) k_ic_factor<2><<<g.tiles(), kSweepThreads, 0, s>>>(g, A, M, w.sweep());
-  else k_ic_factor<1><<<g.tiles(), kSweepThreads, 0, s>>>(g, A, M, w.sweep());
+  auto *form = kind == 2 ? (g.full() ? k_ic_factor<2, true> : k_ic_factor<2, false>)
+                         : (g.full() ? k_ic_factor<1, true> : k_ic_factor<1, false>);
+  form<<<g.tiles(), kSweepThreads, 0, s>>>(g, A, M, w.sweep());
   note_launch();
 }
 
@@ -1284,7 +1285,7 @@ void enqueue_ref_setup(const MatView<double> &A, double *x, const double *b, con
     if (solver == 4 && !A.per) {  // the sweeps' operands in march order
       const SweepGeo sg = SweepGeo::make(A.nx, A.ny, A.nz, sweep_a(1));
       w.sweep_alloc(sg.words(), s);
-      k_gs_pack<<<grid_for((long long)sg.all_rows() * kSweepCols), kThreads, 0, s>>>(sg, A, w.ci, b, x,
+      k_gs_pack<<<grid_for((long long)sg.all_rows() * sg.cols), kThreads, 0, s>>>(sg, A, w.ci, b, x,
                                                                                  w.march(sg, kGsPlanes)); note_launch();
     }
     (exact ? k_it_init<true> : k_it_init<false>)<<<g, kThreads, 0, s>>>(A, x, b, w.r.p, st, red.slot_part(0), red.slot_count(0),
@@ -1327,14 +1328,12 @@ static void ic_apply(const MatView<double> &A, int prec, RefKrylovWork &w, const
   }
   const SweepGeo g = SweepGeo::make(A.nx, A.ny, A.nz, sweep_a(prec));
   double *M = w.march(g, ic_planes(prec));
-  const int n = g.tiles();
-  if (prec == 2) {
-    k_ic_sweep<2, false><<<n, kSweepThreads, 0, s>>>(g, M, r, z, w.sweep(), st);
-    k_ic_sweep<2, true><<<n, kSweepThreads, 0, s>>>(g, M, r, z, w.sweep(), st);
-  } else {
-    k_ic_sweep<1, false><<<n, kSweepThreads, 0, s>>>(g, M, r, z, w.sweep(), st);
-    k_ic_sweep<1, true><<<n, kSweepThreads, 0, s>>>(g, M, r, z, w.sweep(), st);
-  }
+  auto *fwd = prec == 2 ? (g.full() ? k_ic_sweep<2, false, true> : k_ic_sweep<2, false, false>)
+                        : (g.full() ? k_ic_sweep<1, false, true> : k_ic_sweep<1, false, false>);
+  auto *bwd = prec == 2 ? (g.full() ? k_ic_sweep<2, true, true> : k_ic_sweep<2, true, false>)
+                        : (g.full() ? k_ic_sweep<1, true, true> : k_ic_sweep<1, true, false>);
+  fwd<<<g.tiles(), kSweepThreads, 0, s>>>(g, M, r, z, w.sweep(), st);
+  bwd<<<g.tiles(), kSweepThreads, 0, s>>>(g, M, r, z, w.sweep(), st);
   note_launch(); note_launch();
 }
 
@@ -1352,7 +1351,8 @@ void enqueue_ref_iters(const MatView<double> &A, double *x, int solver, int coun
     const SweepGeo sg = SweepGeo::make(A.nx, A.ny, A.nz, sweep_a(1));
     for (int it = 0; it < count; ++it) {
       if (gs && !A.per) {
-        k_gs_sweep<<<sg.tiles(), kSweepThreads, 0, s>>>(sg, w.march(sg, kGsPlanes), x, w.sweep(), st); note_launch();
+        auto *sweep = sg.full() ? k_gs_sweep<true> : k_gs_sweep<false>;
+        sweep<<<sg.tiles(), kSweepThreads, 0, s>>>(sg, w.march(sg, kGsPlanes), x, w.sweep(), st); note_launch();
       } else if (gs) {
         // the halo the exchange fills before each sweep
         if (w.xold.n < (size_t)N) w.xold.alloc(N);

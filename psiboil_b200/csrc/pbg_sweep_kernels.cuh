@@ -140,7 +140,7 @@ __device__ __forceinline__ void sweep_march(const SweepGeo &g, const SweepSync &
   } else if (warp == 3) {
     const SweepPos<BWD> q(g, tile, along_i ? last : m, along_i ? m : last);
     const int start = -A * (last + m) - LOOK;
-    const bool on = used && q.col;
+    const bool on = used && q.col && (along_i ? q.I + 1 < g.ti : q.J + 1 < g.tj);
     const int at = (q.li + 1) * E + q.lj + 1;
     TagWord *p = (along_i ? y.words + ((size_t)q.I * g.ny + q.j) * nz
                             : y.words + g.words_i() + ((size_t)q.J * g.nx + q.i) * nz) + start;
@@ -217,15 +217,28 @@ __device__ __forceinline__ void sweep_march(const SweepGeo &g, const SweepSync &
   sweep_finish(y, g.tiles());
 }
 
+// Distance G of two operands in march order: a constant where tiles have all
+// their columns (0.98-0.99 of the time of the variable one: the memory warps
+// form fewer addresses), else the grid's.
+template <bool FULL> struct MarchStride {
+  static constexpr int G = kSweepCols;
+  __device__ __forceinline__ explicit MarchStride(const SweepGeo &) {}
+};
+template <> struct MarchStride<false> {
+  const int G;
+  __device__ __forceinline__ explicit MarchStride(const SweepGeo &g) : G(g.cols) {}
+};
+
 // Body of a triangular sweep of z = M^-1 r: forward z = (r - lower terms) / c
 // from r (natural order) into the factor's z plane, backward
 // z = (that - upper terms) / c into z (natural order)
 // (preconditioner_solve.cpp:14-110). Terms with a neighbour outside the
 // domain are skipped (the reference multiplies them by its zero halo).
-template <int KIND, bool BWD>
-struct IcBody {
+template <int KIND, bool BWD, bool FULL>
+struct IcBody : MarchStride<FULL> {
+  using MarchStride<FULL>::G;
   static constexpr int P = kSweepAhead, NP = ic_planes(KIND), C = kSweepCols, planes = NP;
-  static constexpr int S = (BWD ? -1 : 1) * NP * C, D = BWD ? -1 : 1;   // a step in march and natural order
+  static constexpr int D = BWD ? -1 : 1;   // a step in natural order
   // coefficient rows: the cell's own (forward), or those of the neighbour
   // whose lower entry is this cell's upper one (backward)
   const double *lO, *lW, *lS, *lr;
@@ -236,8 +249,8 @@ struct IcBody {
   double zB, zW0, zS0;
   __device__ __forceinline__ IcBody(const SweepGeo &g, const SweepPos<BWD> &q, int start, double *M, const double *r,
                                     double *z)
-      : nz(g.nz), hasW(q.hasW), hasS(q.hasS), zB(0.0), zW0(0.0), zS0(0.0) {
-    const long long row = (long long)q.at(g, start) * (NP * C);
+      : MarchStride<FULL>(g), nz(g.nz), hasW(q.hasW), hasS(q.hasS), zB(0.0), zW0(0.0), zS0(0.0) {
+    const long long row = (long long)q.at(g, start) * (NP * G);
     const long long nat = ((long long)q.i * g.ny + q.j) * nz + q.at(g, start);
     lO = zO = M + ((long long)(q.col ? g.off(q.i, q.j, NP) : 0) + row);
     lW = BWD && hasW ? M + ((long long)g.off(q.i + 1, q.j, NP) + row) : lO;
@@ -245,17 +258,18 @@ struct IcBody {
     lr = r + nat;
     lz = z + nat;
   }
+  __device__ __forceinline__ int march_step() const { return D * NP * G; }
   __device__ __forceinline__ void load(int u, int kk, double *d) {
-    const int o = u * S;
-    sweep_copy(d + kIcC * C, lO + o + kIcC * C);
-    sweep_copy(d + kIcY * C, lO + o + kIcY * C);
-    sweep_copy(d + kIcZ * C, BWD ? lO + o + kIcZ * C : lr + u);
-    if (!BWD || hasW) sweep_copy(d + kIcW * C, lW + o + kIcW * C);
-    if (!BWD || hasS) sweep_copy(d + kIcS * C, lS + o + kIcS * C);
-    if (!BWD || kk > 0) sweep_copy(d + kIcB * C, lO + o + kIcB * C - (BWD ? S : 0));
+    const int S = march_step(), o = u * S;
+    sweep_copy(d + kIcC * C, lO + o + kIcC * G);
+    sweep_copy(d + kIcY * C, lO + o + kIcY * G);
+    sweep_copy(d + kIcZ * C, BWD ? lO + o + kIcZ * G : lr + u);
+    if (!BWD || hasW) sweep_copy(d + kIcW * C, lW + o + kIcW * G);
+    if (!BWD || hasS) sweep_copy(d + kIcS * C, lS + o + kIcS * G);
+    if (!BWD || kk > 0) sweep_copy(d + kIcB * C, lO + o + kIcB * G - (BWD ? S : 0));
     if constexpr (KIND == 2) {
-      if (!BWD || (hasW && kk + 1 < nz)) sweep_copy(d + kIcTw * C, lW + o + kIcTw * C + (BWD ? S : 0));
-      if (!BWD || (hasS && kk + 1 < nz)) sweep_copy(d + kIcTs * C, lS + o + kIcTs * C + (BWD ? S : 0));
+      if (!BWD || (hasW && kk + 1 < nz)) sweep_copy(d + kIcTw * C, lW + o + kIcTw * G + (BWD ? S : 0));
+      if (!BWD || (hasS && kk + 1 < nz)) sweep_copy(d + kIcTs * C, lS + o + kIcTs * G + (BWD ? S : 0));
     }
   }
   __device__ __forceinline__ void fetch(const double *d) {
@@ -264,11 +278,12 @@ struct IcBody {
     if constexpr (KIND == 2) { ctw = d[kIcTw * C]; cts = d[kIcTs * C]; }
   }
   __device__ __forceinline__ void next() {
+    const int S = march_step();
     lO += P * S; lW += P * S; lS += P * S; lr += P * D; zO += P * S; lz += P * D;
   }
   __device__ __forceinline__ void store(int u, double z) {
     if (BWD) lz[u * D] = z;
-    else zO[u * S + kIcZ * C] = z;
+    else zO[u * march_step() + kIcZ * G] = z;
   }
   __device__ __forceinline__ void before(const double *w, const double *s) {
     if constexpr (KIND == 1) { zW0 = w[0]; zS0 = s[0]; }
@@ -288,12 +303,12 @@ struct IcBody {
   }
 };
 
-template <int KIND, bool BWD>
+template <int KIND, bool BWD, bool FULL>
 __global__ void __launch_bounds__(kSweepThreads) k_ic_sweep(SweepGeo g, double *M, const double *__restrict__ r,
                                                             double *__restrict__ z, SweepSync y,
                                                             const KrylovState *st) {
   if (st->done) return;
-  sweep_march<1, sweep_a(KIND), KIND == 2 ? 1 : 0, BWD, IcBody<KIND, BWD>>(g, y, M, r, z);
+  sweep_march<1, sweep_a(KIND), KIND == 2 ? 1 : 0, BWD, IcBody<KIND, BWD, FULL>>(g, y, M, r, z);
 }
 
 // IncompleteCholesky0/2::form (preconditioner_form.cpp:16-98) in march
@@ -305,8 +320,9 @@ __global__ void __launch_bounds__(kSweepThreads) k_ic_sweep(SweepGeo g, double *
 //   c = sqrt(A.c - w^2 - tw^2 - s^2 - ts^2 - b^2),
 // so only c and b travel between columns. Entries whose p lies outside the
 // domain are zero.
-template <int KIND>
-struct IcFormBody {
+template <int KIND, bool FULL>
+struct IcFormBody : MarchStride<FULL> {
+  using MarchStride<FULL>::G;
   static constexpr int P = kSweepAhead, NP = ic_planes(KIND), C = kSweepCols, planes = 4;
   const double *ac, *aw, *as, *ab;
   double *o_;
@@ -316,16 +332,16 @@ struct IcFormBody {
   double cB, twB, tsB, cW0, cS0;
   __device__ __forceinline__ IcFormBody(const SweepGeo &g, const SweepPos<false> &q, int start,
                                         const MatView<double> &A, double *M)
-      : nz(g.nz), hasW(q.hasW), hasS(q.hasS), cB(0.0), twB(0.0), tsB(0.0), cW0(0.0), cS0(0.0) {
+      : MarchStride<FULL>(g), nz(g.nz), hasW(q.hasW), hasS(q.hasS), cB(0.0), twB(0.0), tsB(0.0), cW0(0.0), cS0(0.0) {
     const long long nat = ((long long)q.i * g.ny + q.j) * nz + start;
     ac = A.c + nat; aw = A.w + nat; as = A.s + nat; ab = A.b + nat;
-    o_ = M + ((long long)(q.col ? g.off(q.i, q.j, NP) : 0) + (long long)start * (NP * C));
+    o_ = M + ((long long)(q.col ? g.off(q.i, q.j, NP) : 0) + (long long)start * (NP * G));
   }
   __device__ __forceinline__ void load(int u, int, double *d) {
     sweep_copy(d, ac + u); sweep_copy(d + C, aw + u); sweep_copy(d + 2 * C, as + u); sweep_copy(d + 3 * C, ab + u);
   }
   __device__ __forceinline__ void fetch(const double *d) { rc = d[0]; rw = d[C]; rs = d[2 * C]; rb = d[3 * C]; }
-  __device__ __forceinline__ void next() { ac += P; aw += P; as += P; ab += P; o_ += P * NP * C; }
+  __device__ __forceinline__ void next() { ac += P; aw += P; as += P; ab += P; o_ += P * NP * G; }
   __device__ __forceinline__ void store(int, double) {}   // the arithmetic warps hold the factor
   __device__ __forceinline__ void before(const double *w, const double *s) {
     if constexpr (KIND == 1) { cW0 = w[0]; cS0 = s[0]; }
@@ -354,36 +370,36 @@ struct IcFormBody {
     c = __dsqrt_rn(msub(c, b, b));
     out[0] = c;
     if constexpr (KIND == 2) out[1] = b;
-    double *o = o_ + u * (NP * C);
-    o[kIcC * C] = c;
-    o[kIcY * C] = KnownDiv(c).recip();
-    o[kIcW * C] = w; o[kIcS * C] = s; o[kIcB * C] = b;
-    if constexpr (KIND == 2) { o[kIcTw * C] = tw; o[kIcTs * C] = ts; }
+    double *o = o_ + u * (NP * G);
+    o[kIcC * G] = c;
+    o[kIcY * G] = KnownDiv(c).recip();
+    o[kIcW * G] = w; o[kIcS * G] = s; o[kIcB * G] = b;
+    if constexpr (KIND == 2) { o[kIcTw * G] = tw; o[kIcTs * G] = ts; }
     cB = c; twB = tw; tsB = ts;
   }
 };
 
-template <int KIND>
+template <int KIND, bool FULL>
 __global__ void __launch_bounds__(kSweepThreads) k_ic_factor(SweepGeo g, MatView<double> A, double *M, SweepSync y) {
-  sweep_march<KIND == 2 ? 2 : 1, sweep_a(KIND), KIND == 2 ? 1 : 0, false, IcFormBody<KIND>>(g, y, A, M);
+  sweep_march<KIND == 2 ? 2 : 1, sweep_a(KIND), KIND == 2 ? 1 : 0, false, IcFormBody<KIND, FULL>>(g, y, A, M);
 }
 
 __global__ void k_gs_pack(SweepGeo g, MatView<double> A, const double *__restrict__ ci,
                           const double *__restrict__ b, const double *__restrict__ x, double *o) {
-  const size_t n = g.all_rows() * kSweepCols;
+  const size_t n = g.all_rows() * g.cols;
   for (size_t m = blockIdx.x * (size_t)blockDim.x + threadIdx.x; m < n; m += (size_t)gridDim.x * blockDim.x) {
-    const int c = (int)(m % kSweepCols);
-    const size_t row = m / kSweepCols;
-    const int tile = (int)(row / g.rows), li = c / kSweepTile, lj = c % kSweepTile;
+    const size_t row = m / g.cols;
+    const int c = (int)(m - row * g.cols);
+    const int tile = (int)(row / g.rows), li = c / g.wj, lj = c - li * g.wj;
     const int k = (int)(row - (size_t)tile * g.rows) - g.skew * (li + lj);
     const int i = tile / g.tj * kSweepTile + li, j = tile % g.tj * kSweepTile + lj;
     if (i >= g.nx || j >= g.ny || k < 0 || k >= g.nz) continue;
     const long long p = ((long long)i * g.ny + j) * g.nz + k;
     const Nb<double> a = coeffs(A, p, Pos{i, j, k});
-    double *w = o + row * (kGsPlanes * kSweepCols) + c;
+    double *w = o + row * (kGsPlanes * g.cols) + c;
     const double v[kGsPlanes] = {b[p], ci[p], a.w, a.e, a.s, a.n, a.b, a.t, x[p]};
 #pragma unroll
-    for (int f = 0; f < kGsPlanes; ++f) w[f * kSweepCols] = v[f];
+    for (int f = 0; f < kGsPlanes; ++f) w[f * g.cols] = v[f];
   }
 }
 
@@ -393,8 +409,10 @@ __global__ void k_gs_pack(SweepGeo g, MatView<double> A, const double *__restric
 // old values are loaded before their cells' new ones are formed: those wait,
 // directly or through the exchange, for this cell's own result. A neighbour
 // outside the domain counts as zero.
-struct GsBody {
-  static constexpr int P = kSweepAhead, C = kSweepCols, S = kGsPlanes * C, planes = kGsPlanes + 2;
+template <bool FULL>
+struct GsBody : MarchStride<FULL> {
+  using MarchStride<FULL>::G;
+  static constexpr int P = kSweepAhead, C = kSweepCols, planes = kGsPlanes + 2;
   const double *lO, *lE, *lN;
   double *xO, *lx;
   int nz;
@@ -402,30 +420,36 @@ struct GsBody {
   double rb, rci, rw, re, rs, rn, rbt, rt, xe, xn, xt;
   double xB;
   __device__ __forceinline__ GsBody(const SweepGeo &g, const SweepPos<false> &q, int start, double *M, double *x)
-      : nz(g.nz), hasW(q.hasW), hasS(q.hasS), hasE(q.col && q.i + 1 < g.nx), hasN(q.col && q.j + 1 < g.ny), xB(0.0) {
-    const long long row = (long long)start * S;
+      : MarchStride<FULL>(g), nz(g.nz), hasW(q.hasW), hasS(q.hasS), hasE(q.col && q.i + 1 < g.nx),
+        hasN(q.col && q.j + 1 < g.ny), xB(0.0) {
+    const long long row = (long long)start * march_step();
     lO = M + ((long long)(q.col ? g.off(q.i, q.j, kGsPlanes) : 0) + row);
     lE = hasE ? M + ((long long)g.off(q.i + 1, q.j, kGsPlanes) + row) : lO;
     lN = hasN ? M + ((long long)g.off(q.i, q.j + 1, kGsPlanes) + row) : lO;
-    xO = const_cast<double *>(lO) + kGsX * C;
+    xO = const_cast<double *>(lO) + kGsX * G;
     lx = x + (((long long)q.i * g.ny + q.j) * nz + start);
   }
+  __device__ __forceinline__ int march_step() const { return kGsPlanes * G; }
   // planes of a stage: the cell's eight operands, then the old x at i + 1, j + 1 and k + 1
   __device__ __forceinline__ void load(int u, int kk, double *d) {
+    const int S = march_step();
     const double *l = lO + u * S;
 #pragma unroll
-    for (int f = 0; f < kGsX; ++f) sweep_copy(d + f * C, l + f * C);
-    if (hasE) sweep_copy(d + kGsX * C, lE + u * S + kGsX * C);
-    if (hasN) sweep_copy(d + (kGsX + 1) * C, lN + u * S + kGsX * C);
-    if (kk + 1 < nz) sweep_copy(d + (kGsX + 2) * C, l + kGsX * C + S);
+    for (int f = 0; f < kGsX; ++f) sweep_copy(d + f * C, l + f * G);
+    if (hasE) sweep_copy(d + kGsX * C, lE + u * S + kGsX * G);
+    if (hasN) sweep_copy(d + (kGsX + 1) * C, lN + u * S + kGsX * G);
+    if (kk + 1 < nz) sweep_copy(d + (kGsX + 2) * C, l + kGsX * G + S);
   }
   __device__ __forceinline__ void fetch(const double *d) {
     rb = d[kGsB * C]; rci = d[kGsCi * C];
     rw = d[kGsW * C]; re = d[kGsE * C]; rs = d[kGsS * C]; rn = d[kGsN * C]; rbt = d[kGsBt * C]; rt = d[kGsT * C];
     xe = d[kGsX * C]; xn = d[(kGsX + 1) * C]; xt = d[(kGsX + 2) * C];
   }
-  __device__ __forceinline__ void next() { lO += P * S; lE += P * S; lN += P * S; xO += P * S; lx += P; }
-  __device__ __forceinline__ void store(int u, double v) { xO[u * S] = v; lx[u] = v; }
+  __device__ __forceinline__ void next() {
+    const int S = march_step();
+    lO += P * S; lE += P * S; lN += P * S; xO += P * S; lx += P;
+  }
+  __device__ __forceinline__ void store(int u, double v) { xO[u * march_step()] = v; lx[u] = v; }
   __device__ __forceinline__ void before(const double *, const double *) {}
   __device__ __forceinline__ void after(const double *, const double *) {}
   __device__ __forceinline__ void step(int u, int kk, const double *w, const double *s, double *o) {
@@ -441,10 +465,11 @@ struct GsBody {
   }
 };
 
+template <bool FULL>
 __global__ void __launch_bounds__(kSweepThreads) k_gs_sweep(SweepGeo g, double *M, double *__restrict__ x, SweepSync y,
                                                             const KrylovState *st) {
   if (st->done) return;
-  sweep_march<1, 1, 0, false, GsBody>(g, y, M, x);
+  sweep_march<1, 1, 0, false, GsBody<FULL>>(g, y, M, x);
 }
 
 }  // namespace pbg

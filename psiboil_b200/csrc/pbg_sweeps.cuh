@@ -13,12 +13,13 @@
 // One block owns the 8 x 8 columns of a tile of the (i, j) plane, a thread
 // each, and marches along k: at step t thread (li, lj) is at
 // k = t - a (li + lj), so the values it needs from the columns beside it
-// were formed in the step before and come from shared memory. Values crossing a tile's edge go through global memory as 16-byte
-// (value, epoch) words written and read whole: a word is valid when it
-// carries the sweep's epoch, so no fence and no reset is needed, and a
-// reader that finds an old word polls it (bounded). Blocks take their tiles
-// by ticket in an order in which every tile's predecessors come first, so a
-// block only ever waits for blocks that are already running.
+// were formed in the step before and come from shared memory. Values crossing
+// a tile's edge go through global memory as 16-byte (value, epoch) words
+// written and read whole: a word is valid when it carries the sweep's epoch,
+// so no fence and no reset is needed, and a reader that finds an old word
+// polls it (bounded). Blocks take their tiles by ticket in an order in which
+// every tile's predecessors come first, so a block only ever waits for blocks
+// that are already running.
 //
 // What bounds it: the chain of a (nx + ny - 2) + nz dependent steps, 0.16 us
 // each for IC0 and 0.21 us for IC2 (shared loads, four to six dependent FP64
@@ -53,6 +54,7 @@ __host__ __device__ constexpr int sweep_a(int kind) { return kind == 2 ? 2 : 1; 
 // Tiles of a grid and the march-order storage of a cell array.
 struct SweepGeo {
   int nx, ny, nz, ti, tj;
+  int wj, cols;     // stored columns of a tile: along j, and in all
   int skew;         // of the storage rows (0 on short columns)
   int rows;         // rows of a tile's storage
   __host__ static SweepGeo make(int nx, int ny, int nz, int a) {
@@ -60,23 +62,28 @@ struct SweepGeo {
     g.nx = nx; g.ny = ny; g.nz = nz;
     g.ti = (nx + kSweepTile - 1) / kSweepTile;
     g.tj = (ny + kSweepTile - 1) / kSweepTile;
+    const int wi = nx < kSweepTile ? nx : kSweepTile;   // a thin grid stores the columns it has
+    g.wj = ny < kSweepTile ? ny : kSweepTile;
+    g.cols = wi * g.wj;
     g.skew = nz >= kSweepSkewMin ? a : 0;
-    g.rows = nz + 2 * g.skew * (kSweepTile - 1);
+    g.rows = nz + g.skew * (wi - 1 + g.wj - 1);
     return g;
   }
+  __host__ bool full() const { return cols == kSweepCols; }
   __host__ __device__ int tiles() const { return ti * tj; }
   __host__ __device__ size_t all_rows() const { return (size_t)tiles() * rows; }
-  // Storage: a row holds `planes` operands of its 64 cells one after the
-  // other. Index of operand 0 of cell (i, j, 0); the cell (i, j, k) is k
-  // rows further, the next operand kSweepCols further.
+  // Storage: a row holds `planes` operands of its cells one after the other.
+  // Index of operand 0 of cell (i, j, 0); the cell (i, j, k) is k rows
+  // further, the next operand cols further.
   __device__ __forceinline__ size_t off(int i, int j, int planes) const {
     const int li = i % kSweepTile, lj = j % kSweepTile;
     const size_t tile = (size_t)(i / kSweepTile) * tj + j / kSweepTile;
-    return (tile * rows + skew * (li + lj)) * planes * kSweepCols + li * kSweepTile + lj;
+    return (tile * rows + skew * (li + lj)) * planes * cols + li * wj + lj;
   }
-  // words of one exchanged value: the tiles' last columns along i, then along j
-  __host__ __device__ size_t words_i() const { return (size_t)ti * ny * nz; }
-  __host__ __device__ size_t words() const { return words_i() + (size_t)tj * nx * nz; }
+  // words of one exchanged value: the last columns along i, then along j, of
+  // the tiles that have one after them
+  __host__ __device__ size_t words_i() const { return (size_t)(ti - 1) * ny * nz; }
+  __host__ __device__ size_t words() const { return words_i() + (size_t)(tj - 1) * nx * nz; }
 };
 
 // Shared state of the sweeps of one solver's workspace.

@@ -7,7 +7,8 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-DIMS = [(7, 9, 5), (8, 8, 8), (9, 17, 33), (24, 16, 31), (2, 30, 67), (33, 3, 2), (17, 25, 1), (40, 41, 32)]
+DIMS = [(7, 9, 5), (8, 8, 8), (9, 17, 33), (24, 16, 31), (2, 30, 67), (33, 3, 2), (17, 25, 1), (40, 41, 32),
+        (1, 20, 33), (19, 1, 33), (1, 1, 44), (3, 5, 33)]
 
 
 def problem(dims, convect):
@@ -53,3 +54,28 @@ def test_sweeps_bit_exact(engine, oracle, dims, solver, prec, steps, convect):
             x[:] = 0.0
             kr.solve(x, P.b.copy(), 1, steps, None, 1e-30, 1e-30)
             assert np.array_equal(x, xo)
+
+
+@pytest.mark.parametrize("dims", [(1, 700, 800), (700, 1, 800), (1, 1, 200000), (3, 400, 400)])
+@pytest.mark.parametrize("solver,prec", [("cg", "ic2"), ("gs", "di")])
+def test_thin_grids_take_memory_by_their_cells(engine, dims, solver, prec):
+    """The sweeps' storage holds the columns that exist: a grid of one or few
+    columns along i or j takes no more than 1.5 times the memory per cell of
+    one whose tiles are full (8, 8, 64 and 2.7 times with whole tiles)."""
+    torch = pytest.importorskip("torch")
+
+    def mem(d):
+        n = d[0] * d[1] * d[2]
+        rho = torch.ones(n, dtype=torch.float64, device="cuda")
+        solid = torch.zeros(n, dtype=torch.uint8, device="cuda")
+        b = torch.sin(torch.arange(n, dtype=torch.float64, device="cuda"))
+        x = torch.zeros(n, dtype=torch.float64, device="cuda")
+        with engine.Session(*d, 1.0) as s:
+            s.assemble_pressure(rho, solid)
+            kr = engine.GaussSeidel(s) if solver == "gs" else engine.CG(s, prec=prec)
+            torch.cuda.synchronize()
+            free = torch.cuda.mem_get_info()[0]
+            kr.solve(x, b, 1, 2, None, 1e-30, 1e-30)
+            torch.cuda.synchronize()
+            return (free - torch.cuda.mem_get_info()[0]) / n
+    assert mem(dims) <= 1.5 * mem((40, 40, 800))
