@@ -1040,8 +1040,8 @@ __global__ void k_ac_resnorm(MatView<double> A, const double *__restrict__ phi,
 // cells after it. Every neighbour of (i, j, k) lies on the hyperplane
 // i + j + k - 1 (those before it) or i + j + k + 1 (those after it), so a
 // schedule that keeps the planes' order computes every cell from exactly the
-// values the sequential sweep uses: k_gs_sweep (pbg_sweeps.cuh), or on
-// periodic matrices one launch of k_gs_plane per plane.
+// values the sequential sweep uses: k_gs_sweep (pbg_sweeps.cuh), or one
+// launch of k_gs_plane per plane.
 // ---------------------------------------------------------------------------
 // all entries unreal (gaussseidel.cpp:28-33; CG also seeds the last with res0)
 __device__ void stale_fill_dev(KrylovState *st) {
@@ -1102,7 +1102,8 @@ __global__ void k_jacobi_x(long long N, const double *__restrict__ c, const doub
     x[p] = __dmul_rn(ci[p], __dadd_rn(r[p], __dmul_rn(c[p], x[p])));
 }
 
-// periodic matrices: the cells of hyperplane h: x = ci (b + w xw + e xe + s xs + n xn + b xb
+// periodic matrices, and where the one-launch sweep's operands do not fit in
+// memory: the cells of hyperplane h: x = ci (b + w xw + e xe + s xs + n xn + b xb
 // + t xt), summed left to right (gaussseidel.cpp:50-60). One thread per
 // (i, j) column; k = h - i - j. Across a periodic face the reference reads
 // its halo, filled by the exchange before the sweep: xold, a copy of x
@@ -1237,6 +1238,19 @@ void RefKrylovWork::sweep_alloc(size_t n, cudaStream_t s) {
   }
 }
 
+// Memory of the Gauss-Seidel sweep; false where it does not fit beside the
+// rest (72 bytes a cell): the sweeps then run plane by plane, the same bits.
+bool RefKrylovWork::gs_alloc(const SweepGeo &g, cudaStream_t s) {
+  try {
+    march(g, kGsPlanes);
+    sweep_alloc(g.words(), s);
+  } catch (const CudaError &) {
+    mo.release();
+    return false;
+  }
+  return true;
+}
+
 void RefKrylovWork::sweep_check_enqueue(cudaStream_t s) {
   if (ticket.n) PBG_CUDA(cudaMemcpyAsync(hstuck, ticket.p + 2, sizeof(int), cudaMemcpyDeviceToHost, s));
 }
@@ -1282,9 +1296,9 @@ void enqueue_ref_setup(const MatView<double> &A, double *x, const double *b, con
       k_recip<<<grid_for(N), kThreads, 0, s>>>(N, A.c, w.mcd.p); note_launch();
       w.ci = w.mcd.p;
     }
-    if (solver == 4 && !A.per) {  // the sweeps' operands in march order
-      const SweepGeo sg = SweepGeo::make(A.nx, A.ny, A.nz, sweep_a(1));
-      w.sweep_alloc(sg.words(), s);
+    const SweepGeo sg = SweepGeo::make(A.nx, A.ny, A.nz, sweep_a(1));
+    w.gs_march = solver == 4 && !A.per && w.gs_alloc(sg, s);
+    if (w.gs_march) {  // the sweeps' operands in march order
       k_gs_pack<<<grid_for((long long)sg.all_rows() * sg.cols), kThreads, 0, s>>>(sg, A, w.ci, b, x,
                                                                                  w.march(sg, kGsPlanes)); note_launch();
     }
@@ -1350,13 +1364,14 @@ void enqueue_ref_iters(const MatView<double> &A, double *x, int solver, int coun
     const int H = A.nx + A.ny + A.nz - 2, gp = grid_for((long long)A.nx * A.ny);
     const SweepGeo sg = SweepGeo::make(A.nx, A.ny, A.nz, sweep_a(1));
     for (int it = 0; it < count; ++it) {
-      if (gs && !A.per) {
+      if (gs && w.gs_march) {
         auto *sweep = sg.full() ? k_gs_sweep<true> : k_gs_sweep<false>;
         sweep<<<sg.tiles(), kSweepThreads, 0, s>>>(sg, w.march(sg, kGsPlanes), x, w.sweep(), st); note_launch();
       } else if (gs) {
-        // the halo the exchange fills before each sweep
-        if (w.xold.n < (size_t)N) w.xold.alloc(N);
-        PBG_CUDA(cudaMemcpyAsync(w.xold.p, x, sizeof(double) * N, cudaMemcpyDeviceToDevice, s));
+        if (A.per) {  // the halo the exchange fills before each sweep
+          if (w.xold.n < (size_t)N) w.xold.alloc(N);
+          PBG_CUDA(cudaMemcpyAsync(w.xold.p, x, sizeof(double) * N, cudaMemcpyDeviceToDevice, s));
+        }
         for (int h = 0; h < H; ++h) {
           k_gs_plane<<<gp, kThreads, 0, s>>>(A, w.ci, w.rhs, x, h, st, w.xold.p); note_launch();
         }

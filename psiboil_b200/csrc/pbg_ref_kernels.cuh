@@ -40,7 +40,9 @@ struct RefKrylovWork {
   ~RefKrylovWork();
   void ensure(size_t n, int solver);
   Ic3Factor ic3(size_t n);
+  bool gs_march = false;                          // this Gauss-Seidel solve runs k_gs_sweep
   double *march(const SweepGeo &g, int planes);
+  bool gs_alloc(const SweepGeo &g, cudaStream_t s);
   void sweep_alloc(size_t words_needed, cudaStream_t s);
   SweepSync sweep() {
     return {words.p, ticket.p, reinterpret_cast<int *>(ticket.p + 2), ++epoch};

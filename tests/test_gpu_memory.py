@@ -5,6 +5,13 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
+
+@pytest.fixture(autouse=True)
+def give_memory_back():
+    yield
+    import torch
+    torch.cuda.empty_cache()   # torch keeps what it freed
+
 DIMS = (160, 152, 161)   # 3.9 M cells: 31 MB an FP64 array
 
 
@@ -58,6 +65,34 @@ def test_failed_allocation_leaves_the_session_usable(engine, kind):
                 assert "out of memory" in str(e)
                 failed += 1
             del hold
-        torch.cuda.empty_cache()
+        torch.cuda.empty_cache()   # torch keeps what it freed
         assert failed >= 1
         assert torch.equal(run(s), ref)
+
+
+def test_gauss_seidel_without_room_for_its_sweep(engine):
+    """The one-launch sweep's operands (72 bytes a cell, 281 MB here) do not
+    fit: the solve goes plane by plane, with the same result."""
+    torch = pytest.importorskip("torch")
+    n = DIMS[0] * DIMS[1] * DIMS[2]
+    rho = torch.ones(n, dtype=torch.float64, device="cuda")
+    rho[: n // 3] = 100.0
+    solid = torch.zeros(n, dtype=torch.uint8, device="cuda")
+    b = torch.sin(torch.arange(n, dtype=torch.float64, device="cuda"))
+    out, launches = [], []
+    for left in (None, 200):
+        with engine.Session(*DIMS, 1.0 / 160) as s:
+            s.assemble_pressure(rho, solid)
+            x = torch.zeros(n, dtype=torch.float64, device="cuda")
+            torch.cuda.synchronize()
+            torch.cuda.empty_cache()
+            hold = None
+            if left:
+                hold = torch.empty(torch.cuda.mem_get_info()[0] - (left << 20), dtype=torch.uint8, device="cuda")
+            before = engine.launch_count()
+            engine.GaussSeidel(s).solve(x, b, 1, 2, None, 1e-30, 1e-30)
+            launches.append(engine.launch_count() - before)
+            out.append(x.cpu())
+            del hold
+    assert torch.equal(out[0], out[1])
+    assert launches[0] < 20 < launches[1]
