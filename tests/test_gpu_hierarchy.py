@@ -76,6 +76,53 @@ def test_fp64_solve_does_not_depend_on_a_mixed_one_before(engine, dims):
         assert np.array_equal(solve(engine, E, P, precision=engine.FP64), ref)
 
 
+def relres(oracle, P, x):
+    return np.linalg.norm(oracle.resid(P, x, P.b)) / np.linalg.norm(P.b)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("dims", [
+    (17, 17, 19), (24, 26, 7), (66, 71, 1),                        # padded rows, k and j
+    (64, 65, 2), (48, 50, 5), (60, 61, 9), (5000, 1, 1), (900, 9, 1), (2100, 2, 1)])   # thin
+@pytest.mark.parametrize("convect", [0, 0.02])   # weak: the refinement around the symmetric part converges
+def test_padded_and_thin_grids_converge(engine, oracle, dims, precision, convect):
+    """The solution in the caller's rows: its FP64 residual, formed on the
+    host, with symmetric matrices and, by the residual of the seven arrays,
+    non-symmetric ones."""
+    P = problem(dims, convect, solids=0.1 if min(dims) > 2 else 0.0)   # no pockets on 1-D and 2-D grids
+    x = np.zeros(P.N)
+    with engine.Session(*dims, P.h) as s:
+        s.upload_matrix(P.A)
+        assert s.symmetric() == (convect == 0)
+        E = engine.Engine(s)
+        assert E.solve(x, P.b.copy(), tol=1e-9, precision=precision)
+        assert relres(oracle, P, x) <= 1.0001e-9
+        assert E.last.relres == pytest.approx(relres(oracle, P, x), rel=1e-3, abs=1e-13)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("convect", [0, 0.02])   # weak: the refinement around the symmetric part converges
+@pytest.mark.parametrize("dims", [(17, 17, 19), (66, 71, 1)])
+def test_refresh_of_padded_rows(engine, oracle, dims, convect, precision):
+    """A changed matrix of the same shape, uploaded into the buffers that the
+    hierarchy's padded copy was made from: the bits of a fresh session."""
+    P, Q = problem(dims, convect), problem(dims, convect)
+    for k in "cwesnbt":
+        Q.A[k] = 3.0 * P.A[k]
+    Q.A["c"] = Q.A["c"] + 0.01 * P.A["c"].max()
+    with engine.Session(*dims, P.h) as s:
+        s.upload_matrix(Q.A)
+        ref = solve(engine, engine.Engine(s), Q, precision=precision)
+    with engine.Session(*dims, P.h) as s:
+        s.upload_matrix(P.A)
+        E = engine.Engine(s)
+        solve(engine, E, P, precision=precision)
+        s.upload_matrix(Q.A)
+        x = solve(engine, E, Q, precision=precision)
+    assert np.array_equal(x, ref)
+    assert relres(oracle, Q, x) <= 1.0001e-9
+
+
 def device_bytes(f):
     """Device memory that f() takes and keeps (allocations of the library)."""
     torch = pytest.importorskip("torch")

@@ -11,7 +11,7 @@ DIMS = [(7, 9, 5), (8, 8, 8), (9, 17, 33), (24, 16, 31), (2, 30, 67), (33, 3, 2)
         (1, 20, 33), (19, 1, 33), (1, 1, 44), (3, 5, 33)]
 
 
-def problem(dims, convect):
+def problem(dims, convect, solids=0.1):
     import flow
     g = np.random.default_rng(sum(dims))
     nx, ny, nz = dims
@@ -19,12 +19,12 @@ def problem(dims, convect):
     bc[5 if nz > 1 else 3] = 1
     h = 1.0 / max(dims)
     col = g.random(dims)
-    solid = (g.random(dims) < 0.1).astype(np.uint8)
+    solid = (g.random(dims) < solids).astype(np.uint8)
     A = flow.assemble_mix(dims, h, bc, col, 100.0, 1.0, solid=solid)
     if convect:  # first-order upwind convection along x: a non-symmetric matrix
         ok = (solid[1:] == 0) & (solid[:-1] == 0)
         F = np.zeros(dims)
-        F[1:] = 0.002 * h * ok
+        F[1:] = 0.002 * convect * h * ok
         A["w"] = A["w"] + F.reshape(-1)
         A["c"] = A["c"] + F.reshape(-1)
         A["ci"] = 1.0 / A["c"]
