@@ -276,10 +276,6 @@ struct KnownDiv {
 // the partials in block order and runs the finalize step. No spin waits: the
 // "last block" is found with one atomic counter that the last block resets.
 // ---------------------------------------------------------------------------
-struct RedScratch {
-  double *part;        // [kRedSlots][kMaxBlocks] partial sums
-  unsigned *count;     // [kRedSlots] arrival counters (zero between uses)
-};
 constexpr int kRedVals = 4;   // values reduced by one kernel at most
 
 template <int NV, int First = 16>

@@ -26,7 +26,10 @@ struct LevelOut {
 __global__ void k_level_finish(EMat<double> A, LevelOut o) {
   GRID_LOOP(p, A.g.n) {
     const double c = A.c[p];
-    const double d = c != 0.0 ? 1.0 / c : 0.0;   // a pad cell has no diagonal and stays zero
+    // A pad cell (RowPad) has no diagonal and no couplings: its right-hand side
+    // and A times anything are zero there, so whatever the prolongation leaves
+    // in it reaches neither a dot product nor another cell.
+    const double d = c != 0.0 ? 1.0 / c : 0.0;
     o.d[p] = d;
     if (o.c32) {
       const Pos q = A.g.pos(p);
@@ -209,7 +212,8 @@ constexpr int kCoarseAuto = 1024;
 // depend on which came first), where that adds at most a seventh. Measured
 // there: 7, 14, 22 and 30 cells a row mixed 2 to 7% faster, FP64 from 1.4%
 // slower to even. Above: 10, 13 and 17 cells mixed 2% faster, FP64 3 to 4.5%
-// slower; 5 and 6 cells 3 to 12% slower, and 2 cells 512x512 2.7 -> 3.1 ms.
+// slower; 5 and 6 cells mixed within 3% either way, FP64 12% slower; 2 cells
+// (512x512) mixed 2.7 -> 3.1 ms, FP64 2.7 -> 3.7 ms.
 constexpr int kRowVec = VecTraits<float>::V;
 static int padded_row(int n) {
   const int up = (n + kRowVec - 1) / kRowVec * kRowVec;

@@ -60,16 +60,6 @@ __device__ __forceinline__ T ax_at(const EMat<T> &A, uint32_t p, Pos q, const T 
 // ---------------------------------------------------------------- smoothers
 // Damped Jacobi with the stored inverse diagonal:
 //   x' = x + w (D^-1 (r + sum_nb a_nb x_nb) - x)   (= x + w D^-1 (r - A x))
-
-// x = w D^-1 r   (first sweep from a zero guess)
-template <typename T>
-__global__ void __launch_bounds__(kThreads, 8) k_jac0(EMat<T> A, const T *__restrict__ r, T *__restrict__ x, T omega,
-                       const int *stop) {
-  PBG_PDL_ENTRY();
-  if (stop && *stop) return;
-  GRID_LOOP(p, A.g.n) x[p] = omega * r[p] * A.dinv[p];
-}
-
 template <typename T>
 __global__ void __launch_bounds__(kThreads, 8) k_jac(EMat<T> A, const T *__restrict__ r, const T *__restrict__ xi,
                       T *__restrict__ xo, T omega, const int *stop) {
@@ -271,15 +261,6 @@ __global__ void __launch_bounds__(kThreads, 8) k_kc_q1(EMat<T> A, const T *__res
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kThreads, 8) k_kc_r1(long long N, const T *__restrict__ b, const T *__restrict__ q1,
-                        T *__restrict__ r1, const KScal *ks, const int *stop) {
-  PBG_PDL_ENTRY();
-  if (stop && *stop) return;
-  const T a1 = (T)ks->a1;
-  GRID_LOOP(p, N) r1[p] = b[p] - a1 * q1[p];
-}
-
-template <typename T>
 __global__ void __launch_bounds__(kThreads, 8) k_kc_q2(EMat<T> A, const T *__restrict__ z2, const T *__restrict__ q1,
                         const T *__restrict__ r1, T *__restrict__ vv, KScal *ks, double *part,
                         unsigned *count, const int *stop) {
@@ -306,15 +287,6 @@ __global__ void __launch_bounds__(kThreads, 8) k_kc_q2(EMat<T> A, const T *__res
     ks->beta = beta;
     ks->a2 = a2;
   }
-}
-
-template <typename T>
-__global__ void __launch_bounds__(kThreads, 8) k_kc_x(long long N, const T *__restrict__ z1, const T *__restrict__ z2,
-                       T *__restrict__ x, const KScal *ks, const int *stop) {
-  PBG_PDL_ENTRY();
-  if (stop && *stop) return;
-  const T c1 = (T)(ks->a1 - ks->a2 * ks->beta), c2 = (T)ks->a2;
-  GRID_LOOP(p, N) x[p] = c1 * z1[p] + c2 * z2[p];
 }
 
 // Coarsest level: z = Ainv r with the dense inverse (FP64, or its FP32

@@ -68,16 +68,8 @@ __device__ __forceinline__ double ref_bmax(const MatView<double> &A, long long p
   return v;
 }
 
-// element of Scalar::dot_voldiv_avg: x*y/dV/dV (scalar.h:317-326). Two FP64
-// divisions a cell (125 cycles each) bounded the kernels that form this sum;
-// the corrected products give the same bits.
-__device__ __forceinline__ double voldiv(double x, double y, const KnownDiv &dV) {
-  return dV(dV(__dmul_rn(x, y)));
-}
-
-// res = sqrt(d/N/N)/scale (cg.cpp:68 and :115)
 __device__ __forceinline__ double res_of(double d, const KrylovState *st) {
-  return __ddiv_rn(__dsqrt_rn(__ddiv_rn(__ddiv_rn(d, st->ncell), st->ncell)), st->scale);
+  return res_norm(d, st->ncell, st->scale);
 }
 
 // ---------------------------------------------------------------------------
@@ -179,15 +171,7 @@ __device__ void stale_init_dev(KrylovState *st, double res0) {
 
 // true when stale (cg.cpp:138-160); otherwise rotates the window
 __device__ bool stale_step_dev(KrylovState *st, double res) {
-  int n = st->stalecount > kStaleMax ? kStaleMax : st->stalecount;
-  if (n <= 0) return false;
-  bool stale = true;
-  for (int q = 0; q < n; ++q)
-    if (res < st->stale[q]) { stale = false; break; }
-  if (stale) return true;
-  for (int q = 0; q < n - 1; ++q) st->stale[q] = st->stale[q + 1];
-  st->stale[n - 1] = res;
-  return false;
+  return stale_step(st->stale, stale_entries(st->stalecount), res);
 }
 
 __global__ void k_cg_init(MatView<double> A, const double *__restrict__ x,
@@ -1281,12 +1265,26 @@ static void ic_form(const MatView<double> &A, int kind, RefKrylovWork &w, cudaSt
   note_launch();
 }
 
+// Launch of a kernel that ends in grid_reduce: its form with the exact-order
+// code, or the one without, which keeps its occupancy.
+struct SumLaunch {
+  bool exact;
+  int grid;
+  cudaStream_t s;
+  template <typename... P, typename... A>
+  void operator()(void (*seq)(P...), void (*tree)(P...), A... a) const {
+    (exact ? seq : tree)<<<grid, kThreads, 0, s>>>(a...);
+    note_launch();
+  }
+};
+
 void enqueue_ref_setup(const MatView<double> &A, double *x, const double *b, const KrylovParams &pr,
                        int solver, RefKrylovWork &w, const RedPool &red, KrylovState *st,
                        cudaStream_t s) {
   const long long N = A.ncell();
-  const bool exact = pr.seq != nullptr;   // kernels without the exact-order code keep their occupancy
+  const bool exact = pr.seq != nullptr;
   const int g = exact ? grid_exact(N) : grid_for(N);
+  const SumLaunch sum{exact, g, s};
   w.ensure((size_t)N, solver);
   k_krylov_setup<<<1, 1, 0, s>>>(st, pr, N); note_launch();
   if (solver >= 3) {  // Jacobi, Gauss-Seidel: ci as stored with the matrix, else 1/c
@@ -1302,8 +1300,8 @@ void enqueue_ref_setup(const MatView<double> &A, double *x, const double *b, con
       k_gs_pack<<<grid_for((long long)sg.all_rows() * sg.cols), kThreads, 0, s>>>(sg, A, w.ci, b, x,
                                                                                  w.march(sg, kGsPlanes)); note_launch();
     }
-    (exact ? k_it_init<true> : k_it_init<false>)<<<g, kThreads, 0, s>>>(A, x, b, w.r.p, st, red.slot_part(0), red.slot_count(0),
-                                     solver == 4 ? 1 : 0); note_launch();
+    sum(k_it_init<true>, k_it_init<false>, A, x, b, w.r.p, st, red.slot_part(0), red.slot_count(0),
+        solver == 4 ? 1 : 0);
     PBG_CUDA(cudaGetLastError());
     return;
   }
@@ -1322,11 +1320,11 @@ void enqueue_ref_setup(const MatView<double> &A, double *x, const double *b, con
     ic_form(A, pr.prec, w, s);
   }
   k_recip<<<grid_for(N), kThreads, 0, s>>>(N, A.c, w.mcd.p); note_launch();
-  if (solver == 0)
-    k_cg_init<<<g, kThreads, 0, s>>>(A, x, b, w.r.p, st, red.slot_part(0), red.slot_count(0), w.mcd.p);
-  else
-    (exact ? k_bi_init<true> : k_bi_init<false>)<<<g, kThreads, 0, s>>>(A, x, b, w.r.p, w.rt.p, st, red.slot_part(0), red.slot_count(0));
-  note_launch();
+  if (solver == 0) {
+    k_cg_init<<<g, kThreads, 0, s>>>(A, x, b, w.r.p, st, red.slot_part(0), red.slot_count(0), w.mcd.p); note_launch();
+  } else {
+    sum(k_bi_init<true>, k_bi_init<false>, A, x, b, w.r.p, w.rt.p, st, red.slot_part(0), red.slot_count(0));
+  }
   PBG_CUDA(cudaGetLastError());
 }
 
@@ -1356,6 +1354,7 @@ void enqueue_ref_iters(const MatView<double> &A, double *x, int solver, int coun
                        cudaStream_t s, bool exact, int prec) {
   const long long N = A.ncell();
   const int g = exact ? grid_exact(N) : grid_for(N);
+  const SumLaunch sum{exact, g, s};
   double *P0 = red.slot_part(0), *P1 = red.slot_part(1);
   unsigned *C0 = red.slot_count(0), *C1 = red.slot_count(1);
   const int diag = prec > 0 ? 0 : 1;
@@ -1378,7 +1377,7 @@ void enqueue_ref_iters(const MatView<double> &A, double *x, int solver, int coun
       } else {
         k_jacobi_x<<<grid_for(N), kThreads, 0, s>>>(N, A.c, w.ci, w.r.p, x, st); note_launch();
       }
-      (exact ? k_it_resid<true> : k_it_resid<false>)<<<g, kThreads, 0, s>>>(A, x, w.rhs, w.r.p, st, hist, P0, C0, gs); note_launch();
+      sum(k_it_resid<true>, k_it_resid<false>, A, x, w.rhs, w.r.p, st, hist, P0, C0, gs);
     }
     PBG_CUDA(cudaGetLastError());
     return;
@@ -1387,7 +1386,7 @@ void enqueue_ref_iters(const MatView<double> &A, double *x, int solver, int coun
     if (solver == 0 && prec > 0) {
       // z = M^-1 r (forward and backward sweeps), rho = r.z, then the CG step
       ic_apply(A, prec, w, w.r.p, w.z.p, st, s);
-      (exact ? k_cg_rho<true> : k_cg_rho<false>)<<<g, kThreads, 0, s>>>(N, w.r.p, w.z.p, st, P0, C0); note_launch();
+      sum(k_cg_rho<true>, k_cg_rho<false>, N, w.r.p, w.z.p, st, P0, C0);
       k_cg_pq<<<g, kThreads, 0, s>>>(A, w.r.p, w.pA.p, w.pB.p, w.q.p, st, P0, C0, w.z.p, w.mcd.p); note_launch();
       k_cg_xr<<<g, kThreads, 0, s>>>(N, w.mcd.p, x, w.r.p, w.pA.p, w.pB.p, w.q.p, st, hist, P1, C1, 1); note_launch();
     } else if (solver == 0 && !exact && A.nz % 2 == 0 && !A.per) {
@@ -1403,22 +1402,22 @@ void enqueue_ref_iters(const MatView<double> &A, double *x, int solver, int coun
       k_cg_pq<<<g, kThreads, 0, s>>>(A, w.r.p, w.pA.p, w.pB.p, w.q.p, st, P0, C0, nullptr, w.mcd.p); note_launch();
       k_cg_xr<<<g, kThreads, 0, s>>>(N, w.mcd.p, x, w.r.p, w.pA.p, w.pB.p, w.q.p, st, hist, P1, C1, 0); note_launch();
     } else if (solver == 1) {
-      (exact ? k_bi_rho<true> : k_bi_rho<false>)<<<g, kThreads, 0, s>>>(N, w.rt.p, w.r.p, st, P0, C0); note_launch();
+      sum(k_bi_rho<true>, k_bi_rho<false>, N, w.rt.p, w.r.p, st, P0, C0);
       k_bi_p<<<g, kThreads, 0, s>>>(N, w.mcd.p, w.r.p, w.pA.p, w.v.p, w.ph.p, st, diag); note_launch();
       if (!diag) ic_apply(A, prec, w, w.pA.p, w.ph.p, st, s);
-      (exact ? k_bi_spmv<true> : k_bi_spmv<false>)<<<g, kThreads, 0, s>>>(A, w.ph.p, w.v.p, w.rt.p, 0, st, P1, C1); note_launch();
-      (exact ? k_bi_s<true> : k_bi_s<false>)<<<g, kThreads, 0, s>>>(N, w.mcd.p, w.r.p, w.v.p, w.s.p, w.sh.p, st, P0, C0, diag); note_launch();
+      sum(k_bi_spmv<true>, k_bi_spmv<false>, A, w.ph.p, w.v.p, w.rt.p, 0, st, P1, C1);
+      sum(k_bi_s<true>, k_bi_s<false>, N, w.mcd.p, w.r.p, w.v.p, w.s.p, w.sh.p, st, P0, C0, diag);
       if (!diag) ic_apply(A, prec, w, w.s.p, w.sh.p, st, s);
-      (exact ? k_bi_spmv<true> : k_bi_spmv<false>)<<<g, kThreads, 0, s>>>(A, w.sh.p, w.t.p, w.s.p, 1, st, P1, C1); note_launch();
-      (exact ? k_bi_xr<true> : k_bi_xr<false>)<<<g, kThreads, 0, s>>>(N, x, w.r.p, w.ph.p, w.sh.p, w.s.p, w.t.p, st, hist, P0, C0); note_launch();
+      sum(k_bi_spmv<true>, k_bi_spmv<false>, A, w.sh.p, w.t.p, w.s.p, 1, st, P1, C1);
+      sum(k_bi_xr<true>, k_bi_xr<false>, N, x, w.r.p, w.ph.p, w.sh.p, w.s.p, w.t.p, st, hist, P0, C0);
     } else {
-      (exact ? k_cgs_rho<true> : k_cgs_rho<false>)<<<g, kThreads, 0, s>>>(N, w.rt.p, w.r.p, st, P0, C0); note_launch();
+      sum(k_cgs_rho<true>, k_cgs_rho<false>, N, w.rt.p, w.r.p, st, P0, C0);
       k_cgs_up<<<g, kThreads, 0, s>>>(N, w.mcd.p, w.r.p, w.q.p, w.u.p, w.pA.p, w.ph.p, st, diag); note_launch();
       if (!diag) ic_apply(A, prec, w, w.pA.p, w.ph.p, st, s);
-      (exact ? k_bi_spmv<true> : k_bi_spmv<false>)<<<g, kThreads, 0, s>>>(A, w.ph.p, w.v.p, w.rt.p, 0, st, P1, C1); note_launch();
+      sum(k_bi_spmv<true>, k_bi_spmv<false>, A, w.ph.p, w.v.p, w.rt.p, 0, st, P1, C1);
       k_cgs_qs<<<g, kThreads, 0, s>>>(N, w.mcd.p, w.u.p, w.v.p, w.q.p, w.s.p, w.sh.p, st, diag); note_launch();
       if (!diag) ic_apply(A, prec, w, w.s.p, w.sh.p, st, s);
-      (exact ? k_cgs_xr<true> : k_cgs_xr<false>)<<<g, kThreads, 0, s>>>(A, x, w.r.p, w.sh.p, st, hist, P0, C0); note_launch();
+      sum(k_cgs_xr<true>, k_cgs_xr<false>, A, x, w.r.p, w.sh.p, st, hist, P0, C0);
     }
   }
   PBG_CUDA(cudaGetLastError());

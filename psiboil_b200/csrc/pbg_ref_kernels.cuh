@@ -10,6 +10,32 @@
 
 namespace pbg {
 
+// element of Scalar::dot_voldiv_avg: x*y/dV/dV (scalar.h:317-326). Two FP64
+// divisions a cell (125 cycles each) bounded the kernels that form this sum;
+// the corrected products give the same bits.
+__device__ __forceinline__ double voldiv(double x, double y, const KnownDiv &dV) {
+  return dV(dV(__dmul_rn(x, y)));
+}
+
+// res = sqrt(d/N/N)/scale (cg.cpp:68 and :115)
+__device__ __forceinline__ double res_norm(double d, double ncell, double scale) {
+  return __ddiv_rn(__dsqrt_rn(__ddiv_rn(__ddiv_rn(d, ncell), ncell)), scale);
+}
+
+// The staleness window of n residuals (cg.cpp:138-160): true if res is below
+// none of them, else res takes the place of the oldest.
+__device__ __forceinline__ int stale_entries(int stalecount) { return stalecount > kStaleMax ? kStaleMax : stalecount; }
+__device__ __forceinline__ bool stale_step(double *win, int n, double res) {
+  if (n <= 0) return false;
+  bool stale = true;
+  for (int q = 0; q < n; ++q)
+    if (res < win[q]) { stale = false; break; }
+  if (stale) return true;
+  for (int q = 0; q < n - 1; ++q) win[q] = win[q + 1];
+  win[n - 1] = res;
+  return false;
+}
+
 // IC3 factor (compact arrays), run one launch per plane h = 5 i + 2 j + k.
 // The other sweeps (IC0, IC2, Gauss-Seidel) are in pbg_sweeps.cuh.
 struct Ic3Factor {

@@ -94,9 +94,8 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_cg_small(MatView<double> A
   const int first = rank * m;
   double *cf = sh, *ps = sh + 7 * (size_t)kSmallCells;
   const KnownDiv dV(pr.dV);
-  auto voldiv = [&](double a) { return dV(dV(a)); };
   const double nc = (double)N;
-  auto res_of = [&](double d) { return __ddiv_rn(__dsqrt_rn(__ddiv_rn(__ddiv_rn(d, nc), nc)), pr.scale); };
+  auto res_of = [&](double d) { return res_norm(d, nc, pr.scale); };
 
   // own cells: e = threadIdx + 512 u; neighbours' p by their address in the
   // cluster's shared memory
@@ -140,7 +139,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_cg_small(MatView<double> A
       t = __dadd_rn(t, __dadd_rn(__dmul_rn(a.b, xs[4]), __dmul_rn(a.t, xs[5])));
       r[u] = t;
       mc[u] = __ddiv_rn(1.0, c);
-      v2[0] += voldiv(__dmul_rn(t, t));
+      v2[0] += voldiv(t, t, dV);
       v2[1] += __dmul_rn(t, __dmul_rn(t, mc[u]));
     }
   }
@@ -149,7 +148,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_cg_small(MatView<double> A
   const double res0 = res_of(v2[0]);
   double res = res0, rho = v2[1], rho_old = 0.0, alfa = 0.0, beta = 0.0, pq = 0.0;
   int iterations = 0, it = 0, status = ST_RUNNING, converged = 0;
-  const int ns = pr.stalecount > kStaleMax ? kStaleMax : pr.stalecount;
+  const int ns = stale_entries(pr.stalecount);
   if (threadIdx.x == 0 && ns > 0) {
     for (int q = 0; q < ns; ++q) stale[q] = 1.0e24;   // boil::unreal
     stale[ns - 1] = res0;
@@ -189,7 +188,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_cg_small(MatView<double> A
       xv[u] = __dadd_rn(xv[u], __dmul_rn(alfa, p[u]));
       r[u] = __dsub_rn(r[u], __dmul_rn(alfa, q[u]));
       if (first + threadIdx.x + kSmallThreads * u < N && threadIdx.x + kSmallThreads * u < m) {
-        v2[0] += voldiv(__dmul_rn(r[u], r[u]));
+        v2[0] += voldiv(r[u], r[u], dV);
         v2[1] += __dmul_rn(r[u], __dmul_rn(r[u], mc[u]));
       }
     }
@@ -203,14 +202,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_cg_small(MatView<double> A
       break;
     }
     if (ns > 0) {   // the staleness window (cg.cpp:138-160), the same in every block
-      if (threadIdx.x == 0) {
-        bool all = true;
-        for (int w = 0; w < ns; ++w)
-          if (res < stale[w]) { all = false; break; }
-        stop_flag = all ? 1 : 0;
-        for (int w = 0; !all && w < ns - 1; ++w) stale[w] = stale[w + 1];
-        if (!all) stale[ns - 1] = res;
-      }
+      if (threadIdx.x == 0) stop_flag = stale_step(stale, ns, res);
       __syncthreads();
       if (stop_flag) { status = ST_STALE; break; }
     }
