@@ -109,7 +109,8 @@ __global__ void k_dense_dmax(int n, const double *__restrict__ D, double *dmax) 
 
 constexpr int kGjB = 32;     // pivots per block step
 constexpr int kGjRows = 32;  // rows per CTA
-constexpr int kGjCols = 128; // columns per CTA, two threads a column
+constexpr int kGjCols = 128; // columns per CTA at a time, two threads a column
+constexpr int kGjGrid = 296; // CTAs at most: one wave, two an SM
 
 // One blocked Gauss-Jordan exchange on the pivots k0 .. k0+kb-1 (out of
 // place, A -> B). With A11 the pivot block, G = A11^-1 (by scalar
@@ -121,10 +122,13 @@ constexpr int kGjCols = 128; // columns per CTA, two threads a column
 // zero, which gives a generalised inverse of a consistent singular system
 // (in a positive semi-definite matrix a zero Schur pivot has a zero row
 // and column, so nothing else changes).
-// A step is bound by its pivot block (32 dependent exchanges with a barrier
-// pair each) and its launch; a CTA of 32 rows x 128 columns keeps the rest,
-// 128 multiply-adds a thread per pivot, below that. 32 rows x all columns
-// took 67 us a step at n = 512, this form 12.
+// A small step is bound by its pivot block (32 dependent exchanges with a
+// barrier pair each), which every CTA forms; the columns of its 32 rows are
+// shared out over CTAs as far as one wave of them goes, and a CTA takes the
+// rest 128 at a time. Whole set-up per step of 32 pivots, with 32 rows and all
+// columns a CTA / 32 x 128 a CTA / this form: n = 512 51 / 31 / 26 us, n = 1872
+// 103 / 73 / 43 us, n = 4096 331 / 335 / 189 us. Two waves of CTAs took 206 us
+// at n = 4096, half a wave 326.
 __global__ void __launch_bounds__(256) k_gj_block(int n, int k0, const double *__restrict__ A,
                                                   double *__restrict__ B, const double *dmax,
                                                   double rel_tol) {
@@ -176,29 +180,28 @@ __global__ void __launch_bounds__(256) k_gj_block(int n, int k0, const double *_
     U[ii][l] = u;
   }
   __syncthreads();
-  const int j = blockIdx.y * kGjCols + threadIdx.x % kGjCols;
   const int half = threadIdx.x / kGjCols * (kGjRows / 2);
-  if (j >= n) return;
-  const bool jin = j >= k0 && j < k0 + kb;
-  double a[kGjB];
+  for (int j = blockIdx.y * kGjCols + threadIdx.x % kGjCols; j < n; j += gridDim.y * kGjCols) {
+    const bool jin = j >= k0 && j < k0 + kb;
+    double a[kGjB];
 #pragma unroll
-  for (int l = 0; l < kGjB; ++l) a[l] = (!jin && l < kb) ? A[(size_t)(k0 + l) * n + j] : 0.0;
-  for (int ii = half; ii < half + kGjRows / 2; ++ii) {
-    const int i = i0 + ii;
-    if (i >= n) break;
-    const bool iin = i >= k0 && i < k0 + kb;
-    double v;
-    if (jin) v = iin ? U[ii][j - k0] : -U[ii][j - k0];
-    else {
-      double acc = 0.0;
+    for (int l = 0; l < kGjB; ++l) a[l] = (!jin && l < kb) ? A[(size_t)(k0 + l) * n + j] : 0.0;
+    for (int ii = half; ii < half + kGjRows / 2; ++ii) {
+      const int i = i0 + ii;
+      if (i >= n) break;
+      const bool iin = i >= k0 && i < k0 + kb;
+      double v;
+      if (jin) v = iin ? U[ii][j - k0] : -U[ii][j - k0];
+      else {
+        double acc = 0.0;
 #pragma unroll
-      for (int l = 0; l < kGjB; ++l) acc += U[ii][l] * a[l];
-      v = iin ? acc : A[(size_t)i * n + j] - acc;
+        for (int l = 0; l < kGjB; ++l) acc += U[ii][l] * a[l];
+        v = iin ? acc : A[(size_t)i * n + j] - acc;
+      }
+      B[(size_t)i * n + j] = v;
     }
-    B[(size_t)i * n + j] = v;
   }
 }
-
 
 // Grids whose rows are padded: below kPadMin the passes are bound by their
 // chains of loads whatever the rows, and the pad cells would be a larger
@@ -495,7 +498,8 @@ void Engine::compute(cudaStream_t s) {
   k_dense_fill<<<grid_for(n), kThreads, 0, s>>>(L.back().m64, Dtmp.p); note_launch();
   k_dense_dmax<<<1, 1024, 0, s>>>(n, Dtmp.p, dsc.p + 7); note_launch();
   double *src = Dtmp.p, *dst = Ainv.p;
-  const dim3 tiles((n + kGjRows - 1) / kGjRows, (n + kGjCols - 1) / kGjCols);
+  const int gjr = (n + kGjRows - 1) / kGjRows, gjc = (n + kGjCols - 1) / kGjCols;
+  const dim3 tiles(gjr, std::min(gjc, std::max(1, kGjGrid / gjr)));
   for (int k0 = 0; k0 < n; k0 += kGjB) {
     k_gj_block<<<tiles, 256, 0, s>>>(n, k0, src, dst, dsc.p + 7, 1e-10); note_launch();
     std::swap(src, dst);

@@ -123,6 +123,23 @@ def test_refresh_of_padded_rows(engine, oracle, dims, convect, precision):
     assert relres(oracle, Q, x) <= 1.0001e-9
 
 
+@pytest.mark.parametrize("dims", [(1, 1, 31), (3, 11, 1), (1, 1, 127), (43, 3, 1), (8, 9, 10), (10, 11, 10), (11, 12, 16),
+                                  (15, 16, 17)])
+def test_dense_inverse_of_the_whole_grid(engine, oracle, dims):
+    """A grid that is its own coarsest level (31 to 4080 cells: block steps of
+    32 pivots and column tiles of 128 with remainders, CTAs with one and with
+    several column tiles): the dense inverse solves it in one FCG iteration,
+    two where rounding leaves the first above the tolerance."""
+    P = problem(dims, False, solids=0.0)
+    x = np.zeros(P.N)
+    with engine.Session(*dims, P.h) as s:
+        s.upload_matrix(P.A)
+        E = engine.Engine(s)
+        assert E.solve(x, P.b.copy(), tol=1e-10, precision=engine.FP64, coarse_max=4096)
+        assert s.levels(1) == [dims] and E.last.iterations <= 2
+    assert relres(oracle, P, x) <= 1.0001e-10
+
+
 def device_bytes(f):
     """Device memory that f() takes and keeps (allocations of the library)."""
     torch = pytest.importorskip("torch")
