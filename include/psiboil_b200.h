@@ -125,9 +125,9 @@ typedef struct {
   int exact_sums;
   /* engine: cells of the dense coarsest level at most, until a later call
    * names another size; 0: as an earlier call on this session chose, else the
-   * first level of at most 1024. Larger (4096) saves launches in repeated
-   * solves with one matrix and costs a longer set-up after every matrix change
-   * (a dense inverse, O(cells^3)). */
+   * first level of at most 1024 (768 on the two finest levels). Larger (4096)
+   * saves launches in repeated solves with one matrix and costs a longer set-up
+   * after every matrix change (a dense inverse, O(cells^3)). */
   int coarse_max;
   /* Krylov preconditioner (CG, BiCGS, CGS), the reference's Prec codes
    * (preconditioner.h:15-29): 0 diagonal (Prec::di, default), 1 IC0, 2 IC2,

@@ -122,62 +122,86 @@ constexpr int kGjGrid = 296; // CTAs at most: one wave, two an SM
 // zero, which gives a generalised inverse of a consistent singular system
 // (in a positive semi-definite matrix a zero Schur pivot has a zero row
 // and column, so nothing else changes).
-// A small step is bound by its pivot block (32 dependent exchanges with a
-// barrier pair each), which every CTA forms; the columns of its 32 rows are
-// shared out over CTAs as far as one wave of them goes, and a CTA takes the
-// rest 128 at a time. Whole set-up per step of 32 pivots, with 32 rows and all
-// columns a CTA / 32 x 128 a CTA / this form: n = 512 51 / 31 / 26 us, n = 1872
-// 103 / 73 / 43 us, n = 4096 331 / 335 / 189 us. Two waves of CTAs took 206 us
-// at n = 4096, half a wave 326.
-__global__ void __launch_bounds__(256) k_gj_block(int n, int k0, const double *__restrict__ A,
-                                                  double *__restrict__ B, const double *dmax,
-                                                  double rel_tol) {
+// Every CTA forms G, so a small step is bound by it: 32 dependent exchanges,
+// each a barrier, a shared load, a division and two multiply-adds. A thread
+// holds four entries (row w + 8 u, column lane): the pivot column comes by
+// shuffle, the pivot row from shared memory in two buffers by turns, which
+// makes one barrier do (8 us a step where two barriers and a round trip of
+// every entry through shared memory took 21). The columns of a CTA's 32 rows
+// are shared out over CTAs as far as one wave of them goes, and a CTA takes
+// the rest 128 at a time; a thread loads eight rows' entries before their
+// sums, as the loads' latency bounds large steps. Time per step of 32 pivots:
+//   n                                          512   720  1000  1872  4096
+//   32 rows x 128 columns a CTA, one a column tile
+//                                               31    30    34    73   335 us
+//   one wave of CTAs                            24    24    28    43   187 us
+//   and G in registers, loads in eights         15    14    18    32   121 us
+__global__ void __launch_bounds__(256, 2) k_gj_block(int n, int k0, const double *__restrict__ A,
+                                                     double *__restrict__ B, const double *dmax,
+                                                     double rel_tol) {
+  constexpr int GR = kGjB / 8, AHEAD = 8;
   __shared__ double G[kGjB][kGjB + 1];
-  __shared__ double U[kGjRows][kGjB + 1];
-  __shared__ double S[kGjRows][kGjB + 1];
-  __shared__ double rowk[kGjB], colk[kGjB];
+  __shared__ __align__(16) double U[kGjRows][kGjB + 2];
+  __shared__ __align__(16) double S[kGjRows][kGjB + 2];
+  __shared__ double rowb[2][kGjB];
   const int kb = min(kGjB, n - k0);
   const double thr = rel_tol * (*dmax);
-  for (int e = threadIdx.x; e < kGjB * kGjB; e += blockDim.x) {
-    const int r = e / kGjB, c = e % kGjB;
-    G[r][c] = (r < kb && c < kb) ? A[(size_t)(k0 + r) * n + k0 + c] : 0.0;
-  }
-  __syncthreads();
-  for (int k = 0; k < kb; ++k) {
-    if (threadIdx.x < kGjB) { rowk[threadIdx.x] = G[k][threadIdx.x]; colk[threadIdx.x] = G[threadIdx.x][k]; }
-    __syncthreads();
-    const double akk = rowk[k];
-    const bool sk = !(akk > thr);
-    const double piv = sk ? 0.0 : 1.0 / akk;
-#pragma unroll
-    for (int u = 0; u < kGjB * kGjB / 256; ++u) {
-      const int e = threadIdx.x + 256 * u, i = e / kGjB, j = e % kGjB;
-      double v;
-      if (sk) v = (i == k || j == k) ? 0.0 : G[i][j];
-      else if (i == k && j == k) v = piv;
-      else if (i == k) v = rowk[j] * piv;
-      else if (j == k) v = -colk[i] * piv;
-      else v = G[i][j] - colk[i] * rowk[j] * piv;
-      if (i < kb && j < kb) G[i][j] = v;
-    }
-    __syncthreads();
-  }
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int i0 = blockIdx.x * kGjRows;
-  // U: the row coefficients on the pivot rows; S: the rows' pivot-column entries
-  for (int e = threadIdx.x; e < kGjRows * kGjB; e += 256) {
-    const int ii = e / kGjB, l = e % kGjB, i = i0 + ii;
-    S[ii][l] = (i < n && l < kb) ? A[(size_t)i * n + k0 + l] : 0.0;
+  double g[GR];
+#pragma unroll
+  for (int u = 0; u < GR; ++u) {
+    const int i = w + 8 * u;
+    g[u] = i < kb && lane < kb ? A[(size_t)(k0 + i) * n + k0 + lane] : 0.0;
+    S[i][lane] = i0 + i < n && lane < kb ? A[(size_t)(i0 + i) * n + k0 + lane] : 0.0;   // the rows' pivot-column entries
   }
+  if (w == 0) rowb[0][lane] = g[0];
   __syncthreads();
-  for (int e = threadIdx.x; e < kGjRows * kGjB; e += 256) {
-    const int ii = e / kGjB, l = e % kGjB, i = i0 + ii;
-    double u = 0.0;
-    if (i < n && l < kb) {
-      if (i >= k0 && i < k0 + kb) u = G[i - k0][l];
-      else
-        for (int m = 0; m < kb; ++m) u += S[ii][m] * G[m][l];
+#pragma unroll
+  for (int ku = 0; ku < GR; ++ku)
+    for (int kw = 0; kw < 8; ++kw) {
+      const int k = 8 * ku + kw;
+      if (k >= kb) break;
+      const double rk = rowb[k & 1][lane], akk = rowb[k & 1][k];
+      const bool sk = !(akk > thr);
+      const double piv = sk ? 0.0 : 1.0 / akk;
+#pragma unroll
+      for (int u = 0; u < GR; ++u) {
+        const double c = __shfl_sync(0xffffffffu, g[u], k);
+        const bool ik = u == ku && w == kw, jk = lane == k;
+        double v;
+        if (sk) v = ik || jk ? 0.0 : g[u];
+        else if (ik) v = jk ? piv : rk * piv;
+        else v = jk ? -c * piv : g[u] - c * rk * piv;
+        g[u] = v;
+      }
+      // the row of pivot k + 1, into the buffer that step k - 1 read
+      if (kw < 7) {
+        if (w == kw + 1) rowb[(k + 1) & 1][lane] = g[ku];
+      } else if (ku + 1 < GR && w == 0) {
+        rowb[(k + 1) & 1][lane] = g[ku + 1 < GR ? ku + 1 : 0];
+      }
+      __syncthreads();
     }
-    U[ii][l] = u;
+#pragma unroll
+  for (int u = 0; u < GR; ++u) G[w + 8 * u][lane] = g[u];
+  __syncthreads();
+  // U: the row coefficients on the pivot rows
+  double acc[GR] = {};
+#pragma unroll 4
+  for (int m = 0; m < kGjB; m += 2) {
+    const double g0 = G[m][lane], g1 = G[m + 1][lane];
+#pragma unroll
+    for (int u = 0; u < GR; ++u) {
+      const double2 sv = *reinterpret_cast<const double2 *>(&S[w + 8 * u][m]);
+      acc[u] += sv.x * g0;
+      acc[u] += sv.y * g1;
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < GR; ++u) {
+    const int i = i0 + w + 8 * u;
+    U[w + 8 * u][lane] = i >= k0 && i < k0 + kb ? G[i - k0][lane] : acc[u];
   }
   __syncthreads();
   const int half = threadIdx.x / kGjCols * (kGjRows / 2);
@@ -185,20 +209,33 @@ __global__ void __launch_bounds__(256) k_gj_block(int n, int k0, const double *_
     const bool jin = j >= k0 && j < k0 + kb;
     double a[kGjB];
 #pragma unroll
-    for (int l = 0; l < kGjB; ++l) a[l] = (!jin && l < kb) ? A[(size_t)(k0 + l) * n + j] : 0.0;
-    for (int ii = half; ii < half + kGjRows / 2; ++ii) {
-      const int i = i0 + ii;
-      if (i >= n) break;
-      const bool iin = i >= k0 && i < k0 + kb;
-      double v;
-      if (jin) v = iin ? U[ii][j - k0] : -U[ii][j - k0];
-      else {
-        double acc = 0.0;
+    for (int l = 0; l < kGjB; ++l) a[l] = !jin && l < kb ? A[(size_t)(k0 + l) * n + j] : 0.0;
+    for (int r0 = half; r0 < half + kGjRows / 2; r0 += AHEAD) {
+      double o[AHEAD];
 #pragma unroll
-        for (int l = 0; l < kGjB; ++l) acc += U[ii][l] * a[l];
-        v = iin ? acc : A[(size_t)i * n + j] - acc;
+      for (int r = 0; r < AHEAD; ++r) {
+        const int i = i0 + r0 + r;
+        o[r] = i < n && !jin && !(i >= k0 && i < k0 + kb) ? A[(size_t)i * n + j] : 0.0;
       }
-      B[(size_t)i * n + j] = v;
+#pragma unroll
+      for (int r = 0; r < AHEAD; ++r) {
+        const int ii = r0 + r, i = i0 + ii;
+        if (i >= n) continue;
+        const bool iin = i >= k0 && i < k0 + kb;
+        double v;
+        if (jin) v = iin ? U[ii][j - k0] : -U[ii][j - k0];
+        else {
+          double sum = 0.0;
+#pragma unroll
+          for (int l = 0; l < kGjB; l += 2) {
+            const double2 q = *reinterpret_cast<const double2 *>(&U[ii][l]);
+            sum += q.x * a[l];
+            sum += q.y * a[l + 1];
+          }
+          v = iin ? sum : o[r] - sum;
+        }
+        B[(size_t)i * n + j] = v;
+      }
     }
   }
 }
@@ -208,7 +245,18 @@ __global__ void __launch_bounds__(256) k_gj_block(int n, int k0, const double *_
 // share of the level; above kPadMax the copy of the operator (32 bytes a
 // cell) could cost a grid its place in device memory.
 constexpr long long kPadMin = 4096, kPadMax = 1ll << 28;
-constexpr int kCoarseAuto = 1024;
+// Cells of the coarsest level at most, unless the caller has chosen: a level
+// of 513 to 1024 cells is inverted rather than coarsened once more. It is
+// visited 2^(l-1) times an iteration, so the deeper it lies the more the inverse
+// saves, while its set-up (15 to 20 us for each 32 cells) is paid once for a
+// matrix. Measured against coarsening on, ms of a solve on a known matrix / of a
+// step with a new one: level 1 of 720 cells 1.24 -> 0.80 / 0.90 -> 1.10; of 1000
+// cells 0.99 -> 0.67 / 0.87 -> 1.25; level 2 of 1000 cells 1.83 -> 1.08 / 1.46 ->
+// 1.59; level 3 of 1000 cells 6.0 -> 3.7 / 3.2 -> 2.7; level 4 of 1000 cells 14.1
+// -> 10.1 / 8.1 -> 6.4. So levels 0 and 1 end at 768 cells, where a step with a
+// new matrix takes no longer than it did with an end at 512 and the cycle's former
+// weights.
+constexpr int kCoarseAuto = 1024, kCoarseAutoTop = 768;
 
 // Stored cells of a row of n: whole FP32 vectors in both precisions (a
 // hierarchy serves mixed and FP64 solves, and an FP64 solve's bits do not
@@ -318,8 +366,8 @@ Engine::~Engine() {
 
 template <> EMat<double> Engine::mat<double>(int l) const { return L[l].m64; }
 template <> EMat<float> Engine::mat<float>(int l) const { return L[l].m32; }
-template <> const void *Engine::ainv<double>() const { return Ainv.p; }
-template <> const void *Engine::ainv<float>() const { return Ainv32.p; }
+template <> const void *Engine::ainv<double>() const { return Ainv; }
+template <> const void *Engine::ainv<float>() const { return Ainv32; }
 
 // Row-scaled FP16 copy of the dense inverse: row i is stored as a / s_i with
 // s_i = max_j |a_ij|, so every entry lies in [-1, 1] (one warp per row).
@@ -420,14 +468,13 @@ void Engine::build(const EMat<double> &A0_, cudaStream_t s, bool mixed) {
       l0.m64 = make_emat<double>(A0.nx, A0.ny, A0.nz, A0.c, A0.w, A0.s, A0.b, l0.d64.p);
     }
   }
-  // Unless the caller has chosen a size, the coarsest level is the first of at
-  // most kCoarseAuto cells: a level of 513 to 1024 cells is inverted rather
-  // than coarsened once more, whose visits (two of a level of 65 to 128 cells
-  // for each of its own) cost more than the larger inverse.
-  const long long dense = opt.coarse_auto ? std::max(opt.coarse_max, kCoarseAuto) : opt.coarse_max;
+  auto dense = [this] {
+    if (!opt.coarse_auto) return (long long)opt.coarse_max;
+    return (long long)std::max(opt.coarse_max, L.size() <= 2 ? kCoarseAutoTop : kCoarseAuto);
+  };
   // Cells of the grid count, not pad cells: padding adds no level.
   auto half = [](int n) { return (n + 1) / 2; };
-  while (L.back().grid.ncell() > dense) {
+  while (L.back().grid.ncell() > dense()) {
     const ELevel &f = L.back();
     ELevel c;
     c.grid = {half(f.grid.nx), half(f.grid.ny), half(f.grid.nz)};
@@ -441,15 +488,19 @@ void Engine::build(const EMat<double> &A0_, cudaStream_t s, bool mixed) {
     L.push_back(std::move(c));
   }
   ncoarse = (int)L.back().ncell();
-  Ainv.alloc((size_t)ncoarse * ncoarse);
-  if (mixed) Ainv32.alloc((size_t)ncoarse * ncoarse);
+  // one allocation for the inverse and what it is formed in: each of a
+  // megabyte or more costs about 0.4 ms of a first solve
+  const size_t nn = (size_t)ncoarse * ncoarse;
+  dense_mem.fit(2 * nn + (mixed ? (nn + 1) / 2 : 0));
+  Ainv = dense_mem.p;
+  Dtmp = Ainv + nn;
+  Ainv32 = mixed ? reinterpret_cast<float *>(Dtmp + nn) : nullptr;
   Ainv16.release();
   Ainv16s.release();
   if (mixed && dense_half_enabled() && ncoarse >= kDenseHalfMin && ncoarse % 8 == 0) {
     Ainv16.alloc((size_t)ncoarse * ncoarse);
     Ainv16s.alloc((size_t)ncoarse);
   }
-  Dtmp.alloc((size_t)ncoarse * ncoarse);
   have32 = false;
   if (mixed) {
     for (auto &lv : L) {
@@ -494,23 +545,22 @@ void Engine::compute(cudaStream_t s) {
   // dense inverse of the coarsest operator: blocked Gauss-Jordan, out of place
   const int n = ncoarse;
   const size_t nn = (size_t)n * n;
-  PBG_CUDA(cudaMemsetAsync(Dtmp.p, 0, nn * sizeof(double), s));
-  k_dense_fill<<<grid_for(n), kThreads, 0, s>>>(L.back().m64, Dtmp.p); note_launch();
-  k_dense_dmax<<<1, 1024, 0, s>>>(n, Dtmp.p, dsc.p + 7); note_launch();
-  double *src = Dtmp.p, *dst = Ainv.p;
+  double *src = Dtmp, *dst = Ainv;
+  if ((n + kGjB - 1) / kGjB % 2 == 0) std::swap(src, dst);   // the last step writes Ainv
+  PBG_CUDA(cudaMemsetAsync(src, 0, nn * sizeof(double), s));
+  k_dense_fill<<<grid_for(n), kThreads, 0, s>>>(L.back().m64, src); note_launch();
+  k_dense_dmax<<<1, 1024, 0, s>>>(n, src, dsc.p + 7); note_launch();
   const int gjr = (n + kGjRows - 1) / kGjRows, gjc = (n + kGjCols - 1) / kGjCols;
   const dim3 tiles(gjr, std::min(gjc, std::max(1, kGjGrid / gjr)));
   for (int k0 = 0; k0 < n; k0 += kGjB) {
     k_gj_block<<<tiles, 256, 0, s>>>(n, k0, src, dst, dsc.p + 7, 1e-10); note_launch();
     std::swap(src, dst);
   }
-  if (src != Ainv.p)
-    PBG_CUDA(cudaMemcpyAsync(Ainv.p, src, nn * sizeof(double), cudaMemcpyDeviceToDevice, s));
   if (have32) {
-    k_to_float<<<grid_for((long long)nn), kThreads, 0, s>>>((long long)nn, Ainv.p, Ainv32.p); note_launch();
+    k_to_float<<<grid_for((long long)nn), kThreads, 0, s>>>((long long)nn, Ainv, Ainv32); note_launch();
     if (Ainv16.n) {
       const int blocks = (int)(((long long)ncoarse * 32 + kThreads - 1) / kThreads);
-      k_to_half_rows<<<blocks, kThreads, 0, s>>>(ncoarse, Ainv.p, Ainv16.p, Ainv16s.p); note_launch();
+      k_to_half_rows<<<blocks, kThreads, 0, s>>>(ncoarse, Ainv, Ainv16.p, Ainv16s.p); note_launch();
     }
   }
   PBG_CUDA(cudaGetLastError());

@@ -97,7 +97,7 @@ struct EWork {
 struct EngineOpts {
   double omega_a = kOmegaA, omega_b = kOmegaB, over = kOverCorr;   // CycleW
   int coarse_max = 512;      // coarsest level size (dense direct solve)
-  bool coarse_auto = true;   // not chosen by the caller: up to 1024 where that ends the levels
+  bool coarse_auto = true;   // not chosen by the caller: kCoarseAuto where that ends the levels
   int kc_max = 99;           // levels 1..kc_max run a K-cycle, deeper levels one visit
   EngineOpts();
 };
@@ -128,11 +128,12 @@ class Engine {
   RowPad pad;                          // rows of level 0
   EMat<double> A0{};                   // the operator in the caller's rows
   DBuf<double> pc, pw, ps, pb;         // its copy in padded rows
-  DBuf<double> Ainv;           // dense inverse of the coarsest operator
-  DBuf<float> Ainv32;          // its FP32 copy (mixed path)
+  DBuf<double> dense_mem;      // memory of the next three
+  double *Ainv = nullptr;      // dense inverse of the coarsest operator
+  double *Dtmp = nullptr;      // its Gauss-Jordan work copy
+  float *Ainv32 = nullptr;     // its FP32 copy (mixed path)
   DBuf<__half> Ainv16;         // row-scaled FP16 copy (mixed path, large coarsest levels)
   DBuf<float> Ainv16s;         // the row scales
-  DBuf<double> Dtmp;           // its Gauss-Jordan work copy
   int ncoarse = 0;
   bool have32 = false;
   EngineOpts opt;

@@ -43,15 +43,19 @@ def test_explicit_coarse_max_is_a_limit(engine, precision, before):
     ((20, 16, 18), 100, [(20, 16, 18), (10, 8, 9), (5, 4, 5)]),
     ((17, 33, 30), 0, [(17, 33, 30), (9, 17, 15), (5, 9, 8)]),        # padded rows
     ((66, 71, 1), 0, [(66, 71, 1), (33, 36, 1), (17, 18, 1)]),        # 2-D, padded
-    ((24, 18, 17), 0, [(24, 18, 17), (12, 9, 9)]),                    # 972 cells, stored as 1080
+    ((24, 18, 17), 0, [(24, 18, 17), (12, 9, 9), (6, 5, 5)]),         # 972 cells on level 1: coarsened
+    ((36, 33, 38), 0, [(36, 33, 38), (18, 17, 19), (9, 9, 10)]),      # 810 cells on level 2: the coarsest
+    ((41, 31, 35), 0, [(41, 31, 35), (21, 16, 18), (11, 8, 9)]),      # 792 cells, stored as 880
+    ((12, 8, 8), 0, [(12, 8, 8)]),
+    ((10, 10, 10), 0, [(10, 10, 10), (5, 5, 5)]),
     ((31, 32, 35), 4096, [(31, 32, 35), (16, 16, 18), (8, 8, 9)]),
-    ((64, 64, 2), 0, [(64, 64, 2), (32, 32, 1)]),                     # thin
+    ((64, 64, 2), 0, [(64, 64, 2), (32, 32, 1), (16, 16, 1)]),        # thin
     ((9, 5, 7), 0, [(9, 5, 7)]),
 ])
 def test_levels_are_those_of_the_hierarchy(engine, dims, coarse_max, levels):
     """pbg_levels and pbg_result.levels: the levels that are solved on, with
     the extents of the caller's grid halved (no pad cells)."""
-    P = problem(dims, False)
+    P = problem(dims, False, solids=0.0)
     with engine.Session(*dims, P.h) as s:
         s.upload_matrix(P.A)
         E = engine.Engine(s)
