@@ -174,6 +174,7 @@ __device__ bool stale_step_dev(KrylovState *st, double res) {
   return stale_step(st->stale, stale_entries(st->stalecount), res);
 }
 
+template <bool Seq>
 __global__ void k_cg_init(MatView<double> A, const double *__restrict__ x,
                           const double *__restrict__ b, double *__restrict__ r,
                           KrylovState *st, double *part, unsigned *count, const double *__restrict__ mc) {
@@ -189,7 +190,7 @@ __global__ void k_cg_init(MatView<double> A, const double *__restrict__ x,
     v[1] += __dmul_rn(rv, __dmul_rn(rv, mc[p]));
   }
   double o[2];
-  if (grid_reduce<2>(v, part, count, o, st->seq, N)) {
+  if (grid_reduce<2>(v, part, count, o, Seq ? st->seq : nullptr, N)) {
     double res = res_of(o[0], st);
     st->res0 = res;
     st->res = res;
@@ -213,7 +214,8 @@ __global__ void k_cg_init(MatView<double> A, const double *__restrict__ x,
   }
 }
 
-__global__ void __launch_bounds__(kThreads, 3) k_cg_pq(MatView<double> A, const double *__restrict__ r, double *pA, double *pB,
+template <bool Seq>
+__global__ void __launch_bounds__(kThreads, Seq ? 3 : 4) k_cg_pq(MatView<double> A, const double *__restrict__ r, double *pA, double *pB,
                         double *__restrict__ qv, KrylovState *st, double *part, unsigned *count,
                         const double *__restrict__ zarr, const double *__restrict__ mc) {
   if (st->done) return;
@@ -238,7 +240,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_cg_pq(MatView<double> A, const 
     v[0] += __dmul_rn(pp, qq);
   }
   double o[1];
-  if (grid_reduce<1>(v, part, count, o, st->seq, N)) {
+  if (grid_reduce<1>(v, part, count, o, Seq ? st->seq : nullptr, N)) {
     st->beta = beta;
     st->pq = o[0];
     st->alfa = __ddiv_rn(st->rho, o[0]);
@@ -269,7 +271,8 @@ __device__ __forceinline__ void cg_step_end(KrylovState *st, double *hist, int i
   }
 }
 
-__global__ void __launch_bounds__(kThreads, 3) k_cg_xr(long long N, const double *__restrict__ mc, double *__restrict__ x,
+template <bool Seq>
+__global__ void __launch_bounds__(kThreads, Seq ? 3 : 4) k_cg_xr(long long N, const double *__restrict__ mc, double *__restrict__ x,
                         double *__restrict__ r, const double *pA, const double *pB,
                         const double *__restrict__ qv, KrylovState *st, double *hist,
                         double *part, unsigned *count, int ic) {
@@ -288,7 +291,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_cg_xr(long long N, const double
     v[1] += __dmul_rn(rv, __dmul_rn(rv, mc[p]));
   }
   double o[2];
-  if (grid_reduce<2>(v, part, count, o, st->seq, N)) cg_step_end(st, hist, it, o[0], o[1], ic);
+  if (grid_reduce<2>(v, part, count, o, Seq ? st->seq : nullptr, N)) cg_step_end(st, hist, it, o[0], o[1], ic);
 }
 
 // ---------------------------------------------------------------------------
@@ -1326,7 +1329,7 @@ void enqueue_ref_setup(const MatView<double> &A, double *x, const double *b, con
   }
   k_recip<<<grid_for(N), kThreads, 0, s>>>(N, A.c, w.mcd.p); note_launch();
   if (solver == 0) {
-    k_cg_init<<<g, kThreads, 0, s>>>(A, x, b, w.r.p, st, red.slot_part(0), red.slot_count(0), w.mcd.p); note_launch();
+    sum(k_cg_init<true>, k_cg_init<false>, A, x, b, w.r.p, st, red.slot_part(0), red.slot_count(0), w.mcd.p);
   } else {
     sum(k_bi_init<true>, k_bi_init<false>, A, x, b, w.r.p, w.rt.p, st, red.slot_part(0), red.slot_count(0));
   }
@@ -1392,20 +1395,20 @@ void enqueue_ref_iters(const MatView<double> &A, double *x, int solver, int coun
       // z = M^-1 r (forward and backward sweeps), rho = r.z, then the CG step
       ic_apply(A, prec, w, w.r.p, w.z.p, st, s);
       sum(k_cg_rho<true>, k_cg_rho<false>, N, w.r.p, w.z.p, st, P0, C0);
-      k_cg_pq<<<g, kThreads, 0, s>>>(A, w.r.p, w.pA.p, w.pB.p, w.q.p, st, P0, C0, w.z.p, w.mcd.p); note_launch();
-      k_cg_xr<<<g, kThreads, 0, s>>>(N, w.mcd.p, x, w.r.p, w.pA.p, w.pB.p, w.q.p, st, hist, P1, C1, 1); note_launch();
+      sum(k_cg_pq<true>, k_cg_pq<false>, A, w.r.p, w.pA.p, w.pB.p, w.q.p, st, P0, C0, w.z.p, w.mcd.p);
+      sum(k_cg_xr<true>, k_cg_xr<false>, N, w.mcd.p, x, w.r.p, w.pA.p, w.pB.p, w.q.p, st, hist, P1, C1, 1);
     } else if (solver == 0 && !exact && A.nz % 2 == 0 && !A.per) {
       const int gq = grid_for(N / 2);
       k_cg_p<<<gq, kThreads, 0, s>>>(N, w.r.p, w.mcd.p, w.pA.p, st); note_launch();
       k_cg_q<<<gq, kThreads, 0, s>>>(A, Geo(A.nx, A.ny, A.nz), w.pA.p, w.q.p, st, P0, C0); note_launch();
-      if (reinterpret_cast<uintptr_t>(x) % 16 == 0)   // x is the caller's
-        k_cg_xr2<<<gq, kThreads, 0, s>>>(N, w.mcd.p, x, w.r.p, w.pA.p, w.q.p, st, hist, P1, C1);
-      else
-        k_cg_xr<<<g, kThreads, 0, s>>>(N, w.mcd.p, x, w.r.p, w.pA.p, w.pA.p, w.q.p, st, hist, P1, C1, 0);
-      note_launch();
+      if (reinterpret_cast<uintptr_t>(x) % 16 == 0) {   // x is the caller's
+        k_cg_xr2<<<gq, kThreads, 0, s>>>(N, w.mcd.p, x, w.r.p, w.pA.p, w.q.p, st, hist, P1, C1); note_launch();
+      } else {
+        sum(k_cg_xr<true>, k_cg_xr<false>, N, w.mcd.p, x, w.r.p, w.pA.p, w.pA.p, w.q.p, st, hist, P1, C1, 0);
+      }
     } else if (solver == 0) {
-      k_cg_pq<<<g, kThreads, 0, s>>>(A, w.r.p, w.pA.p, w.pB.p, w.q.p, st, P0, C0, nullptr, w.mcd.p); note_launch();
-      k_cg_xr<<<g, kThreads, 0, s>>>(N, w.mcd.p, x, w.r.p, w.pA.p, w.pB.p, w.q.p, st, hist, P1, C1, 0); note_launch();
+      sum(k_cg_pq<true>, k_cg_pq<false>, A, w.r.p, w.pA.p, w.pB.p, w.q.p, st, P0, C0, nullptr, w.mcd.p);
+      sum(k_cg_xr<true>, k_cg_xr<false>, N, w.mcd.p, x, w.r.p, w.pA.p, w.pB.p, w.q.p, st, hist, P1, C1, 0);
     } else if (solver == 1) {
       sum(k_bi_rho<true>, k_bi_rho<false>, N, w.rt.p, w.r.p, st, P0, C0);
       k_bi_p<<<g, kThreads, 0, s>>>(N, w.mcd.p, w.r.p, w.pA.p, w.v.p, w.ph.p, st, diag); note_launch();
