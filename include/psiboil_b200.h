@@ -120,8 +120,8 @@ typedef struct {
   int max_sweeps;         /* mixed: refinement sweeps at most                    */
   /* reference-parity solvers: 1 = every global sum rounded as the
    * reference's sequential i,j,k loop rounds it (bit-for-bit reference
-   * results; computed in parallel, see pbg_seq_sum, about 15x the time of
-   * a tree sum); 0 = deterministic tree sums */
+   * results; computed in parallel, see pbg_seq_sum; a CG step takes 11 to
+   * 13 times as long from 128^3 cells on); 0 = deterministic tree sums */
   int exact_sums;
   /* engine: cells of the dense coarsest level at most, until a later call
    * names another size; 0: as an earlier call on this session chose, else the

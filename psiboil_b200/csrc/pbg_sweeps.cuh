@@ -21,13 +21,13 @@
 // every tile's predecessors come first, so a block only ever waits for blocks
 // that are already running.
 //
-// What bounds it: the chain of a (nx + ny - 2) + nz dependent steps, 0.16 us
-// each for IC0 and 0.21 us for IC2 (shared loads, four to six dependent FP64
-// operations of 9 cycles, the division's correction, a barrier), and about
-// 3 us for each tile edge on the way. One launch per plane, the form before
-// this, paid 4.5 us a step. Measured (B200): an IC2 sweep at 64^3 117 us
-// (1290 before), CG with IC2 64x56x50, 20 iterations, 52.5 -> 5.9 ms;
-// Gauss-Seidel 64x72x60, 10 sweeps, 10.9 -> 1.14 ms. All operands that the
+// What bounds it: the chain of a (nx + ny - 2) + nz dependent steps, 0.15 us
+// each for IC0, 0.20 us for IC2 and 0.12 us for Gauss-Seidel (shared loads, four
+// to six dependent FP64 operations of 9 cycles, the division's correction, a
+// barrier), and 2.6 to 2.9 us for each tile edge on the way. One launch per plane,
+// the form before this, paid 4.5 us a step. Measured (B200): an IC2 sweep at 64^3
+// 109 us (1290 before), CG with IC2 64x56x50, 20 iterations, 52.6 -> 5.9 ms;
+// Gauss-Seidel 64x72x60, 10 sweeps, 10.9 -> 1.13 ms. All operands that the
 // sweeps own are stored in march order (SweepGeo::off), so that a step reads
 // contiguous rows at constant offsets from one pointer.
 #pragma once
