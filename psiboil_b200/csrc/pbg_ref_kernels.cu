@@ -1220,13 +1220,13 @@ void RefKrylovWork::sweep_alloc(size_t n, cudaStream_t s) {
     words.alloc(n);
     PBG_CUDA(cudaMemsetAsync(words.p, 0, words.bytes(), s));
   }
+  if (!hstuck) {   // before the tickets, whose presence says that it is there
+    PBG_CUDA(cudaMallocHost((void **)&hstuck, sizeof(int)));
+    *hstuck = 0;
+  }
   if (!ticket.n) {
     ticket.alloc(4);
     PBG_CUDA(cudaMemsetAsync(ticket.p, 0, ticket.bytes(), s));
-  }
-  if (!hstuck) {
-    PBG_CUDA(cudaMallocHost((void **)&hstuck, sizeof(int)));
-    *hstuck = 0;
   }
 }
 
